@@ -15,6 +15,7 @@
 #include <vector>
 
 #include "drivers.cuh"
+#include "even.cuh"
 #include "linalg.cuh"
 
 namespace pgb {
@@ -270,6 +271,19 @@ void upload_inputs(Inputs& in, const int64_t* kmap, const int64_t* invk, const i
   }
 }
 
+// The even form of the convolutions and vertices (even.cuh) where the model has
+// it: H, and what the bands give, symmetric on every k point.  elem_bytes: the
+// widest bulk element the solve may use.
+void detect_even(Inputs& in, const double* Smat, const double* Cmat, const double2* hamk, const double* eig,
+                 const double2* uni, int elem_bytes) {
+  if (hamk && !symmetric_h(hamk, in.Nk, in.Norb)) return;
+  if (eig && uni && !symmetric_bands(eig, uni, in.Nk, in.Norb)) return;
+  in.g.even = make_even(in.g, in.p, Smat, Cmat, elem_bytes);
+}
+// chi holds the class representatives only (and every element at nu = 0)
+// between the stages of an even model whose vertex runs in the real basis
+bool compact_chi(const Inputs& in) { return in.g.even && in.g.even->vertex_ok; }
+
 // ================================================================ mkself ==
 // One bulk step of the FLEX loop: chi0 (plain or tail-corrected) -> Stoner
 // factor (and the sw_rescale clamp) -> V_sigma -> Sigma (FP64 out).  Each of
@@ -281,7 +295,7 @@ double stage_chi0(Inputs& in, const FlexParams& a, const double2* G, double mu, 
   Timer tm;
   tm.start();
   TailRef tail{in.eig.p, in.uni.p, mu};
-  chi0<R>(g, in.p, G, a.temp, a.sw_tail ? &tail : nullptr, chi);
+  chi0<R>(g, in.p, G, a.temp, a.sw_tail ? &tail : nullptr, chi, !compact_chi(in));
   g_stats.t_chi0 += tm.stop();
   double sdw = 0, cdw = 0;
   int qs = 0, qc = 0;
@@ -301,6 +315,13 @@ double stage_chi0(Inputs& in, const FlexParams& a, const double2* G, double mu, 
   g_stats.t_stoner += tm.stop();
   return sdw;
 }
+// the vertex of nmat matrices (element stride nmat): in the real basis of an
+// even model, or the general form
+template <typename R>
+bool vertex_of(const Inputs& in, cx<R>* chi, long long nmat, int mode, bool full) {
+  if (compact_chi(in)) return vertex_even<R>(*in.g.even, chi, nmat, nmat, mode, full);
+  return vertex<R>(chi, nmat, nmat, in.Nchi, in.S.p, in.C.p, mode);
+}
 template <typename R>
 void stage_vertex(Inputs& in, cx<R>* chi) {
   Timer tm;
@@ -309,7 +330,7 @@ void stage_vertex(Inputs& in, cx<R>* chi) {
     PGB_CHECK((std::is_same<R, double>::value), "the spin-orbit loop runs in FP64");
     PGB_CHECK(vertex_soc(reinterpret_cast<double2*>(chi), in.g.K, in.Nchi, in.V.p), "zgesv failed in V_sigma");
   } else {
-    PGB_CHECK(vertex<R>(chi, in.g.K, in.g.K, in.Nchi, in.S.p, in.C.p, 0), "zgesv failed in V_sigma");
+    PGB_CHECK(vertex_of<R>(in, chi, in.g.K, 0, false), "zgesv failed in V_sigma");
   }
   g_stats.t_vertex += tm.stop();
 }
@@ -341,14 +362,19 @@ struct ChiBufs {
   }
 };
 
-void convert_chi(void* out, int to, const void* in, int from, long long n) {
+template <typename To, typename From>
+void convert_chi_as(const Inputs& in, void* out, const void* src) {
+  if (compact_chi(in)) convert_even<To, From>(*in.g.even, (cx<To>*)out, (const cx<From>*)src, in.g.K);
+  else convert<To, From>((cx<To>*)out, (const cx<From>*)src, in.g.K * in.Nchi * in.Nchi);
+}
+void convert_chi(const Inputs& in, void* out, int to, const void* src, int from) {
   if (to == from) return;
-  if (to == 32 && from == 64) convert<float, double>((float2*)out, (const double2*)in, n);
-  else if (to == 64 && from == 32) convert<double, float>((double2*)out, (const float2*)in, n);
-  else if (to == 32 && from == 48) convert<float, dfl>((float2*)out, (const cdf*)in, n);
-  else if (to == 48 && from == 32) convert<dfl, float>((cdf*)out, (const float2*)in, n);
-  else if (to == 64 && from == 48) convert<double, dfl>((double2*)out, (const cdf*)in, n);
-  else convert<dfl, double>((cdf*)out, (const double2*)in, n);
+  if (to == 32 && from == 64) convert_chi_as<float, double>(in, out, src);
+  else if (to == 64 && from == 32) convert_chi_as<double, float>(in, out, src);
+  else if (to == 32 && from == 48) convert_chi_as<float, dfl>(in, out, src);
+  else if (to == 48 && from == 32) convert_chi_as<dfl, float>(in, out, src);
+  else if (to == 64 && from == 48) convert_chi_as<double, dfl>(in, out, src);
+  else convert_chi_as<dfl, double>(in, out, src);
 }
 
 // Bosonic frequencies whose vertex the middle phase of the mixed schedule
@@ -382,16 +408,16 @@ double flex_bulk(Inputs& in, const FlexParams& a, const double2* G, double mu, c
     low.alloc(nlow * (long long)nel);
     PGB_CUDA(cudaMemcpy2DAsync(low.p, nlow * sizeof(cdf), c0, K * sizeof(cdf), nlow * sizeof(cdf), nel,
                                cudaMemcpyDeviceToDevice, ctx().stream));
-    PGB_CHECK(vertex<dfl>(low.p, nlow, nlow, in.Nchi, in.S.p, in.C.p, 0), "zgesv failed in V_sigma");
+    PGB_CHECK(vertex_of<dfl>(in, low.p, nlow, 0, false), "zgesv failed in V_sigma");
     g_stats.t_vertex += tl.stop();
   }
   void* cv = b.get(sp.vertex, KC);
-  convert_chi(cv, sp.vertex, c0, sp.chi0, KC);
+  convert_chi(in, cv, sp.vertex, c0, sp.chi0);
   if (sp.vertex == 32) stage_vertex<float>(in, (float2*)cv);
   else if (sp.vertex == 48) stage_vertex<dfl>(in, (cdf*)cv);
   else stage_vertex<double>(in, (double2*)cv);
   void* cs = b.get(sp.sigma, KC);
-  convert_chi(cs, sp.sigma, cv, sp.vertex, KC);
+  convert_chi(in, cs, sp.sigma, cv, sp.vertex);
   if (nlow > 0)
     PGB_CUDA(cudaMemcpy2DAsync(cs, K * sizeof(cdf), low.p, nlow * sizeof(cdf), nlow * sizeof(cdf), nel,
                                cudaMemcpyDeviceToDevice, ctx().stream));
@@ -517,6 +543,8 @@ void mkself_core(Inputs& in, const FlexParams& a, double2* sig_out, double* mu_o
       log("[FLEX] scale loaded sigma seed by%10.6f\n", a.sigma_scale);
       scal(sig.p, a.sigma_scale, KE);
     }
+    // a seed without the model's symmetry takes the solve to the general form
+    if (in.g.even && !symmetric_blocks(sig.p, K, Norb, 1.0e-12)) in.g.even.reset();
     PGB_CUDA(cudaMemcpyAsync(sig0.p, sig.p, KE * sizeof(double2), cudaMemcpyDeviceToDevice, st));
     PGB_CHECK(dyson(G.p, sig.p, H.p, mu, a.temp, Nk, Nw, Norb), "singular G^-1 in the Dyson step");
   } else {
@@ -796,6 +824,7 @@ void run_mkself(const MkselfArgs& a, int prec) {
                 a.hamk, a.eig, a.uni);
   FlexParams prm{a.mu_init, a.fill, a.temp, a.scf_loop, a.pp, a.eps, a.sub_sigma, a.sw_out, a.sw_in, a.m_diis,
                  a.sw_rescale, a.sw_tail, a.sigma_scale};
+  detect_even(in, a.Smat, a.Cmat, a.hamk, a.eig, a.uni, prec == 32 ? 8 : 16);
   const long long KE = in.g.K * a.Norb * a.Norb;
   DBuf<double2> sig(KE);
   mkself_core(in, prm, sig.p, a.mu_out, nullptr, 0.0, 0.0, prec);
@@ -978,18 +1007,19 @@ int eliash_fp32_cycles() {
 // V_Delta in the bulk type of the Eliashberg stage; for double-float the
 // solve runs in double-float, or in FP64 with PYRPA_GB_ELIASH=df64
 template <typename R>
-bool vertex_delta(cx<R>* chi, long long K, int Nchi, const double* S, const double* C, int mode) {
+bool vertex_delta(const Inputs& in, cx<R>* chi, int mode, bool full) {
+  const long long K = in.g.K;
   const char* e = std::getenv("PYRPA_GB_ELIASH");
   if constexpr (std::is_same<R, dfl>::value) {
-    if (!(e && std::string(e) == "df64")) return vertex<dfl>(chi, K, K, Nchi, S, C, mode);
-    const long long n = K * Nchi * Nchi;
+    if (!(e && std::string(e) == "df64")) return vertex_of<dfl>(in, chi, K, mode, full);
+    const long long n = K * in.Nchi * in.Nchi;
     DBuf<double2> t(n);
     widen<dfl>(t.p, chi, n);
-    const bool ok = vertex<double>(t.p, K, K, Nchi, S, C, mode);
+    const bool ok = vertex_of<double>(in, t.p, K, mode, full);
     narrow<dfl>(chi, t.p, n);
     return ok;
   } else {
-    return vertex<R>(chi, K, K, Nchi, S, C, mode);
+    return vertex_of<R>(in, chi, K, mode, full);
   }
 }
 
@@ -1009,10 +1039,16 @@ double eliash_core(Inputs& in, cx<R>* chi, const double2* G, const double* init,
   DBuf<double>& S = in.S;
   DBuf<double>& C = in.C;
   DBuf<double2>& uni = in.uni;
+  std::vector<double> hprt(Norb);
+  PGB_CUDA(cudaMemcpyAsync(hprt.data(), prt, sizeof(double) * Norb, cudaMemcpyDeviceToHost, st));
+  sync();
+  // F is even in k for a singlet of orbitals of one parity
+  bool even_delta = in.g.even && singlet;
+  for (double x : hprt) even_delta = even_delta && (x == 1.0 || x == -1.0) && x == hprt[0];
   {
     Timer tv;
     tv.start();
-    PGB_CHECK(vertex_delta<R>(chi, K, Nchi, S.p, C.p, singlet ? 1 : 2), "zgesv failed in V_delta");
+    PGB_CHECK(vertex_delta<R>(in, chi, singlet ? 1 : 2, chi_host || !even_delta), "zgesv failed in V_delta");
     g_stats.t_vertex += tv.stop();
     if (chi_host) {
       DBuf<double2> tmp(KC);
@@ -1051,9 +1087,6 @@ double eliash_core(Inputs& in, cx<R>* chi, const double2* G, const double* init,
   std::unique_ptr<DBuf<cdf>> Gdf, Fdf;
   if constexpr (std::is_same<R, dfl>::value) {
     const char* e = std::getenv("PYRPA_GB_MKFK_DF");
-    std::vector<double> hprt(Norb);
-    PGB_CUDA(cudaMemcpyAsync(hprt.data(), prt, sizeof(double) * Norb, cudaMemcpyDeviceToHost, st));
-    sync();
     bool signs = true;
     for (double x : hprt) signs = signs && (x == 1.0 || x == -1.0);
     if (!(e && std::string(e) == "0") && signs && Norb <= 5) {
@@ -1066,15 +1099,17 @@ double eliash_core(Inputs& in, cx<R>* chi, const double2* G, const double* init,
     ta.start();
     if (chi32) {
       mkfk(F.p, G, v, K, Norb);
-      mkdelta<float>(g, p, F.p, chi32->p, S.p, C.p, prt, singlet, scale, out, cache32.get());
+      mkdelta<float>(g, p, F.p, chi32->p, S.p, C.p, prt, singlet, scale, out, cache32.get(), nullptr,
+                     even_delta);
     } else if (Fdf) {
       if constexpr (std::is_same<R, dfl>::value) {
         PGB_CHECK(mkfk_df(Fdf->p, Gdf->p, v, K, Norb), "no double-float mkfk for this orbital count");
-        mkdelta<R>(g, p, nullptr, chi, S.p, C.p, prt, singlet, scale, out, &cache, Fdf->p);
+        mkdelta<R>(g, p, nullptr, chi, S.p, C.p, prt, singlet, scale, out, &cache, Fdf->p,
+                   even_delta);
       }
     } else {
       mkfk(F.p, G, v, K, Norb);
-      mkdelta<R>(g, p, F.p, chi, S.p, C.p, prt, singlet, scale, out, &cache);
+      mkdelta<R>(g, p, F.p, chi, S.p, C.p, prt, singlet, scale, out, &cache, nullptr, even_delta);
     }
     g_stats.t_apply += ta.stop();
     g_stats.applies += 1;
@@ -1178,6 +1213,11 @@ void run_lin_eliash(const LinEliashArgs& a) {
   {
     DBuf<double2> tmp(KC);
     tmp.upload(a.chi, KC);
+    // the even form for a G and a chi that have an even model's relations
+    if (symmetric_blocks(G.p, in.g.K, (int)a.Norb, 1.0e-12)) {
+      in.g.even = make_even(in.g, in.p, a.Smat, a.Cmat, (int)sizeof(cx<R>));
+      if (in.g.even && (!in.g.even->vertex_ok || !even_chi(in.g, *in.g.even, tmp.p, 1.0e-12))) in.g.even.reset();
+    }
     if (std::is_same<R, double>::value)
       PGB_CUDA(cudaMemcpyAsync(chi.p, tmp.p, KC * sizeof(double2), cudaMemcpyDeviceToDevice, ctx().stream));
     else narrow<R>(chi.p, tmp.p, KC);
@@ -1254,6 +1294,13 @@ void coarse_seed_level(Inputs& in, const HostBands& hb, int64_t kdiv, int64_t wd
                            ctx().stream));
   PGB_CUDA(cudaMemcpyAsync(ic.C.p, in.C.p, sizeof(double) * in.Nchi * in.Nchi, cudaMemcpyDeviceToDevice,
                            ctx().stream));
+  if (in.g.even) {
+    std::vector<double> hS((size_t)in.Nchi * in.Nchi), hC(hS.size());
+    in.S.download(hS.data(), hS.size());
+    in.C.download(hC.data(), hC.size());
+    sync();
+    ic.g.even = make_even(ic.g, ic.p, hS.data(), hC.data(), 16);
+  }
   FlexParams pc = prm;
   pc.eps = prm.eps;
   pc.stop_at_fp32_floor = true;
@@ -1275,6 +1322,8 @@ void coarse_seed_level(Inputs& in, const HostBands& hb, int64_t kdiv, int64_t wd
   g_stats.iterations = g_stats.iterations32 = 0;
   seed.alloc((size_t)g.K * No * No);
   sigma_interp(ic.g, g, sc.p, seed.p, No, prm.temp);
+  // the interpolation runs in FP32: its rounding must not break the symmetry
+  if (g.even) symmetrize_blocks(seed.p, g.K, No);
   *mu_seed = mu_c;
 }
 
@@ -1293,6 +1342,7 @@ void run_pipeline_impl(const PipelineArgs& a, int prec) {
   upload_inputs(in, a.kmap, a.invk, a.olist, a.Nx, a.Ny, a.Nz, a.Nkall, a.Nk, a.Nw, a.Norb, a.Nchi, a.Smat, a.Cmat,
                 a.hamk, a.eig, a.uni);
   const long long K = in.g.K, KE = K * a.Norb * a.Norb, KC = K * a.Nchi * a.Nchi;
+  detect_even(in, a.Smat, a.Cmat, a.hamk, a.eig, a.uni, 16);
   DBuf<double> prt(a.Norb), init(a.Nk * a.Norb);
   prt.upload(a.prt, a.Norb);
   init.upload(a.init_delta, a.Nk * a.Norb);
@@ -1325,7 +1375,7 @@ void run_pipeline_impl(const PipelineArgs& a, int prec) {
   {
     DBuf<cx<R>> chi(KC);
     TailRef tr{in.eig.p, in.uni.p, mu};
-    chi0<R>(in.g, in.p, G.p, a.temp, a.sw_tail ? &tr : nullptr, chi.p);
+    chi0<R>(in.g, in.p, G.p, a.temp, a.sw_tail ? &tr : nullptr, chi.p, !compact_chi(in));
     double cdw = 0;
     int qs = 0, qc = 0;
     stoner<R>(in.g, chi.p, in.S.p, in.C.p, &stoner_v, &cdw, &qs, &qc);

@@ -1,0 +1,997 @@
+// Kernels and stages of even.cuh, instantiated per bulk type in even_*.cu.
+#pragma once
+
+#include <algorithm>
+#include <map>
+#include <mutex>
+#include <type_traits>
+
+#include "even.cuh"
+#include "fft_dev.cuh"
+#include "flex_dev.cuh"
+
+namespace pgb {
+namespace {
+
+// ------------------------------------------------------------ space transform
+enum SpaceIn { kInPlain, kInBoson, kInFermi64, kInFermi, kInPostBoson, kInPostFermi, kInAny };
+enum SpaceOut { kOutPlain, kOutChi, kOutSigma, kOutAny };  // kInAny, kOutAny: SpaceArgs says which
+__host__ __device__ constexpr bool fermi_mode(int in) { return in == kInFermi || in == kInFermi64 || in == kInPostFermi; }
+
+template <typename R> struct SpaceArgs {
+  const void* src;
+  void* dst;
+  int nx, ny, nplanes;         // nplanes: planes per slot (1, or Nz/2 + 1)
+  int H, Nk, Nw, sign;
+  int in, out;                 // SpaceIn, SpaceOut
+  int nst[2], radix[2][8];
+  const cx<R>* tab[2];         // roots of nx and ny
+  const cx<R>* root;           // roots of M (bosons) or 2M (fermions)
+  const int *h_irr, *irr_h;
+  const int *korder, *koff;    // irreducible k by plane of the half grid
+  const int* el;               // boson in: element per array; fermion in / Sigma out: orbital element
+  const R* stat;               // boson in: static slot per array
+  // chi out
+  const int *mem, *memcj, *nmem;
+  const cx<R>* J;              // per array; null without the tail
+  const cx<R>* sawc;
+  int full;
+  // Sigma out
+  const int* elt;              // transposed element
+  double scale;
+  int thresh;
+};
+
+// slot of block b: a slot and its partner of the pre/post-processing are
+// neighbours in the launch, so that their common inputs meet in L2
+__device__ __forceinline__ int boson_slot(int b, int Nw) { return (b & 1) ? (b + 1) >> 1 : (b ? Nw - (b >> 1) : 0); }
+__device__ __forceinline__ int fermi_slot(int b, int Nw) { return (b & 1) ? Nw - 1 - (b >> 1) : (b >> 1); }
+
+template <typename R>
+__device__ __forceinline__ cx<R> pre_mix(cx<R> p, cx<R> q, cx<R> w) {
+  return (p + q) + muli((p - q) * w, (R)1);
+}
+// F(j) from C(j) and C(partner): E + conj(w) O
+template <typename R>
+__device__ __forceinline__ cx<R> post_mix(cx<R> c, cx<R> cp, cx<R> w) {
+  const R half = (R)0.5f;
+  const cx<R> e = half * (c + conj(cp)), o = muli(half * (c - conj(cp)), (R)-1);
+  return e + conj(w) * o;
+}
+template <typename R> __device__ __forceinline__ cx<R> from64(double2 v) { return cmk<R>((R)v.x, (R)v.y); }
+
+// value of the space transform's input at half-grid point h of slot j
+template <typename R, int IN>
+__device__ __forceinline__ cx<R> space_load(const SpaceArgs<R>& a, int h, int j, int arr, cx<R> w, R stat) {
+  if constexpr (IN == kInAny) {
+    switch (a.in) {
+      case kInBoson: return space_load<R, kInBoson>(a, h, j, arr, w, stat);
+      case kInFermi64: return space_load<R, kInFermi64>(a, h, j, arr, w, stat);
+      case kInFermi: return space_load<R, kInFermi>(a, h, j, arr, w, stat);
+      case kInPostBoson: return space_load<R, kInPostBoson>(a, h, j, arr, w, stat);
+      case kInPostFermi: return space_load<R, kInPostFermi>(a, h, j, arr, w, stat);
+      default: return space_load<R, kInPlain>(a, h, j, arr, w, stat);
+    }
+  } else if constexpr (IN == kInBoson) {
+    const cx<R>* v = static_cast<const cx<R>*>(a.src) + (long long)a.el[arr] * a.Nk * a.Nw + a.h_irr[h];
+    const cx<R> p = v[(long long)a.Nk * j];
+    const cx<R> q = j ? conj(v[(long long)a.Nk * (a.Nw - j)]) : cmk<R>(stat, (R)0);
+    return pre_mix<R>(p, q, w);
+  } else if constexpr (IN == kInFermi64) {
+    const double2* v = static_cast<const double2*>(a.src) + (long long)a.el[arr] * a.Nk * a.Nw + a.h_irr[h];
+    return pre_mix<R>(from64<R>(v[(long long)a.Nk * j]), conj(from64<R>(v[(long long)a.Nk * (a.Nw - 1 - j)])), w);
+  } else if constexpr (IN == kInFermi) {
+    const cx<R>* v = static_cast<const cx<R>*>(a.src) + (long long)a.el[arr] * a.Nk * a.Nw + a.h_irr[h];
+    return pre_mix<R>(v[(long long)a.Nk * j], conj(v[(long long)a.Nk * (a.Nw - 1 - j)]), w);
+  } else {
+    const cx<R>* v = static_cast<const cx<R>*>(a.src) + (long long)arr * a.H * a.Nw + h;
+    const cx<R> c = v[(long long)a.H * j];
+    if constexpr (IN == kInPostBoson) return post_mix<R>(c, v[(long long)a.H * (j ? a.Nw - j : 0)], w);
+    if constexpr (IN == kInPostFermi) return post_mix<R>(c, v[(long long)a.H * (a.Nw - 1 - j)], w);
+    return c;
+  }
+}
+
+template <typename R> __device__ __forceinline__ cx<R> space_root(const SpaceArgs<R>& a, int in, int j) {
+  if (in == kInPlain) return cmk<R>((R)0, (R)0);
+  return twid<R>(a.root, fermi_mode(in) ? 2 * j + 1 : j, -1);
+}
+
+template <typename R>
+__device__ __forceinline__ void space_store(const SpaceArgs<R>& a, int out, cx<R> v, int k, int j, int arr, cx<R> J, cx<R> saw) {
+  const long long K = (long long)a.Nk * a.Nw, at = k + (long long)a.Nk * j;
+  if (out == kOutChi) {
+    cx<R>* chi = static_cast<cx<R>*>(a.dst);
+    if (a.J) v += J * saw;
+    if (abs_below(v.x, kThresh)) v.x = 0;
+    if (abs_below(v.y, kThresh)) v.y = 0;
+    const int n = (a.full || j == 0) ? a.nmem[arr] : 1;
+    for (int i = 0; i < n; ++i) chi[a.mem[4 * arr + i] * K + at] = a.memcj[4 * arr + i] ? conj(v) : v;
+  } else {
+    double2* s = static_cast<double2*>(a.dst);
+    double2 d = mkc((double)v.x, (double)v.y);
+    d = a.scale * d;
+    if (a.thresh) d = thresh(d);
+    s[a.el[arr] * K + at] = d;
+    if (a.elt[arr] != a.el[arr]) s[a.elt[arr] * K + at] = d;
+  }
+}
+
+template <typename R, int N>
+__device__ __forceinline__ void axis_stages(cx<R>*& in, cx<R>*& out, int L, int nl, int es, int ls, int nst,
+                                            const int* radix, int sign, const cx<R>* tab) {
+  if constexpr (N > 0) {
+    stage_strided<R, 8>(in, out, N, 1, nl, es, ls, sign, tab);
+    __syncthreads();
+    stage_strided<R, N / 8>(out, in, N, 8, nl, es, ls, sign, tab);
+    __syncthreads();
+  } else {
+    plane_axis<R, N < 0>(in, out, L, nl, es, ls, nst, radix, sign, tab);
+  }
+}
+
+// One (x, y) plane of one slot and array per CTA.  HALF (2-D meshes): the half
+// plane y <= Ny/2 of a function even in (x, y); rows are transformed in x,
+// column x <= Nx/2 in y with its upper half read from the mirrored column, and
+// the result is again even.  Otherwise the whole plane.  N: the compile-time
+// side of square planes (0: sides of radices up to 8, -1: any sides).  The pre- and post-processing of the
+// half-length time transform, the gather from the irreducible points and the
+// scatter to them ride on the load and the store, so that no padded copy of
+// the array exists.
+template <typename R, int IN, int OUT, bool HALF, int N>
+__global__ void __launch_bounds__(256) k_space(SpaceArgs<R> a) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  const int nx = N > 0 ? N : a.nx, ny = N > 0 ? N : a.ny;
+  const int mi = IN == kInAny ? a.in : IN, mo = OUT == kOutAny ? a.out : OUT;
+  const int sx = nx + 1, rows = HALF ? ny / 2 + 1 : ny, nxc = nx / 2 + 1;
+  const int buf = HALF ? (rows * sx > ny * nxc ? rows * sx : ny * nxc) : ny * sx;
+  cx<R>* in = reinterpret_cast<cx<R>*>(smem_raw);
+  cx<R>* out = in + buf;
+  const int arr = blockIdx.y;
+  const int b = HALF ? blockIdx.x : blockIdx.x / a.nplanes, z = HALF ? 0 : blockIdx.x % a.nplanes;
+  const int j = fermi_mode(mi) ? fermi_slot(b, a.Nw) : boson_slot(b, a.Nw);
+  const cx<R> w = space_root<R>(a, mi, j);
+  const R stat = mi == kInBoson ? a.stat[arr] : (R)0;
+  const int npl = rows * nx, h0 = z * npl;
+  for (int e = threadIdx.x; e < npl; e += blockDim.x) {
+    const int y = e / nx, x = e - y * nx;
+    in[y * sx + x] = space_load<R, IN>(a, h0 + e, j, arr, w, stat);
+  }
+  __syncthreads();
+  axis_stages<R, N>(in, out, nx, rows, 1, sx, a.nst[0], a.radix[0], a.sign, a.tab[0]);
+  int cs = sx;
+  if constexpr (HALF) {
+    // columns x <= Nx/2, all rows: row y above Ny/2 is row Ny - y at -x
+    for (int e = threadIdx.x; e < ny * nxc; e += blockDim.x) {
+      const int y = e / nxc, x = e - y * nxc;
+      out[e] = y < rows ? in[y * sx + x] : in[(ny - y) * sx + (x ? nx - x : 0)];
+    }
+    __syncthreads();
+    cx<R>* t = in;
+    in = out;
+    out = t;
+    cs = nxc;
+    axis_stages<R, N>(in, out, ny, nxc, cs, 1, a.nst[1], a.radix[1], a.sign, a.tab[1]);
+  } else {
+    axis_stages<R, N>(in, out, ny, nx, cs, 1, a.nst[1], a.radix[1], a.sign, a.tab[1]);
+  }
+  auto at = [&](int x, int y) {
+    if (HALF && x >= nxc) {
+      x = nx - x;
+      y = y ? ny - y : 0;
+    }
+    return in[y * cs + x];
+  };
+  if (mo == kOutPlain) {
+    cx<R>* d = static_cast<cx<R>*>(a.dst) + (long long)arr * a.H * a.Nw + (long long)a.H * j + h0;
+    for (int e = threadIdx.x; e < npl; e += blockDim.x) {
+      const int y = e / nx, x = e - y * nx;
+      d[e] = at(x, y);
+    }
+  } else {
+    cx<R> J = cmk<R>((R)0, (R)0), saw = J;
+    if (mo == kOutChi && a.J) {
+      J = a.J[arr];
+      saw = a.sawc[j];
+    }
+    const int k0 = a.koff[z], k1 = a.koff[z + 1];
+    for (int i = k0 + threadIdx.x; i < k1; i += blockDim.x) {
+      const int k = a.korder[i], h = a.irr_h[k] - h0;
+      const int y = h / nx, x = h - y * nx;
+      space_store<R>(a, mo, at(x, y), k, j, arr, J, saw);
+    }
+  }
+}
+
+template <typename R, int IN, int OUT>
+void space_launch(const Even& ev, SpaceArgs<R>& a, int narr, int sign, cudaStream_t st) {
+  a.nx = ev.nx;
+  a.ny = ev.ny;
+  a.H = ev.H;
+  a.Nw = ev.Nw;
+  a.sign = sign;
+  a.h_irr = ev.h_irr.p;
+  a.irr_h = ev.irr_h.p;
+  a.korder = ev.korder.p;
+  a.koff = ev.koff.p;
+  a.nplanes = ev.three_d ? ev.nz / 2 + 1 : 1;
+  PGB_CHECK(fft_factor(ev.nx, a.radix[0], &a.nst[0]) && fft_factor(ev.ny, a.radix[1], &a.nst[1]),
+            "mesh side with a prime factor above 13");
+  a.tab[0] = fft_roots<R>(ev.nx);
+  a.tab[1] = fft_roots<R>(ev.ny);
+  a.root = fft_roots<R>(fermi_mode(IN) ? 4 * ev.Nw : 2 * ev.Nw);
+  a.in = IN;
+  a.out = OUT;
+  bool small = true;  // no radix above 8
+  for (int x = 0; x < 2; ++x)
+    for (int s = 0; s < a.nst[x]; ++s) small = small && a.radix[x][s] <= 8 && a.radix[x][s] != 7;
+  const int rows = ev.three_d ? ev.ny : ev.ny / 2 + 1;
+  const size_t buf = ev.three_d ? (size_t)ev.ny * (ev.nx + 1)
+                                : std::max((size_t)rows * (ev.nx + 1), (size_t)ev.ny * (ev.nx / 2 + 1));
+  const size_t smem = 2 * buf * sizeof(cx<R>);
+  constexpr size_t lim = 200 * 1024;
+  const dim3 grid((unsigned)(ev.Nw * a.nplanes), (unsigned)narr);
+#define PGB_SPACE(IN_, OUT_, HALF_, N_)                                \
+  do {                                                                 \
+    PGB_SMEM_LIMIT_ONCE((k_space<R, IN_, OUT_, HALF_, N_>), lim);      \
+    k_space<R, IN_, OUT_, HALF_, N_><<<grid, 256, smem, st>>>(a);      \
+  } while (0)
+  // the sides of most meshes with their stages and index arithmetic at compile
+  // time; other sides choose stages and modes at run time, in a build that
+  // leaves out the large radices (128 instead of 250 registers) where it can
+  if (!ev.three_d && ev.nx == 64 && ev.ny == 64) PGB_SPACE(IN, OUT, true, 64);
+  else if (!ev.three_d && ev.nx == 32 && ev.ny == 32) PGB_SPACE(IN, OUT, true, 32);
+  else if (!ev.three_d && ev.nx == 16 && ev.ny == 16) PGB_SPACE(IN, OUT, true, 16);
+  else if (ev.three_d && small) PGB_SPACE(kInAny, kOutAny, false, 0);
+  else if (ev.three_d) PGB_SPACE(kInAny, kOutAny, false, -1);
+  else if (small) PGB_SPACE(kInAny, kOutAny, true, 0);
+  else PGB_SPACE(kInAny, kOutAny, true, -1);
+#undef PGB_SPACE
+  count_launch("even_space");
+}
+
+// The z axis of a 3-D mesh: each line pair (p, -p) of plane cells takes one
+// transform of the whole axis, whose upper half is the mirrored line; with
+// IN = post the halves of the time transform are taken apart on the load
+// (both cells are still real there), into another array.
+template <typename R, bool BIG>
+__global__ void __launch_bounds__(256) k_zaxis(SpaceArgs<R> a, const int2* pairs, int npairs, int nz, int nst,
+                                               SpaceArgs<R> rad, int lines) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  const int nch = (npairs + lines - 1) / lines;
+  const int b = blockIdx.x / nch, p0 = (blockIdx.x % nch) * lines, arr = blockIdx.y;
+  const int nl = min(lines, npairs - p0), half = nz / 2 + 1, nxy = a.nx * a.ny;
+  const int j = fermi_mode(a.in) ? fermi_slot(b, a.Nw) : boson_slot(b, a.Nw);
+  const cx<R> w = space_root<R>(a, a.in, j);
+  cx<R>* in = reinterpret_cast<cx<R>*>(smem_raw);
+  cx<R>* out = in + lines * nz;
+  for (int e = threadIdx.x; e < nl * nz; e += blockDim.x) {
+    const int z = e / nl, l = e - z * nl;
+    const int2 pp = pairs[p0 + l];
+    const int h = z < half ? pp.x + nxy * z : pp.y + nxy * (nz - z);
+    in[z * nl + l] = space_load<R, kInAny>(a, h, j, arr, w, (R)0);
+  }
+  __syncthreads();
+  plane_axis<R, BIG>(in, out, nz, nl, nl, 1, nst, rad.radix[0], a.sign, rad.tab[0]);
+  cx<R>* d = static_cast<cx<R>*>(a.dst) + (long long)arr * a.H * a.Nw + (long long)a.H * j;
+  for (int e = threadIdx.x; e < nl * half; e += blockDim.x) {
+    const int z = e / nl, l = e - z * nl;
+    const int2 pp = pairs[p0 + l];
+    d[pp.x + nxy * z] = in[z * nl + l];
+    if (pp.y != pp.x) d[pp.y + nxy * z] = in[(z ? nz - z : 0) * nl + l];
+  }
+}
+
+template <typename R, int IN>
+void zaxis_launch(const Even& ev, const cx<R>* src, cx<R>* dst, int narr, int sign, cudaStream_t st) {
+  SpaceArgs<R> a{}, rad{};
+  a.src = src;
+  a.dst = dst;
+  a.nx = ev.nx;
+  a.ny = ev.ny;
+  a.H = ev.H;
+  a.Nw = ev.Nw;
+  a.sign = sign;
+  a.root = fft_roots<R>(IN == kInPostFermi ? 4 * ev.Nw : 2 * ev.Nw);
+  a.in = IN;
+  PGB_CHECK(fft_factor(ev.nz, rad.radix[0], &rad.nst[0]), "mesh side with a prime factor above 13");
+  rad.tab[0] = fft_roots<R>(ev.nz);
+  const int lines = std::max(1, std::min(64, (int)(1536 / ev.nz)));
+  const int nch = (ev.nzp + lines - 1) / lines;
+  const size_t smem = 2 * (size_t)lines * ev.nz * sizeof(cx<R>);
+  bool small = true;
+  for (int s = 0; s < rad.nst[0]; ++s) small = small && rad.radix[0][s] <= 8 && rad.radix[0][s] != 7;
+  const dim3 grid((unsigned)(ev.Nw * nch), (unsigned)narr);
+  PGB_SMEM_LIMIT_ONCE((k_zaxis<R, false>), 64 * 1024);
+  PGB_SMEM_LIMIT_ONCE((k_zaxis<R, true>), 64 * 1024);
+  if (small) k_zaxis<R, false><<<grid, 256, smem, st>>>(a, ev.zpairs.p, ev.nzp, ev.nz, rad.nst[0], rad, lines);
+  else k_zaxis<R, true><<<grid, 256, smem, st>>>(a, ev.zpairs.p, ev.nzp, ev.nz, rad.nst[0], rad, lines);
+  count_launch("even_zaxis");
+}
+
+// forward transform of arrays that the load of IN makes from `src`
+template <typename R, int IN>
+void even_forward(const Even& ev, SpaceArgs<R> a, cx<R>* dst, int narr, bool time, cudaStream_t st) {
+  a.dst = dst;
+  space_launch<R, IN, kOutPlain>(ev, a, narr, -1, st);
+  if (ev.three_d) zaxis_launch<R, kInPlain>(ev, dst, dst, narr, -1, st);
+  if (time) fft_plan_t(ev.H, ev.Nw, (int)sizeof(cx<R>)).forward<R>(dst, narr, st);
+}
+// backward transform of T (overwritten); POST and OUT as in k_space
+template <typename R, int POST, int OUT>
+void even_backward(const Even& ev, SpaceArgs<R> a, cx<R>* T, cx<R>* T2, int narr, cudaStream_t st) {
+  fft_plan_t(ev.H, ev.Nw, (int)sizeof(cx<R>)).backward<R>(T, narr, st);
+  if (ev.three_d) {
+    zaxis_launch<R, POST>(ev, T, T2, narr, 1, st);
+    a.src = T2;
+    space_launch<R, kInPlain, OUT>(ev, a, narr, 1, st);
+  } else {
+    a.src = T;
+    space_launch<R, POST, OUT>(ev, a, narr, 1, st);
+  }
+}
+
+// ---------------------------------------------------------- pointwise stages
+// the half-integer phase of a transformed fermionic array: c *= e^{-i pi s/Nw}
+template <typename R>
+__global__ void k_even_phase(cx<R>* F, const cx<R>* root, const int* lt, int H, int Nw) {
+  MeshTau q;
+  if (!mesh_tau(H, Nw, q)) return;
+  cx<R>* f = F + (long long)blockIdx.y * H * Nw + q.r;
+  for (int p = q.t0; p < q.t1; ++p) f[(long long)H * p] = f[(long long)H * p] * twid<R>(root, lt[p], -1);
+}
+
+template <typename R>
+void fermi_transform(const Even& ev, SpaceArgs<R> a, cx<R>* F, int narr, bool bulk, cudaStream_t st) {
+  if (bulk) even_forward<R, kInFermi>(ev, a, F, narr, true, st);
+  else even_forward<R, kInFermi64>(ev, a, F, narr, true, st);
+  const FFT4D& ft = fft_plan_t(ev.H, ev.Nw, (int)sizeof(cx<R>));
+  k_even_phase<R><<<mesh_tau_grid(ev.H, ev.Nw, narr), 256, 0, st>>>(F, fft_roots<R>(2 * ev.Nw), ft.d_logical(3), ev.H,
+                                                                    ev.Nw);
+  count_launch("even_phase");
+}
+
+// The reference bubble's tau kernels on the half grid (k_ref_tau): element
+// (a <= b) at slots 2s and 2s+1 as the two parts of one number
+template <typename R, typename T>
+__global__ void k_even_ref_tau(cx<R>* A, cx<R>* B, const T* gp, const T* gm, const cx<T>* cf, const int* h_irr,
+                               const int* sym_el, int H, int Nk, int No, int Nw) {
+  MeshTau q;
+  if (!mesh_tau(H, Nw, q)) return;
+  const int k = h_irr[q.r];
+  const cx<T>* c = cf + ((long long)k * No * No + sym_el[blockIdx.y]) * No;
+  const long long o = (long long)blockIdx.y * H * Nw + q.r;
+  for (int s = q.t0; s < q.t1; ++s) {
+    T a[2] = {(T)0, (T)0}, b[2] = {(T)0, (T)0};
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+      for (int n = 0; n < No; ++n) {
+        const long long g = ((long long)(2 * s + h) * No + n) * Nk + k;
+        a[h] += gp[g] * c[n].x;
+        b[h] += gm[g] * c[n].x;
+      }
+    A[o + (long long)H * s] = cmk<R>((R)a[0], (R)a[1]);
+    B[o + (long long)H * s] = cmk<R>((R)b[0], (R)b[1]);
+  }
+}
+
+struct EvenPair {
+  int f13, f42;  // a <= b copies of G13 and G42
+};
+// chi0(r, tau) of the classes: G13(tau) G42(-tau) (both fermionic phases gone:
+// their product is -1, except at tau = 0), minus G0's, minus the analytic bubble
+template <typename R>
+__global__ void k_even_product(cx<R>* out, const cx<R>* F, const cx<R>* F0, const cx<R>* A, const cx<R>* B,
+                               const EvenPair* pairs, int H, int Nw, const int* pos, const int* lt, R sc, R sr) {
+  const EvenPair pr = pairs[blockIdx.y];
+  const long long P = (long long)H * Nw;
+  const cx<R>*a13 = F + pr.f13 * P, *b42 = F + pr.f42 * P;
+  cx<R>* o = out + (long long)blockIdx.y * P;
+  MeshTau q;
+  if (!mesh_tau(H, Nw, q)) return;
+  for (int p = q.t0; p < q.t1; ++p) {
+    const int s = lt[p];
+    const long long i = q.r + (long long)H * p, ie = q.r + (long long)H * pos[s ? Nw - s : 0],
+                    io = q.r + (long long)H * pos[Nw - 1 - s];
+    const cx<R> a = a13[i];
+    R vx = a.x * b42[ie].x, vy = a.y * b42[io].y;
+    if (F0) {
+      const cx<R> a0 = F0[pr.f13 * P + i];
+      vx = vx - a0.x * F0[pr.f42 * P + ie].x;
+      vy = vy - a0.y * F0[pr.f42 * P + io].y;
+    }
+    if (s == 0) vx = -vx;
+    vx = sc * vx;
+    vy = sc * vy;
+    if (A) {
+      const long long is = q.r + (long long)H * s;
+      const cx<R> ta = A[pr.f13 * P + is], tb = B[pr.f42 * P + is];
+      vx = vx - sr * (ta.x * tb.x);
+      vy = vy - sr * (ta.y * tb.y);
+    }
+    o[i] = cmk<R>(vx, vy);
+  }
+}
+
+struct EvenTerm {
+  int c, f;  // class of the vertex element, fermionic copy
+  int rev;   // bit 0: the vertex at the reversed tau, bit 1: the fermionic copy (antiperiodic)
+};
+// Fermionic outputs sum_t w_t(r, tau) g_t(r, tau) of real factors, with the
+// half-integer phase of the backward transform; the output runs fastest over the blocks, so
+// that the outputs of one tile of points share its w and g in L2
+template <typename R>
+__global__ void k_even_contract(cx<R>* out, const cx<R>* W, const cx<R>* F, const EvenTerm* terms, const int* tb,
+                                const cx<R>* root, int H, int Nw, const int* pos, const int* lt, int no) {
+  const int o = (int)(blockIdx.x % (unsigned)no);
+  const long long P = (long long)H * Nw;
+  const unsigned tile = blockIdx.x / (unsigned)no, nrb = (unsigned)((H + 255) / 256), rb = tile % nrb;
+  const int h = (int)(rb * 256u + threadIdx.x), p = (int)(tile / nrb);
+  if (h >= H) return;
+  const int s = lt[p];
+  const long long i = h + (long long)H * p, ie = h + (long long)H * pos[s ? Nw - s : 0],
+                  io = h + (long long)H * pos[Nw - 1 - s];
+  R x = (R)0, y = (R)0;
+  for (int t = tb[o]; t < tb[o + 1]; ++t) {
+    const EvenTerm m = terms[t];
+    const cx<R>* w = W + m.c * P;
+    cx<R> g;
+    if (m.rev & 2) {
+      g = cmk<R>(F[m.f * P + ie].x, -F[m.f * P + io].y);
+      if (s) g.x = -g.x;
+    } else {
+      g = F[m.f * P + i];
+    }
+    if (m.rev & 1) {
+      x = mad(w[ie].x, g.x, x);
+      y = mad(w[io].y, g.y, y);
+    } else {
+      const cx<R> v = w[i];
+      x = mad(v.x, g.x, x);
+      y = mad(v.y, g.y, y);
+    }
+  }
+  out[o * P + i] = cmk<R>(x, y) * twid<R>(root, s, 1);
+}
+
+// ------------------------------------------------------------------- vertex
+// Real-basis index tables.  vin, entry (row p, column q) at q N + p:
+// value = ca t[a] + cb t[b] with t[2 c + part] the parts of class c's matrix
+// element; word = a | b << 9 | (ca + 2) << 18 | (cb + 2) << 21.  vout, per class two
+// words (real, imaginary part): value = cf (sa v[a] + sb v[b]) over the result
+// v[q N + p]; word = a | b << 10 | (sa + 1) << 20 | (sb + 1) << 22 | (cf = 1/2) << 24.
+template <typename R> __device__ __forceinline__ R small_coef(int c) {  // -2 .. 2, exact
+  return c == 0 ? (R)0.f : (c == 1 ? (R)1.f : (c == 2 ? (R)2.f : (c == -1 ? (R)-1.f : (R)-2.f)));
+}
+
+__device__ __forceinline__ float real_mag(float a) { return fabsf(a); }
+__device__ __forceinline__ float real_mag(double a) { return (float)fabs(a); }
+__device__ __forceinline__ float real_mag(dfl a) { return fabsf(a.hi); }
+
+template <typename R> __host__ __device__ constexpr int rrow_pad() { return sizeof(R) == 4 ? 4 : 2; }
+template <typename R> __host__ __device__ constexpr int rrow_len(int n) { return (n + rrow_pad<R>() + 2) & ~3; }
+
+// Real warp_inverse_rot (flex.cu) of the group's matrix: lane i of a group of N
+// lanes holds row i.  The pivot row goes through shared memory with entry s at
+// s + pad - 1, so that entries 1.. start a 16-byte word.
+template <typename R, int N>
+__device__ __forceinline__ bool real_inverse_rot(R (&a)[N], R* prow, int* piv, int* pos, int& label, R& scale,
+                                                 int base, int i, bool act) {
+  constexpr int PAD = rrow_pad<R>(), PL = rrow_len<R>(N);
+  label = i;
+  scale = (R)0;
+  bool ok = true;
+#pragma unroll 1
+  for (int k = 0; k < N; ++k) {
+    const R ak = a[0];
+    unsigned best = 0u;
+    if (act && label >= k) {
+      best = (__float_as_uint(real_mag(ak)) & ~31u) | (unsigned)(31 - label);
+    }
+    // the largest key of the group: one redux for a whole warp, else windows
+    // of doubling width around the group (they may overlap: a maximum)
+    if constexpr (N > 16) {
+      best = __reduce_max_sync(0xffffffffu, best);
+    } else {
+#pragma unroll
+      for (int off = 1; off < N; off <<= 1) {
+        const int j = i + off;
+        best = max(best, __shfl_sync(0xffffffffu, best, base + (j < N ? j : j - N)));
+      }
+    }
+    const int plabel = 31 - (int)(best & 31u);
+    if (act && !(__uint_as_float(best & ~31u) > 0.f)) ok = false;
+    const bool is_piv = act && label == plabel;
+    if (label == k) label = plabel;
+    else if (is_piv) label = k;
+    if (act && i == 0) piv[k] = plabel;
+    R* buf = prow + (k & 1) * PL;
+    if (is_piv) {
+#pragma unroll
+      for (int s = 0; s < N; ++s) buf[s + PAD - 1] = a[s];
+    }
+    __syncwarp();
+    const R p = buf[PAD - 1];
+    const R ip = ok ? (R)1 / p : (R)0;
+    if (is_piv) scale = ip;
+    const R f = is_piv ? (R)0 : -(ak * ip);
+    if constexpr (sizeof(R) == 4) {
+      const float4* b4 = reinterpret_cast<const float4*>(buf + PAD);
+#pragma unroll
+      for (int s = 1; s < N; s += 4) {
+        const float4 v = b4[(s - 1) >> 2];
+        a[s - 1] = mad(f, v.x, a[s]);
+        if (s + 1 < N) a[s] = mad(f, v.y, a[s + 1]);
+        if (s + 2 < N) a[s + 1] = mad(f, v.z, a[s + 2]);
+        if (s + 3 < N) a[s + 2] = mad(f, v.w, a[s + 3]);
+      }
+    } else {
+#pragma unroll
+      for (int s = 1; s < N; ++s) a[s - 1] = mad(f, buf[s + PAD - 1], a[s]);
+    }
+    a[N - 1] = is_piv ? (R)1 : f;
+  }
+  __syncwarp();
+  if (act) {
+    int c = i;
+#pragma unroll 1
+    for (int k = N - 1; k >= 0; --k) {
+      const int p = piv[k];
+      if (c == k) c = p;
+      else if (c == p) c = k;
+    }
+    pos[i] = c;
+  }
+  __syncwarp();
+  return ok;
+}
+
+struct EvenVertexTabs {
+  const int *vin, *vout, *rep, *mem, *memcj, *nmem;
+  int ncls, nself, full;
+};
+
+// The FLEX vertex in the real basis.  A warp holds 32 / N matrices (one row per
+// lane), a CTA stages a tile of them through shared memory; the accumulator of
+// V is real.  consts: Si, Ci (inverses of S and C), D = S + C, S, C in the
+// basis, row-major; D is dense on the nself same-orbital pairs and diagonal
+// elsewhere.
+template <typename R, int N, int W>
+__global__ void __launch_bounds__(32 * W, sizeof(R) == 4 ? 4 : 2)
+    k_vertex_even(cx<R>* chi, long long nmat, long long estride, const R* consts, EvenVertexTabs tb, int mode,
+                  int* err) {
+  constexpr int G = 32 / N, T = W * G, TP = T + 1, PL = rrow_len<R>(N);
+  extern __shared__ __align__(16) unsigned char smraw[];
+  R* prow = reinterpret_cast<R*>(smraw);                    // [T][2][PL]
+  cx<R>* tile = reinterpret_cast<cx<R>*>(prow + (size_t)T * 2 * PL);  // [ncls][TP]
+  R* vb = reinterpret_cast<R*>(tile + (size_t)tb.ncls * TP);  // [T][N*N], entry (p, q) at q N + p
+  R* cs = vb + (size_t)T * N * N;                            // Si, Ci (column-major), then D row-major
+  int* vin = reinterpret_cast<int*>(cs + 3 * N * N);         // [N*N]
+  int* pv = vin + N * N;                                     // [T][N]
+  int* ps = pv + T * N;                                      // [T][N]
+  for (int e = threadIdx.x; e < N * N; e += blockDim.x) {
+    const int p = e % N, q = e / N;  // stored column-major for the row-per-lane reads
+    cs[e] = consts[p * N + q];
+    cs[N * N + e] = consts[N * N + p * N + q];
+    cs[2 * N * N + e] = consts[2 * N * N + e];
+    vin[e] = tb.vin[e];
+  }
+  const R* Sm = consts + 3 * N * N;
+  const R* Cm = consts + 4 * N * N;
+  const R* D = cs + 2 * N * N;
+  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int g = lane / N < G ? lane / N : 0;
+  const bool act = lane < G * N;
+  const int i = act ? lane - g * N : 0;
+  const int t = w * G + g;
+  R* pw = prow + (size_t)t * 2 * PL;
+  R* vw = vb + (size_t)t * N * N;
+  int *pvw = pv + t * N, *psw = ps + t * N;
+  const R c1 = mode == 2 ? (R)-0.5f : (R)1.5f;
+  const R c2 = mode == 0 ? (R)-0.5f : (R)0.5f;
+  const R* tr = reinterpret_cast<const R*>(tile);
+  for (long long m0 = (long long)blockIdx.x * T; m0 < nmat; m0 += (long long)gridDim.x * T) {
+    const int nt = (int)min((long long)T, nmat - m0);
+    __syncthreads();
+    for (int idx = threadIdx.x; idx < tb.ncls * T; idx += blockDim.x) {
+      const int tt = idx % T, e = idx / T;
+      // matrices past the end repeat the last one: every group has a regular matrix
+      tile[e * TP + tt] = chi[m0 + min(tt, nt - 1) + estride * tb.rep[e]];
+    }
+    __syncthreads();
+    R a[N];
+    auto entry = [&](int q) {
+      const int word = vin[q * N + i];
+      const int ia = word & 511, ib = (word >> 9) & 511;
+      const int ca = ((word >> 18) & 7) - 2, cb = ((word >> 21) & 7) - 2;
+      R v = tr[((ia >> 1) * TP + t) * 2 + (ia & 1)];
+      if (ca == -1) v = -v;
+      else if (ca == 2) v = v + v;
+      else if (ca == -2) v = -(v + v);
+      if (cb) {
+        const R u = tr[((ib >> 1) * TP + t) * 2 + (ib & 1)];
+        v = v + (cb > 0 ? u : -u);
+      }
+      return v;
+    };
+    int lab;
+    R sc;
+#pragma unroll
+    for (int q = 0; q < N; ++q) a[q] = cs[q * N + i] - entry(q);
+    bool ok = real_inverse_rot<R, N>(a, pw, pvw, psw, lab, sc, g * N, i, act);
+    if (act) {
+      const R s1 = c1 * sc;
+#pragma unroll
+      for (int q = 0; q < N; ++q) {
+        const int c = psw[q];
+        R v = s1 * a[q];
+        if (mode == 1) v = v - Sm[lab * N + c];
+        else if (mode == 2) v = v + (Sm[lab * N + c] - Cm[lab * N + c]);
+        vw[c * N + lab] = v;
+      }
+    }
+    __syncwarp();
+#pragma unroll
+    for (int q = 0; q < N; ++q) a[q] = cs[N * N + q * N + i] + entry(q);
+    ok &= real_inverse_rot<R, N>(a, pw, pvw, psw, lab, sc, g * N, i, act);
+    if (act) {
+      const R s2 = c2 * sc;
+#pragma unroll
+      for (int q = 0; q < N; ++q) {
+        const int c = psw[q];
+        vw[c * N + lab] = vw[c * N + lab] + s2 * a[q];
+      }
+    }
+    __syncwarp();
+    if (mode == 0) {
+      // -1/4 D X D: row i of X D, then D from the left
+      const int ns = tb.nself;
+#pragma unroll
+      for (int q = 0; q < N; ++q) a[q] = entry(q);
+      {
+        R head[N < 8 ? N : 8];
+        constexpr int NH = N < 8 ? N : 8;
+#pragma unroll
+        for (int q = 0; q < NH; ++q) head[q] = (R)0;
+#pragma unroll
+        for (int r = 0; r < NH; ++r)
+          if (r < ns) {
+#pragma unroll
+            for (int q = 0; q < NH; ++q)
+              if (q < ns) head[q] = mad(a[r], D[r * N + q], head[q]);
+          }
+#pragma unroll
+        for (int q = 0; q < N; ++q) {
+          if (q < NH && q < ns) a[q] = head[q < NH ? q : 0];
+          else a[q] = a[q] * D[q * N + q];
+        }
+      }
+      const R m4 = (R)-0.25f;
+      const R dl = m4 * D[i * N + i];
+#pragma unroll
+      for (int q = 0; q < N; ++q) {
+        R v = dl * a[q];
+        R sum = (R)0;
+        for (int r = 0; r < ns; ++r) {
+          const R o = shfl_idx(a[q], g * N + r);
+          sum = mad(m4 * D[i * N + r], o, sum);
+        }
+        if (i < ns) v = sum;
+        if (act) vw[q * N + i] = vw[q * N + i] + v;
+      }
+    }
+    if (!ok && act && t < nt) atomicExch(err, 3);
+    __syncthreads();
+    for (int idx = threadIdx.x; idx < tb.ncls * T; idx += blockDim.x) {
+      const int tt = idx % T, e = idx / T;
+      if (tt >= nt) continue;
+      const R* v = vb + (size_t)tt * N * N;
+      R part[2];
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const int word = tb.vout[2 * e + h];
+        const R x = v[word & 1023], y = v[(word >> 10) & 1023];
+        const int sa = ((word >> 20) & 3) - 1, sb = ((word >> 22) & 3) - 1;
+        R r = sa == 0 ? (R)0 : (sa > 0 ? x : -x);
+        if (sb) r = r + (sb > 0 ? y : -y);
+        if (word >> 24) r = (R)0.5f * r;
+        part[h] = r;
+      }
+      const cx<R> z = cmk<R>(part[0], part[1]);
+      const int n = tb.full ? tb.nmem[e] : 1;
+      for (int m = 0; m < n; ++m)
+        chi[m0 + tt + estride * tb.mem[4 * e + m]] = tb.memcj[4 * e + m] ? conj(z) : z;
+    }
+  }
+}
+
+template <typename R, int N>
+void vertex_even_launch(const Even& ev, cx<R>* chi, long long nmat, long long estride, const R* dc, int mode, bool full) {
+  constexpr int W = 8, T = W * (32 / N);
+  const int nc = (int)ev.cls.size();
+  const size_t smem = sizeof(R) * ((size_t)T * 2 * rrow_len<R>(N) + (size_t)T * N * N + 3 * N * N) +
+                      sizeof(cx<R>) * (size_t)nc * (T + 1) + sizeof(int) * (N * N + 2 * T * N);
+  PGB_SMEM_LIMIT_ONCE((k_vertex_even<R, N, W>), 220 * 1024);
+  EvenVertexTabs tb{ev.d_vin.p, ev.d_vout.p, ev.cls_el.p, ev.mem.p, ev.memcj.p, ev.nmem.p, nc, ev.nself, full ? 1 : 0};
+  const long long tiles = (nmat + T - 1) / T;
+  const long long blocks = std::min<long long>(tiles, (long long)ctx().num_sms * 16);
+  k_vertex_even<R, N, W><<<(unsigned)std::max(1LL, blocks), 32 * W, smem, ctx().stream>>>(chi, nmat, estride, dc, tb,
+                                                                                         mode, ctx().err);
+  count_launch("vertex_even");
+}
+
+template <typename To, typename From>
+__global__ void k_convert_el(cx<To>* out, const cx<From>* in, const int* el, long long K) {
+  const long long o = (long long)el[blockIdx.y] * K;
+  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < K; i += (long long)gridDim.x * blockDim.x)
+    cvt(out[o + i], in[o + i]);
+}
+
+}  // namespace
+
+template <typename To, typename From>
+void convert_even(const Even& ev, cx<To>* out, const cx<From>* in, long long K) {
+  const unsigned nb = (unsigned)std::min<long long>((K + 255) / 256, 1024);
+  k_convert_el<To, From><<<dim3(nb, (unsigned)ev.cls.size()), 256, 0, ctx().stream>>>(out, in, ev.cls_el.p, K);
+  count_launch("convert_even");
+}
+
+// arrays per batch: about 64 MB, so that a batch stays in L2 from the pointwise
+// kernel through the passes
+template <typename R> int even_batch(const Even& ev) {
+  const double bytes = (double)sizeof(cx<R>) * ev.H * ev.Nw;
+  return (int)std::max(1.0, std::min(65535.0, 64e6 / bytes));
+}
+
+template <typename R>
+void chi0_even(const Geom& g, const Pairs& p, const double2* G, double temp, const TailRef* tail, cx<R>* chi, bool full) {
+  const Even& ev = *g.even;
+  cudaStream_t st = ctx().stream;
+  const int ns = ev.nsym, No = g.Norb, H = ev.H, Nw = ev.Nw;
+  const size_t P = (size_t)H * Nw;
+  DBuf<int> sel(ns);
+  sel.upload(ev.sym_el.data(), ns);
+  DBuf<cx<R>> F(ns * P), F0, A, B, sawc, dJ;
+  SpaceArgs<R> a{};
+  a.Nk = g.Nk;
+  a.src = G;
+  a.el = sel.p;
+  fermi_transform<R>(ev, a, F.p, ns, false, st);
+  std::vector<cx<R>> hJ(ev.cls.size());
+  if (tail) {
+    DBuf<double2> G0((size_t)g.K * No * No);
+    green0(G0.p, tail->eig, tail->uni, tail->mu, temp, g.Nk, g.Nw, No);
+    F0.alloc(ns * P);
+    a.src = G0.p;
+    fermi_transform<R>(ev, a, F0.p, ns, false, st);
+    G0.release();
+    using T = typename std::conditional<std::is_same<R, float>::value, float, double>::type;
+    TailTables<T> tt;
+    tail_tables<T>(g, *tail, temp, tt);
+    A.alloc(ns * P);
+    B.alloc(ns * P);
+    k_even_ref_tau<R, T><<<mesh_tau_grid(H, Nw, ns), 256, 0, st>>>(A.p, B.p, tt.gp.p, tt.gm.p, tt.projectors(),
+                                                                  ev.h_irr.p, sel.p, H, g.Nk, No, Nw);
+    count_launch("even_ref_tau");
+    SpaceArgs<R> r{};
+    r.Nk = g.Nk;
+    for (DBuf<cx<R>>* x : {&A, &B}) {
+      r.src = x->p;
+      even_forward<R, kInPlain>(ev, r, x->p, ns, false, st);
+    }
+    const std::vector<double2> rb = tail_rhobar(g, *tail, tt.ff.p);
+    for (size_t c = 0; c < ev.cls.size(); ++c) {
+      const double2 J = tail_jump(p, rb, No, ev.cls[c].l, ev.cls[c].m);
+      hJ[c] = cmk<R>((R)J.x, (R)J.y);
+    }
+    dJ.alloc(hJ.size());
+    dJ.upload(hJ.data(), hJ.size());
+    sawc.alloc(g.Nw);
+    narrow<R>(sawc.p, tail_sawtooth(g, temp), g.Nw);
+  }
+  std::vector<EvenPair> hp(ev.cls.size());
+  for (size_t c = 0; c < hp.size(); ++c) {
+    const int l = ev.cls[c].l, m = ev.cls[c].m;
+    hp[c] = EvenPair{ev.sym_of[p.o1[l] + No * p.o1[m]], ev.sym_of[p.o2[m] + No * p.o2[l]]};
+  }
+  DBuf<EvenPair> dp(hp.size());
+  dp.upload(hp.data(), hp.size());
+  const int nc = (int)ev.cls.size();
+  const int ch = std::min(nc, even_batch<R>(ev));
+  DBuf<cx<R>> T(ch * P), T2;
+  if (ev.three_d) T2.alloc(ch * P);
+  const FFT4D& ft = fft_plan_t(H, Nw, (int)sizeof(cx<R>));
+  const double P4 = (double)g.P;
+  const R sc = (R)(temp / (double)g.Nkall / P4), sr = (R)(1.0 / (temp * (double)g.Nkall) / P4);
+  SpaceArgs<R> o{};
+  o.Nk = g.Nk;
+  o.dst = chi;
+  o.sawc = sawc.p;
+  o.full = full ? 1 : 0;
+  for (int c0 = 0; c0 < nc; c0 += ch) {
+    const int n = std::min(ch, nc - c0);
+    k_even_product<R><<<mesh_tau_grid(H, Nw, n), 256, 0, st>>>(T.p, F.p, F0.p, A.p, B.p, dp.p + c0, H, Nw, ft.d_pos(3),
+                                                               ft.d_logical(3), sc, sr);
+    count_launch("even_product");
+    o.mem = ev.mem.p + 4 * c0;
+    o.memcj = ev.memcj.p + 4 * c0;
+    o.nmem = ev.nmem.p + c0;
+    o.J = tail ? dJ.p + c0 : nullptr;
+    even_backward<R, kInPostBoson, kOutChi>(ev, o, T.p, T2.p, n, st);
+  }
+  sync();  // the host-built tables above go out of scope
+}
+
+// transforms of the classes' vertex elements V, static slots stat (host, per class)
+template <typename R>
+void vertex_transforms(const Geom& g, const cx<R>* V, const std::vector<R>& stat, cx<R>* W, cudaStream_t st) {
+  const Even& ev = *g.even;
+  const int nc = (int)ev.cls.size(), ch = even_batch<R>(ev);
+  const size_t P = (size_t)ev.H * ev.Nw;
+  DBuf<R> dstat(nc);
+  dstat.upload(stat.data(), nc);
+  SpaceArgs<R> b{};
+  b.Nk = g.Nk;
+  b.src = V;
+  for (int c0 = 0; c0 < nc; c0 += ch) {
+    b.el = ev.cls_el.p + c0;
+    b.stat = dstat.p + c0;
+    even_forward<R, kInBoson>(ev, b, W + c0 * P, std::min(ch, nc - c0), true, st);
+  }
+}
+
+template <typename R>
+void sigma_even(const Geom& g, const Pairs& p, const double2* G, const cx<R>* V, const double* S, const double* C,
+                double temp, double2* sig) {
+  const Even& ev = *g.even;
+  cudaStream_t st = ctx().stream;
+  const int ns = ev.nsym, No = g.Norb, Nchi = g.Nchi, H = ev.H, Nw = ev.Nw, nc = (int)ev.cls.size();
+  const size_t P = (size_t)H * Nw;
+  std::vector<double> hS(Nchi * Nchi), hC(Nchi * Nchi);
+  PGB_CUDA(cudaMemcpyAsync(hS.data(), S, sizeof(double) * hS.size(), cudaMemcpyDeviceToHost, st));
+  PGB_CUDA(cudaMemcpyAsync(hC.data(), C, sizeof(double) * hC.size(), cudaMemcpyDeviceToHost, st));
+  sync();
+  std::vector<R> stat(nc);
+  for (int c = 0; c < nc; ++c) stat[c] = (R)(1.5 * hS[ev.cls[c].el] - 0.5 * hC[ev.cls[c].el]);
+  std::vector<int> elt(ns), tb(1, 0);
+  std::vector<EvenTerm> terms;
+  for (int e = 0; e < ns; ++e) {
+    const int el = ev.sym_el[e];
+    elt[e] = el / No + No * (el % No);
+    for (const Term& t : p.sigma[el]) {
+      const int x = t.m + Nchi * t.l;
+      terms.push_back(EvenTerm{ev.cls_of[x], ev.sym_of[t.ef], ev.cj_of[x]});
+    }
+    tb.push_back((int)terms.size());
+  }
+  DBuf<int> sel(ns), delt(ns), dtb(tb.size());
+  DBuf<EvenTerm> dt(terms.size());
+  sel.upload(ev.sym_el.data(), ns);
+  delt.upload(elt.data(), ns);
+  dtb.upload(tb.data(), tb.size());
+  dt.upload(terms.data(), terms.size());
+  DBuf<cx<R>> F(ns * P), W((size_t)nc * P), T(ns * P), T2;
+  if (ev.three_d) T2.alloc(ns * P);
+  SpaceArgs<R> a{};
+  a.Nk = g.Nk;
+  a.src = G;
+  a.el = sel.p;
+  fermi_transform<R>(ev, a, F.p, ns, false, st);
+  vertex_transforms<R>(g, V, stat, W.p, st);
+  const FFT4D& ft = fft_plan_t(H, Nw, (int)sizeof(cx<R>));
+  const unsigned tiles = (unsigned)(((H + 255) / 256) * Nw);
+  k_even_contract<R><<<tiles * ns, 256, 0, st>>>(T.p, W.p, F.p, dt.p, dtb.p, fft_roots<R>(2 * Nw), H, Nw, ft.d_pos(3),
+                                                ft.d_logical(3), ns);
+  count_launch("even_contract");
+  SpaceArgs<R> o{};
+  o.Nk = g.Nk;
+  o.dst = sig;
+  o.el = sel.p;
+  o.elt = delt.p;
+  o.scale = temp / (double)g.Nkall / (double)g.P;
+  o.thresh = 1;
+  even_backward<R, kInPostFermi, kOutSigma>(ev, o, T.p, T2.p, ns, st);
+  sync();
+}
+
+template <typename R>
+void mkdelta_even(const Geom& g, const Pairs& p, const double2* F64, const cx<R>* Fbulk, const cx<R>* Vd,
+                  const double* S, const double* C, double scale, double2* out, DeltaKernelCache<R>& cache) {
+  const Even& ev = *g.even;
+  cudaStream_t st = ctx().stream;
+  const int ns = ev.nsym, No = g.Norb, Nchi = g.Nchi, H = ev.H, Nw = ev.Nw, nc = (int)ev.cls.size();
+  const size_t P = (size_t)H * Nw;
+  if (!cache.built) {
+    cache.built = true;
+    std::vector<double> hS(Nchi * Nchi), hC(Nchi * Nchi);
+    PGB_CUDA(cudaMemcpyAsync(hS.data(), S, sizeof(double) * hS.size(), cudaMemcpyDeviceToHost, st));
+    PGB_CUDA(cudaMemcpyAsync(hC.data(), C, sizeof(double) * hC.size(), cudaMemcpyDeviceToHost, st));
+    sync();
+    std::vector<R> stat(nc);
+    for (int c = 0; c < nc; ++c) stat[c] = (R)(0.5 * (hS[ev.cls[c].el] + hC[ev.cls[c].el]));
+    cache.W.alloc((size_t)nc * P);
+    vertex_transforms<R>(g, Vd, stat, cache.W.p, st);
+    std::vector<EvenTerm> terms;
+    std::vector<int> tb(1, 0), el;
+    for (int e = 0; e < No * No; ++e) {
+      if (p.delta[e].empty()) continue;
+      for (const Term& t : p.delta[e]) {
+        const int x = t.m + Nchi * t.l, a = t.ef % No, b = t.ef / No;
+        // F_ba = conj F_ab: the copy of a <= b at the reversed tau
+        terms.push_back(EvenTerm{ev.cls_of[x], ev.sym_of[t.ef], ev.cj_of[x] | (a > b ? 2 : 0)});
+      }
+      tb.push_back((int)terms.size());
+      el.push_back(e);
+    }
+    cache.out_elems = el;
+    cache.ef.alloc(3 * std::max<size_t>(1, terms.size()));
+    cache.ef.upload(terms.data(), 3 * terms.size());
+    cache.tb.alloc(tb.size());
+    cache.tb.upload(tb.data(), tb.size());
+    el.insert(el.end(), ev.sym_el.begin(), ev.sym_el.end());
+    cache.els.alloc(el.size());
+    cache.els.upload(el.data(), el.size());
+    sync();
+  }
+  const int no = (int)cache.out_elems.size();
+  DBuf<cx<R>> F(ns * P), T((size_t)std::max(1, no) * P), T2;
+  if (ev.three_d) T2.alloc((size_t)std::max(1, no) * P);
+  SpaceArgs<R> a{};
+  a.Nk = g.Nk;
+  a.src = Fbulk ? static_cast<const void*>(Fbulk) : F64;
+  a.el = cache.els.p + no;
+  fermi_transform<R>(ev, a, F.p, ns, Fbulk != nullptr, st);
+  PGB_CUDA(cudaMemsetAsync(out, 0, sizeof(double2) * (size_t)g.K * No * No, st));
+  if (no > 0) {
+    const FFT4D& ft = fft_plan_t(H, Nw, (int)sizeof(cx<R>));
+    const unsigned tiles = (unsigned)(((H + 255) / 256) * Nw);
+    k_even_contract<R><<<tiles * no, 256, 0, st>>>(T.p, cache.W.p, F.p, reinterpret_cast<const EvenTerm*>(cache.ef.p),
+                                                  cache.tb.p, fft_roots<R>(2 * Nw), H, Nw, ft.d_pos(3),
+                                                  ft.d_logical(3), no);
+    count_launch("even_contract");
+    SpaceArgs<R> o{};
+    o.Nk = g.Nk;
+    o.dst = out;
+    o.el = o.elt = cache.els.p;
+    o.scale = scale;
+    even_backward<R, kInPostFermi, kOutSigma>(ev, o, T.p, T2.p, no, st);
+  }
+  hermitize(out, g.K, No);
+}
+
+template <typename R>
+bool vertex_even(const Even& ev, cx<R>* chi, long long nmat, long long estride, int mode, bool full) {
+  const int n = (int)ev.perm.size();
+  std::vector<double> Si(ev.Sb), Ci(ev.Cb);
+  PGB_CHECK(host_inverse(Si, n) && host_inverse(Ci, n), "singular interaction matrix in the real-basis vertex");
+  std::vector<R> consts(5 * n * n);
+  for (int e = 0; e < n * n; ++e) {
+    consts[e] = (R)Si[e];
+    consts[n * n + e] = (R)Ci[e];
+    consts[2 * n * n + e] = (R)(ev.Sb[e] + ev.Cb[e]);
+    consts[3 * n * n + e] = (R)ev.Sb[e];
+    consts[4 * n * n + e] = (R)ev.Cb[e];
+  }
+  DBuf<R> dc(consts.size());
+  dc.upload(consts.data(), consts.size());
+  reset_err();
+  switch (n) {
+    case 1: vertex_even_launch<R, 1>(ev, chi, nmat, estride, dc.p, mode, full); break;
+    case 4: vertex_even_launch<R, 4>(ev, chi, nmat, estride, dc.p, mode, full); break;
+    case 9: vertex_even_launch<R, 9>(ev, chi, nmat, estride, dc.p, mode, full); break;
+    case 16: vertex_even_launch<R, 16>(ev, chi, nmat, estride, dc.p, mode, full); break;
+    case 25: vertex_even_launch<R, 25>(ev, chi, nmat, estride, dc.p, mode, full); break;
+    default: throw Error("no real-basis vertex for this number of orbital pairs");
+  }
+  return fetch_err() == 0;
+}
+
+#define PGB_EVEN_INST(R)                                                                                              \
+  template void chi0_even<R>(const Geom&, const Pairs&, const double2*, double, const TailRef*, cx<R>*, bool);         \
+  template void sigma_even<R>(const Geom&, const Pairs&, const double2*, const cx<R>*, const double*, const double*,   \
+                              double, double2*);                                                                      \
+  template void mkdelta_even<R>(const Geom&, const Pairs&, const double2*, const cx<R>*, const cx<R>*, const double*,  \
+                                const double*, double, double2*, DeltaKernelCache<R>&);                               \
+  template bool vertex_even<R>(const Even&, cx<R>*, long long, long long, int, bool);
+
+}  // namespace pgb

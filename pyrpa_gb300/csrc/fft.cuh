@@ -98,7 +98,8 @@ class FFT4D {
  public:
   FFT4D() = default;
   // tune: per-axis overrides (null: the heuristics)
-  FFT4D(int nx, int ny, int nz, int nt, int elem_bytes, const PlanTune* tune = nullptr);
+  // t_only: the passes of the t axis alone (x, y and z are left as they are)
+  FFT4D(int nx, int ny, int nz, int nt, int elem_bytes, const PlanTune* tune = nullptr, bool t_only = false);
   // frees the device position tables (plans made for timing only)
   void release_tables();
   long long P() const { return P_; }
@@ -132,6 +133,19 @@ class FFT4D {
 // timing the candidates of fft_axis_candidates on a scratch array (one axis
 // at a time, the others fixed at their best so far).
 const FFT4D& fft_plan(int nx, int ny, int nz, int nt, int elem_bytes);
+
+// Cached plan of the t axis alone over `lines` adjacent lines (element stride
+// `lines`); d_pos(3) and the other tables of axis 3 apply.
+const FFT4D& fft_plan_t(int lines, int nt, int elem_bytes);
+
+// Device table of the roots exp(-2 pi i t / n), t < n, in the type of the
+// transforms (cached for the process), and the Stockham radices of a length
+// (false: a prime factor above 13).
+template <typename R> const cx<R>* fft_roots(int n);
+template <> const double2* fft_roots<double>(int n);
+template <> const float2* fft_roots<float>(int n);
+template <> const cdf* fft_roots<dfl>(int n);
+bool fft_factor(int n, int* radix, int* nst);
 
 // Optional live timing of every FFT pass launch with CUDA events on the
 // launching stream: launches, summed milliseconds and algorithmic bytes

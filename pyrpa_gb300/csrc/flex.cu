@@ -8,26 +8,14 @@
 #include <string>
 #include <type_traits>
 
+#include "even.cuh"
 #include "flex.cuh"
+#include "flex_dev.cuh"
 #include "linalg.cuh"
 
 namespace pgb {
 
 namespace {
-constexpr double kPi = 3.141592653589793238462643383279;
-constexpr double kThresh = 1.0e-9;  // small-part zeroing of chi0 and Sigma (fchi.f90:483-506)
-
-__host__ __device__ __forceinline__ long long fidx(long long k, long long j, long long a, long long b,
-                                                   long long Nk, long long Nw, long long n) {
-  return k + Nk * (j + Nw * (a + n * b));
-}
-
-template <typename T> __device__ __forceinline__ T thresh(T v) {
-  if (fabs((double)v.x) < kThresh) v.x = 0;
-  if (fabs((double)v.y) < kThresh) v.y = 0;
-  return v;
-}
-
 // Device error flags, one slot per context: a kernel that finds a singular
 // matrix or an unconverged eigenvalue iteration writes its code to the slot
 // its launch was given (ctx().err), and the host reads it after the stage
@@ -40,33 +28,6 @@ int* err_slot_address(int slot) {
   PGB_CUDA(cudaGetSymbolAddress(&p, g_err_slots));
   return static_cast<int*>(p) + slot;
 }
-
-namespace {
-
-// every launch of a flag-raising kernel follows a reset_err on its context
-void reset_err() {
-  PGB_CHECK(ctx().err != nullptr, "the engine context is not set up (no device error flag)");
-  PGB_CUDA(cudaMemsetAsync(ctx().err, 0, sizeof(int), ctx().stream));
-}
-int fetch_err() {
-  int e = 0;
-  PGB_CUDA(cudaMemcpyAsync(&e, ctx().err, sizeof(int), cudaMemcpyDeviceToHost, ctx().stream));
-  sync();
-  return e;
-}
-
-inline void count_launch(const char* what) {
-  launch_check(what);
-  ctx().kernel_launches++;
-}
-
-inline unsigned grid_1d(long long n, int threads, long long cap = 1LL << 30) {
-  long long b = (n + threads - 1) / threads;
-  if (b < 1) b = 1;
-  if (b > cap) b = cap;
-  return (unsigned)b;
-}
-}  // namespace
 
 void log(const char* fmt, ...) {
   if (!ctx().verbose) return;
@@ -366,33 +327,6 @@ bool invert_blocks(double2* G, long long nmat, int Norb, long long stride_mat, l
                                                                          stride_el, ctx().err);
   count_launch("invert_blocks");
   return fetch_err() == 0;
-}
-
-// ====================================================== mesh x time grids ==
-// Kernels over a padded array of P = Nkall x M points (mesh point r fastest)
-// give each thread one mesh point r and up to kTauChunk consecutive slices t
-// (blocks of 256 threads: the mesh in blocks, then the slices in chunks).
-// The mesh index is split once per thread in 32-bit arithmetic, and the
-// per-point tables (grid_irr, grid_flag, reversed indices) are read once;
-// a grid-stride loop over P would split every element's index with 64-bit
-// divisions, which on GB300 cost far more than the element's own loads.
-constexpr int kTauChunk = 8;
-
-dim3 mesh_tau_grid(long long Nkall, long long M, unsigned ny, int chunk = kTauChunk) {
-  const long long nrb = (Nkall + 255) / 256, nch = (M + chunk - 1) / chunk;
-  return dim3((unsigned)(nrb * nch), ny);
-}
-
-struct MeshTau {
-  int r, t0, t1;
-};
-__device__ __forceinline__ bool mesh_tau(long long Nkall, long long M, MeshTau& q, int chunk = kTauChunk) {
-  const unsigned nrb = (unsigned)((Nkall + 255) / 256);
-  const unsigned rb = blockIdx.x % nrb, tc = blockIdx.x / nrb;
-  q.r = (int)(rb * 256u + threadIdx.x);
-  q.t0 = (int)tc * chunk;
-  q.t1 = min((int)M, q.t0 + chunk);
-  return q.r < Nkall;
 }
 
 // ========================================================== padded grids ==
@@ -742,6 +676,63 @@ __global__ void k_sawc(double2* sawc, int Nw, int M, double temp) {
   sawc[j] = v;
 }
 
+// ---- parts of the analytic reference bubble shared with the even-model form
+template <typename T> void tail_tables(const Geom& g, const TailRef& tail, double temp, TailTables<T>& tt) {
+  const int No2 = g.Norb * g.Norb;
+  const size_t nt = (size_t)g.Nk * g.Norb * g.M, ncf = (size_t)g.Nk * g.Norb * No2;
+  tt.gp.alloc(nt);
+  tt.gm.alloc(nt);
+  tt.ff.alloc((size_t)g.Nk * g.Norb);
+  k_gpm<T><<<mesh_tau_grid((long long)g.Nk * g.Norb, g.M, 1), 256, 0, ctx().stream>>>(
+      tt.gp.p, tt.gm.p, tt.ff.p, tail.eig, tail.mu, temp, g.Nk, g.Norb, (int)g.M);
+  count_launch("gpm");
+  tt.cf64.alloc(ncf);
+  band_projectors(tt.cf64.p, tail.uni, g.Nk, g.Norb);
+  if constexpr (std::is_same<T, float>::value) {
+    tt.cf32.alloc(ncf);
+    convert<float, double>(tt.cf32.p, tt.cf64.p, (long long)ncf);
+  }
+}
+template void tail_tables<float>(const Geom&, const TailRef&, double, TailTables<float>&);
+template void tail_tables<double>(const Geom&, const TailRef&, double, TailTables<double>&);
+
+std::vector<double2> tail_rhobar(const Geom& g, const TailRef& tail, const double* ff) {
+  const int No2 = g.Norb * g.Norb;
+  DBuf<double2> rb(No2);
+  k_rhobar<<<No2, 256, 0, ctx().stream>>>(rb.p, tail.uni, ff, g.grid_irr.p, g.grid_flag.p, g.Nkall, g.Norb);
+  count_launch("rhobar");
+  std::vector<double2> h(No2);
+  rb.download(h.data(), No2);
+  sync();
+  return h;
+}
+
+// tau = 0 jump coefficient of pair (l,m) (fchi.f90:836-844)
+double2 tail_jump(const Pairs& p, const std::vector<double2>& rb, int Norb, int l, int m) {
+  const int a13 = p.o1[l], b13 = p.o1[m], a42 = p.o2[m], b42 = p.o2[l];
+  double2 J = make_double2(0, 0);
+  if (a13 == b13) J = J + rb[a42 + Norb * b42];
+  if (a42 == b42) J = J - rb[a13 + Norb * b13];
+  return J;
+}
+
+// the sawtooth transform depends on (Nw, T) only: computed once per pair
+const double2* tail_sawtooth(const Geom& g, double temp) {
+  static std::map<std::pair<int, double>, DBuf<double2>*> cache;
+  static std::mutex mu;
+  cudaStream_t st = ctx().stream;
+  std::lock_guard<std::mutex> lk(mu);
+  DBuf<double2>*& e = cache[std::make_pair(g.Nw, temp)];
+  if (!e) {
+    e = new DBuf<double2>(g.Nw);
+    k_sawc<<<grid_1d(g.Nw, 128), 128, 0, st>>>(e->p, g.Nw, (int)g.M, temp);
+    count_launch("sawc");
+    // complete before another thread's stream reads the cached entry
+    PGB_CUDA(cudaStreamSynchronize(st));
+  }
+  return e->p;
+}
+
 // PYRPA_GB_CHI0_SWAP=0 computes every exchange class with its own transform
 bool chi0_swap_enabled() {
   const char* s = std::getenv("PYRPA_GB_CHI0_SWAP");
@@ -749,7 +740,11 @@ bool chi0_swap_enabled() {
 }
 
 template <typename R>
-void chi0(const Geom& g, const Pairs& p, const double2* G, double temp, const TailRef* tail, cx<R>* chi) {
+void chi0(const Geom& g, const Pairs& p, const double2* G, double temp, const TailRef* tail, cx<R>* chi, bool full) {
+  if (g.even) {
+    chi0_even<R>(g, p, G, temp, tail, chi, full);
+    return;
+  }
   cudaStream_t st = ctx().stream;
   const FFT4D& fft = fft_plan(g.Nx, g.Ny, g.Nz, (int)g.M, (int)sizeof(cx<R>));
   const int No2 = g.Norb * g.Norb;
@@ -801,66 +796,23 @@ void chi0(const Geom& g, const Pairs& p, const double2* G, double temp, const Ta
     // the tau reference in FP32 for an FP32 chi0 (its rounding is below the
     // FP32 transforms'), in FP64 for the wider types
     using T = typename std::conditional<std::is_same<R, float>::value, float, double>::type;
-    DBuf<T> gp((size_t)g.Nk * g.Norb * g.M), gm((size_t)g.Nk * g.Norb * g.M);
-    DBuf<double> ff((size_t)g.Nk * g.Norb);
-    k_gpm<T><<<mesh_tau_grid((long long)g.Nk * g.Norb, g.M, 1), 256, 0, st>>>(
-        gp.p, gm.p, ff.p, tail->eig, tail->mu, temp, g.Nk, g.Norb, (int)g.M);
-    count_launch("gpm");
-    const size_t ncf = (size_t)g.Nk * g.Norb * No2;
-    DBuf<double2> cf64(ncf);
-    band_projectors(cf64.p, tail->uni, g.Nk, g.Norb);
-    DBuf<cx<float>> cf32;
-    const cx<T>* cf = nullptr;
-    if constexpr (std::is_same<T, float>::value) {
-      cf32.alloc(ncf);
-      convert<float, double>(cf32.p, cf64.p, (long long)ncf);
-      cf = cf32.p;
-    } else {
-      cf = cf64.p;
-    }
+    TailTables<T> tt;
+    tail_tables<T>(g, *tail, temp, tt);
     A.alloc((size_t)No2 * g.P);
     B.alloc((size_t)No2 * g.P);
-    k_ref_tau<R, T><<<mesh_tau_grid(g.Nkall, g.M, No2), 256, 0, st>>>(A.p, B.p, gp.p, gm.p, cf, g.grid_irr.p, g.grid_flag.p, g.Nkall,
+    k_ref_tau<R, T><<<mesh_tau_grid(g.Nkall, g.M, No2), 256, 0, st>>>(A.p, B.p, tt.gp.p, tt.gm.p, tt.projectors(), g.grid_irr.p, g.grid_flag.p, g.Nkall,
                                          g.Nk, g.Norb, (int)g.M, g.P);
     count_launch("ref_tau");
     fft.forward_space<R>(A.p, No2, st);
     fft.forward_space<R>(B.p, No2, st);
-    DBuf<double2> rb(No2);
-    k_rhobar<<<No2, 256, 0, st>>>(rb.p, tail->uni, ff.p, g.grid_irr.p, g.grid_flag.p, g.Nkall, g.Norb);
-    count_launch("rhobar");
-    std::vector<double2> hrb(No2);
-    rb.download(hrb.data(), No2);
-    sync();
-    auto RB = [&](int m, int l) { return hrb[m + g.Norb * l]; };
-    auto Jof = [&](int l, int m) {  // tau = 0 jump coefficient of pair (l,m) (fchi.f90:836-844)
-      const int a13 = p.o1[l], b13 = p.o1[m], a42 = p.o2[m], b42 = p.o2[l];
-      double2 J = make_double2(0, 0);
-      if (a13 == b13) J = J + RB(a42, b42);
-      if (a42 == b42) J = J - RB(a13, b13);
-      return J;
-    };
+    const std::vector<double2> hrb = tail_rhobar(g, *tail, tt.ff.p);
+    auto Jof = [&](int l, int m) { return tail_jump(p, hrb, g.Norb, l, m); };
     for (auto& c : hp) {
       c.J = Jof(c.l, c.m);
       if (c.has_d) c.dJ = Jof(c.dl, c.dm);
     }
-    // the sawtooth transform depends on (Nw, T) only: computed once per pair
-    static std::map<std::pair<int, double>, DBuf<double2>*> sawc_cache;
-    static std::mutex sawc_mu;
-    const double2* sawc64 = nullptr;
-    {
-      std::lock_guard<std::mutex> lk(sawc_mu);
-      DBuf<double2>*& e = sawc_cache[std::make_pair(g.Nw, temp)];
-      if (!e) {
-        e = new DBuf<double2>(g.Nw);
-        k_sawc<<<grid_1d(g.Nw, 128), 128, 0, st>>>(e->p, g.Nw, (int)g.M, temp);
-        count_launch("sawc");
-        // complete before another thread's stream reads the cached entry
-        PGB_CUDA(cudaStreamSynchronize(st));
-      }
-      sawc64 = e->p;
-    }
     sawc.alloc(g.Nw);
-    narrow<R>(sawc.p, sawc64, g.Nw);
+    narrow<R>(sawc.p, tail_sawtooth(g, temp), g.Nw);
   }
   {  // keep only the transforms that are computed
     std::vector<ChiDev> kept;
@@ -1606,35 +1558,6 @@ template <typename R, int N, int W> size_t vertex_vs_smem() {
 template <typename R, int N, int W> size_t vertex_reg_smem() {
   return (sizeof(R) * 5 * N * N + 15) / 16 * 16 + sizeof(cx<R>) * ((size_t)N * N * (2 * W + 1) + (size_t)W * N * N) +
          sizeof(int) * (W * (N + 1) + W * 32);
-}
-
-// host inverse of a small real matrix (row-major), false if (nearly) singular
-bool host_inverse(std::vector<double>& A, int n) {
-  std::vector<int> piv(n);
-  double amax = 0;
-  for (double v : A) amax = std::max(amax, std::fabs(v));
-  for (int k = 0; k < n; ++k) {
-    int p = k;
-    for (int r = k + 1; r < n; ++r)
-      if (std::fabs(A[r * n + k]) > std::fabs(A[p * n + k])) p = r;
-    piv[k] = p;
-    if (std::fabs(A[p * n + k]) <= 1e-12 * std::max(amax, 1e-300)) return false;
-    if (p != k)
-      for (int j = 0; j < n; ++j) std::swap(A[k * n + j], A[p * n + j]);
-    const double d = 1.0 / A[k * n + k];
-    A[k * n + k] = 1.0;
-    for (int j = 0; j < n; ++j) A[k * n + j] *= d;
-    for (int r = 0; r < n; ++r) {
-      if (r == k) continue;
-      const double f = A[r * n + k];
-      A[r * n + k] = 0.0;
-      for (int j = 0; j < n; ++j) A[r * n + j] -= f * A[k * n + j];
-    }
-  }
-  for (int k = n - 1; k >= 0; --k)
-    if (piv[k] != k)
-      for (int r = 0; r < n; ++r) std::swap(A[r * n + k], A[r * n + piv[k]]);
-  return true;
 }
 
 template <typename R, int N>
@@ -2452,6 +2375,10 @@ __global__ void k_contract_mirror(cx<R>* T0, cx<R>* T1, const cx<R>* W, const cx
 template <typename R>
 void sigma(const Geom& g, const Pairs& p, const double2* G, const cx<R>* V, const double* S, const double* C,
            double temp, double2* sig) {
+  if (g.even) {
+    sigma_even<R>(g, p, G, V, S, C, temp, sig);
+    return;
+  }
   cudaStream_t st = ctx().stream;
   const FFT4D& fft = fft_plan(g.Nx, g.Ny, g.Nz, (int)g.M, (int)sizeof(cx<R>));
   const FFT4D& fft3 = fft_plan(g.Nx, g.Ny, g.Nz, 1, (int)sizeof(cx<R>));
@@ -2963,7 +2890,12 @@ void hermitize(double2* D, long long K, int Norb) {
 template <typename R>
 void mkdelta(const Geom& g, const Pairs& p, const double2* F, const cx<R>* Vd, const double* S, const double* C,
              const double* prt, bool singlet, double scale, double2* out, DeltaKernelCache<R>* cache,
-             const cx<R>* Fbulk) {
+             const cx<R>* Fbulk, bool even) {
+  if (even) {
+    DeltaKernelCache<R> own;
+    mkdelta_even<R>(g, p, F, Fbulk, Vd, S, C, scale, out, cache ? *cache : own);
+    return;
+  }
   cudaStream_t st = ctx().stream;
   const FFT4D& fft = fft_plan(g.Nx, g.Ny, g.Nz, (int)g.M, (int)sizeof(cx<R>));
   const int No2 = g.Norb * g.Norb;
@@ -3176,16 +3108,6 @@ template <typename R> void narrow(cx<R>* out, const double2* in, long long n) {
   count_launch("narrow");
 }
 
-// conversions between bulk types (double-float <-> float without the FP64 pipe)
-__device__ __forceinline__ void cvt(float2& o, float2 v) { o = v; }
-__device__ __forceinline__ void cvt(double2& o, double2 v) { o = v; }
-__device__ __forceinline__ void cvt(cdf& o, cdf v) { o = v; }
-__device__ __forceinline__ void cvt(float2& o, double2 v) { o = make_float2((float)v.x, (float)v.y); }
-__device__ __forceinline__ void cvt(double2& o, float2 v) { o = make_double2(v.x, v.y); }
-__device__ __forceinline__ void cvt(cdf& o, float2 v) { o = mkc(dfl(v.x), dfl(v.y)); }
-__device__ __forceinline__ void cvt(float2& o, cdf v) { o = make_float2(v.x.hi + v.x.lo, v.y.hi + v.y.lo); }
-__device__ __forceinline__ void cvt(cdf& o, double2 v) { o = mkc(dfl(v.x), dfl(v.y)); }
-__device__ __forceinline__ void cvt(double2& o, cdf v) { o = make_double2((double)v.x, (double)v.y); }
 template <typename To, typename From>
 __global__ void k_convert(cx<To>* out, const cx<From>* in, long long n) {
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
@@ -3204,7 +3126,7 @@ template void convert<double, float>(double2*, const float2*, long long);
 
 // ======================================================== instantiations ==
 #define PGB_INST(R)                                                                                        \
-  template void chi0<R>(const Geom&, const Pairs&, const double2*, double, const TailRef*, cx<R>*);        \
+  template void chi0<R>(const Geom&, const Pairs&, const double2*, double, const TailRef*, cx<R>*, bool);        \
   template void stoner<R>(const Geom&, const cx<R>*, const double*, const double*, double*, double*, int*, \
                           int*);                                                                           \
   template bool vertex<R>(cx<R>*, long long, long long, int, const double*, const double*, int);          \
@@ -3213,13 +3135,13 @@ template void convert<double, float>(double2*, const float2*, long long);
                          const double*, double, double2*);                                                 \
   template void mkdelta<R>(const Geom&, const Pairs&, const double2*, const cx<R>*, const double*,         \
                            const double*, const double*, bool, double, double2*, DeltaKernelCache<R>*,     \
-                           const cx<R>*);                                                                  \
+                           const cx<R>*, bool);                                                            \
   template void widen<R>(double2*, const cx<R>*, long long);                                               \
   template void narrow<R>(cx<R>*, const double2*, long long);
 PGB_INST(float)
 PGB_INST(double)
 // double-float bulk: the FFT convolution stages and the conversions around them
-template void chi0<dfl>(const Geom&, const Pairs&, const double2*, double, const TailRef*, cx<dfl>*);
+template void chi0<dfl>(const Geom&, const Pairs&, const double2*, double, const TailRef*, cx<dfl>*, bool);
 template void stoner<dfl>(const Geom&, const cx<dfl>*, const double*, const double*, double*, double*, int*, int*);
 template void scale_chi<dfl>(cx<dfl>*, long long, double);
 template void sigma<dfl>(const Geom&, const Pairs&, const double2*, const cx<dfl>*, const double*, const double*,
@@ -3227,7 +3149,7 @@ template void sigma<dfl>(const Geom&, const Pairs&, const double2*, const cx<dfl
 template void widen<dfl>(double2*, const cx<dfl>*, long long);
 template void narrow<dfl>(cx<dfl>*, const double2*, long long);
 template void mkdelta<dfl>(const Geom&, const Pairs&, const double2*, const cx<dfl>*, const double*, const double*,
-                           const double*, bool, double, double2*, DeltaKernelCache<dfl>*, const cx<dfl>*);
+                           const double*, bool, double, double2*, DeltaKernelCache<dfl>*, const cx<dfl>*, bool);
 template bool vertex<dfl>(cx<dfl>*, long long, long long, int, const double*, const double*, int);
 
 }  // namespace pgb

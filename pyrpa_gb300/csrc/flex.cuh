@@ -11,6 +11,7 @@
 #pragma once
 
 #include <cstdint>
+#include <memory>
 #include <vector>
 
 #include "common.cuh"
@@ -28,8 +29,13 @@ struct SpinMap {
   int on;
 };
 
+struct Even;  // even.cuh
+
 struct Geom {
   SpinMap spin;
+  // set by the stage drivers when G (and what is made from it) is known to be
+  // symmetric in its orbitals on every k point: the stages take their even form
+  std::shared_ptr<Even> even;
   int Nx = 1, Ny = 1, Nz = 1, Nw = 1, Nk = 1, Norb = 1, Nchi = 1;
   long long Nkall = 1, M = 2, P = 2, K = 1;
   std::vector<int> h_grid_irr, h_grid_flag, h_irr_grid;
@@ -94,10 +100,28 @@ struct TailRef {
 };
 
 // chi0 by FFT convolution (fchi.f90:508-635), optionally tail-corrected
-// (fchi.f90:637-892).  chi (Nk,Nw,Nchi,Nchi) of type cx<R> is overwritten.
+// (fchi.f90:637-892).  chi (Nk,Nw,Nchi,Nchi) of type cx<R> is overwritten; an
+// even model (g.even) with full = false gets only its class representatives,
+// and every element at nu = 0.
 template <typename R>
 void chi0(const Geom& g, const Pairs& p, const double2* G, double temp, const TailRef* tail,
-          cx<R>* chi);
+          cx<R>* chi, bool full = true);
+// tables of the analytic reference bubble: tau kernels gp, gm and Fermi
+// factors of the bands, band projectors (FP32 for an FP32 chi0)
+template <typename T> struct TailTables {
+  DBuf<T> gp, gm;
+  DBuf<double> ff;
+  DBuf<double2> cf64;
+  DBuf<cx<float>> cf32;
+  const cx<T>* projectors() const {
+    if constexpr (sizeof(T) == 4) return cf32.p;
+    else return cf64.p;
+  }
+};
+template <typename T> void tail_tables(const Geom& g, const TailRef& tail, double temp, TailTables<T>& tt);
+std::vector<double2> tail_rhobar(const Geom& g, const TailRef& tail, const double* ff);
+double2 tail_jump(const Pairs& p, const std::vector<double2>& rb, int Norb, int l, int m);
+const double2* tail_sawtooth(const Geom& g, double temp);
 // Stoner factors: max Re eig(chi0(q,0) S) and of -chi0(q,0) C (fchi.f90:352-399)
 template <typename R>
 void stoner(const Geom& g, const cx<R>* chi, const double* S, const double* C, double* sdw,
@@ -136,13 +160,14 @@ template <typename R> struct DeltaKernelCache {
   // and the first term of each (device)
   std::vector<int> out_elems;
   DBuf<int> ef, tb;
+  DBuf<int> els;  // even form: output elements, then the a <= b elements of F
 };
 // Fbulk: F already in the bulk type (then F is not read; the parity factors
-// prt must be +-1)
+// prt must be +-1).  even: the even form applies to F (mkdelta_even)
 template <typename R>
 void mkdelta(const Geom& g, const Pairs& p, const double2* F, const cx<R>* Vd, const double* S,
              const double* C, const double* prt, bool singlet, double scale, double2* out,
-             DeltaKernelCache<R>* cache, const cx<R>* Fbulk = nullptr);
+             DeltaKernelCache<R>* cache, const cx<R>* Fbulk = nullptr, bool even = false);
 // F = -(G Delta) G^H in double-float (Norb <= 5; false otherwise)
 bool mkfk_df(cdf* F, const cdf* G, const double2* D, long long K, int Norb);
 void hermitize(double2* D, long long K, int Norb);
