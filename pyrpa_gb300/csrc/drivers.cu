@@ -557,7 +557,7 @@ void mkself_core(Inputs& in, const FlexParams& a, double2* sig_out, double* mu_o
   std::vector<double> Bc((size_t)a.m_diis * a.m_diis, 0.0);
   // mu bracket cache
   bool bracket_valid = false;
-  double muS_cache = 0, muL_cache = 0;
+  double muS_cache = 0, muL_cache = 0, cp_center = 0;
   DBuf<double> partmax(1024), dmax(1);
 
   auto compare_sigma = [&]() {
@@ -605,102 +605,21 @@ void mkself_core(Inputs& in, const FlexParams& a, double2* sig_out, double* mu_o
     log("esterr=%9.2E\n", esterr);
   };
 
-  auto get_rn = [&](double rmu) { return filling_cp(eg.p, eig.p, Nk, Nw, Norb, rmu, a.temp); };
-
+  bool cp_current = false;  // eg holds the coefficients of the present sig
   auto renew_mu = [&]() {
-    charpoly_gk(eg.p, H.p, sig.p, Nk, Nw, Norb);
-    const double eps = (esterr > 1.0e-2) ? 1.0e-8 : esterr * 1.0e-1;
-    double dmu = std::fabs(mu - mu_old) * 2.0;
-    if (dmu < eps * 4.0) dmu = eps * 4.0;
-    mu_old = mu;
-    const double fill = a.fill;
-    double muS = 0, muL = 0, rnS = 0, rnL = 0;
-    bool found = false;
-    if (bracket_valid) {
-      rnS = get_rn(muS_cache);
-      rnL = get_rn(muL_cache);
-      if (rnS < fill && rnL > fill) {
-        muS = muS_cache;
-        muL = muL_cache;
-        found = true;
-        log("[mu] cached bracket valid\n");
-      } else {
-        log("[mu] cached bracket invalid, re-searching\n");
-      }
+    if (!cp_current) {
+      cp_center = mu;
+      charpoly_gk(eg.p, H.p, sig.p, cp_center, a.temp, Nk, Nw, Norb);
+      cp_current = true;
     }
-    if (!found) {
-      muL = mu + dmu;
-      muS = mu - dmu;
-      for (int it = 1; it <= 100; ++it) {
-        mu = muL;
-        rnL = get_rn(mu);
-        if (rnL < fill) {
-          if (std::fabs(fill - rnL) > 0.5) muL += 1.0;
-          else if (std::fabs(fill - rnL) > dmu) muL += 0.5;
-          else muL += dmu;
-        } else {
-          break;
-        }
-        PGB_CHECK(it < 100, "Too many");
-      }
-      for (int it = 1; it <= 100; ++it) {
-        mu = muS;
-        rnS = get_rn(mu);
-        if (rnS > fill) {
-          if (std::fabs(rnS - fill) > 0.5) muS -= 1.0;
-          else if (std::fabs(rnS - fill) > dmu) muS -= 0.5;
-          else muS -= dmu;
-        } else {
-          break;
-        }
-        PGB_CHECK(it < 100, "Too many");
-      }
-    }
-    muS_cache = muS;
-    muL_cache = muL;
+    MuState s{mu, mu_old, muS_cache, muL_cache, bracket_valid ? 1 : 0, 0, 0.0, 0};
+    mu_search(s, eg.p, cp_center, eig.p, a.fill, esterr, a.temp, Nk, Nw, Norb);
+    if (s.cached) log(s.cached == 1 ? "[mu] cached bracket valid\n" : "[mu] cached bracket invalid, re-searching\n");
+    mu = mu_old = s.mu;
+    muS_cache = s.muS;
+    muL_cache = s.muL;
     bracket_valid = true;
-    rnL -= fill;
-    rnS -= fill;
-    double rnc = rnS, muc = muS, mud = 0.0, muM = 0.0, rnM = 0.0;
-    bool flag = false;
-    // inverse quadratic interpolation / bisection hybrid (fself.f90:623-654)
-    for (int it = 1; it <= 100; ++it) {
-      if (rnc != rnS && rnc != rnL)
-        muM = (muL * rnS * rnc * (rnS - rnc) + muS * rnL * rnc * (rnc - rnL) + muc * rnL * rnS * (rnL - rnS)) /
-              ((rnL - rnS) * (rnc - rnL) * (rnc - rnS));
-      else
-        muM = muL - rnL * (muL - muS) / (rnL - rnS);
-      if ((0.25 * (3.0 * muS + muL) > muM || muM > muL) || (flag && std::fabs(muM - muL) >= std::fabs(muL - muc) * 0.5) ||
-          (!flag && std::fabs(muM - muL) >= std::fabs(muc - mud) * 0.5) || (flag && std::fabs(muL - muc) < 1.0e-8) ||
-          (!flag && std::fabs(muc - mud) < 1.0e-8)) {
-        muM = (muL + muS) * 0.5;
-        flag = true;
-      } else {
-        flag = false;
-      }
-      if (std::fabs(muL - muM) < eps) break;
-      mu = muM;
-      rnM = get_rn(muM);
-      mud = muc;
-      muc = muL;
-      rnc = rnL;
-      if (rnS * (rnM - fill) < 0) {
-        muL = muM;
-        rnL = rnM - fill;
-      } else {
-        muS = muM;
-        rnS = rnM - fill;
-      }
-      if (std::fabs(rnS) < std::fabs(rnL)) {
-        std::swap(muL, muS);
-        std::swap(rnL, rnS);
-      }
-      PGB_CHECK(it < 100, "Too many loop!");
-    }
-    mu = (rnL == rnS) ? (muS + muL) * 0.5 : (muS * rnL - muL * rnS) / (rnL - rnS);
-    rnM = get_rn(mu);
-    mu_old = mu;
-    log("mu  =%8.4f filling =%8.4f\n", mu, rnM);
+    log("mu  =%8.4f filling =%8.4f\n", mu, s.filling);
   };
 
   Timer tm;
@@ -733,6 +652,7 @@ void mkself_core(Inputs& in, const FlexParams& a, double2* sig_out, double* mu_o
   int judged = 0;  // iterations of the mixed schedule's judging phase
   for (it = 1; it <= a.scf_loop; ++it) {
     log("iter=%5d\n", it);
+    cp_current = false;
     maxchi0s = flex_bulk(in, a, G.p, mu, prec_of(phase), bufs, sig.p);
     tm.start();
     if (a.sub_sigma > 0) hf_subtract(sig.p, Nk, Nw, Norb, (int)a.sub_sigma);
@@ -792,6 +712,7 @@ void mkself_core(Inputs& in, const FlexParams& a, double2* sig_out, double* mu_o
       tm.start();
       PGB_CHECK(dyson(G.p, sig.p, H.p, mu, a.temp, Nk, Nw, Norb), "singular G^-1 in the Dyson step");
       g_stats.t_dyson += tm.stop();
+      cp_current = false;
       maxchi0s = flex_bulk(in, a, G.p, mu, prec_of(2), bufs, sig.p);
       if (a.sub_sigma > 0) hf_subtract(sig.p, Nk, Nw, Norb, (int)a.sub_sigma);
       g_stats.stoner = maxchi0s;

@@ -141,12 +141,22 @@ void hf_subtract(double2* sig, int Nk, int Nw, int Norb, int mode);
 // reductions (deterministic two-level)
 double dot_re(const double2* a, const double2* b, long long n);
 double2 inner_w(const double2* a, const double2* b, const double* kw, int Nk, long long n);
-double filling(const double2* eig_g, const double* eig, int Nk, int Nw, int Norb, double mu,
-               double temp);
-bool eig_gkinv(double2* eig_g, const double2* hamk, const double2* sig, int Nk, int Nw, int Norb);
-// coefficients of det(z - H - Sigma) per (k, iw) and the filling from them
-void charpoly_gk(double2* cp, const double2* hamk, const double2* sig, int Nk, int Nw, int Norb);
-double filling_cp(const double2* cp, const double* eig, int Nk, int Nw, int Norb, double mu, double temp);
+// The chemical-potential search of the FLEX loop (fself.f90:544-687).
+// charpoly_gk: coefficients of det(mu + i w_j - H - Sigma) in mu - center, per
+// (k, j): N arrays of Nk Nw.  mu_search: the bracketing and the inverse
+// quadratic / bisection search on them, all on the device.
+struct MuState {
+  double mu, mu_old;            // in: current and previous mu; out: the new one (both)
+  double muS, muL;              // bracket kept between searches
+  int bracket_valid;
+  int cached;                   // out: 1 kept bracket valid, 2 invalid and searched again
+  double filling;               // out: filling at mu
+  int err;                      // out: 1 no bracket, 2 no convergence, 3 a block gave up a wait
+};
+void charpoly_gk(double2* cp, const double2* hamk, const double2* sig, double center, double temp, int Nk, int Nw,
+                 int Norb);
+void mu_search(MuState& s, const double2* cp, double center, const double* eig, double fill, double esterr, double temp,
+               int Nk, int Nw, int Norb);
 
 // Eliashberg
 void mkfk(double2* F, const double2* G, const double2* D, long long K, int Norb);
