@@ -474,8 +474,10 @@ double chi0_entry(double2* chi_out, const double* Smat, const double* Cmat, cons
   // the even form for a symmetric G (and bands); a caller's own pair maps
   // keep the general one
   if (!irr_chi && !chi_map && (!tail || symmetric_bands(eig, uni, Nk, (int)Norb)) &&
-      symmetric_blocks(G.p, g.K, (int)Norb, 1.0e-12))
-    g.even = make_even(g, p, nullptr, nullptr, (int)sizeof(cx<R>));
+      symmetric_blocks(G.p, g.K, (int)Norb, 1.0e-12)) {
+    if (with_stoner) g.even = make_even(g, p, Smat, Cmat, (int)sizeof(cx<R>));
+    if (!g.even) g.even = make_even(g, p, nullptr, nullptr, (int)sizeof(cx<R>));
+  }
   chi0<R>(g, p, G.p, temp, tail ? &tr : nullptr, chi.p);
   G.release();
   double sdw = 0;

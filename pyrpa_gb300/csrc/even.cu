@@ -61,53 +61,12 @@ void build_classes(Even& ev, int n) {
     }
 }
 
-// The real basis: same-orbital pairs, then the sums, then i times the
-// differences, of the pairs (a,b), (b,a) with the smaller index first.  With
-// rows e_l, e_l + e_Pl, i (e_l - e_Pl) and the inverse's columns e_l,
-// (e_l + e_Pl)/2, -i (e_l - e_Pl)/2 all coefficients are 1, 2 or 1/2.
-void build_vertex(Even& ev, int n, const double* S, const double* C) {
-  struct B { int kind, l; };
-  std::vector<B> basis;
-  std::vector<int> idx[3];
-  for (int k = 0; k < 3; ++k) {
-    idx[k].assign(n, -1);
-    for (int l = 0; l < n; ++l) {
-      const bool self = ev.perm[l] == l;
-      if ((k == 0) != self || (k > 0 && l > ev.perm[l])) continue;
-      idx[k][l] = (int)basis.size();
-      if (k > 0) idx[k][ev.perm[l]] = (int)basis.size();
-      basis.push_back({k, l});
-    }
-    if (k == 0) ev.nself = (int)basis.size();
-  }
-  // S and C
-  auto to_basis = [&](const double* X, std::vector<double>& out) {
-    out.assign((size_t)n * n, 0.0);
-    auto x = [&](int a, int b) { return X[a + n * b]; };
-    for (int p = 0; p < n; ++p)
-      for (int q = 0; q < n; ++q) {
-        const B r = basis[p], c = basis[q];
-        const int l = r.l, pl = ev.perm[l], m = c.l, pm = ev.perm[m];
-        double v = 0;
-        if (r.kind == 0 && c.kind == 0) v = x(l, m);
-        else if (r.kind == 0 && c.kind == 1) v = 0.5 * (x(l, m) + x(l, pm));
-        else if (r.kind == 1 && c.kind == 0) v = x(l, m) + x(pl, m);
-        else if (r.kind == 1 && c.kind == 1) v = 0.5 * (x(l, m) + x(l, pm) + x(pl, m) + x(pl, pm));
-        else if (r.kind == 2 && c.kind == 2) v = 0.5 * (x(l, m) - x(l, pm) - x(pl, m) + x(pl, pm));
-        out[(size_t)p * n + q] = v;
-      }
-  };
-  to_basis(S, ev.Sb);
-  to_basis(C, ev.Cb);
-  std::vector<double> si(ev.Sb), ci(ev.Cb);
-  const bool size_ok = n == 1 || n == 4 || n == 9 || n == 16 || n == 25;
-  bool sparse = ev.nself <= 8;
-  for (int p = 0; p < n; ++p)
-    for (int q = 0; q < n; ++q)
-      if (p != q && (p >= ev.nself || q >= ev.nself) && ev.Sb[(size_t)p * n + q] + ev.Cb[(size_t)p * n + q] != 0.0)
-        sparse = false;
-  ev.vertex_ok = size_ok && sparse && host_inverse(si, n) && host_inverse(ci, n);
-  if (!ev.vertex_ok) return;
+struct RealBasis {
+  int kind, l;  // 0 same orbital, 1 sum, 2 i times the difference; the pair of smaller index
+};
+
+// index tables of the real basis: its matrix from the class representatives (vin) and back (vout)
+void build_index(Even& ev, int n, const std::vector<RealBasis>& basis, const std::vector<int>* idx) {
   auto src = [&](int row, int col, int part, int* sign) {  // part of element (row, col) of the vertex matrix
     const int x = row + n * col;
     *sign = (part && ev.cj_of[x]) ? -1 : 1;
@@ -116,7 +75,7 @@ void build_vertex(Even& ev, int n, const double* S, const double* C) {
   ev.vin.assign((size_t)n * n, 0);
   for (int p = 0; p < n; ++p)
     for (int q = 0; q < n; ++q) {
-      const B r = basis[p], c = basis[q];
+      const RealBasis r = basis[p], c = basis[q];
       const int l = r.l, m = c.l, pm = ev.perm[m];
       const bool im = (r.kind == 2) != (c.kind == 2);
       int ca = 1, cb = 0, s = 1;
@@ -162,6 +121,82 @@ void build_vertex(Even& ev, int n, const double* S, const double* C) {
     for (int h = 0; h < 2; ++h)
       ev.vout.push_back(a[h] | b[h] << 10 | (sa[h] + 1) << 20 | (sb[h] + 1) << 22 | half << 24);
   }
+}
+
+// The real basis: same-orbital pairs, then the sums, then i times the
+// differences, of the pairs (a,b), (b,a) with the smaller index first.  With
+// rows e_l, e_l + e_Pl, i (e_l - e_Pl) and the inverse's columns e_l,
+// (e_l + e_Pl)/2, -i (e_l - e_Pl)/2 all coefficients are 1, 2 or 1/2.
+void build_vertex(Even& ev, int n, const double* S, const double* C) {
+  std::vector<RealBasis> basis;
+  std::vector<int> idx[3];
+  for (int k = 0; k < 3; ++k) {
+    idx[k].assign(n, -1);
+    for (int l = 0; l < n; ++l) {
+      const bool self = ev.perm[l] == l;
+      if ((k == 0) != self || (k > 0 && l > ev.perm[l])) continue;
+      idx[k][l] = (int)basis.size();
+      if (k > 0) idx[k][ev.perm[l]] = (int)basis.size();
+      basis.push_back({k, l});
+    }
+    if (k == 0) ev.nself = (int)basis.size();
+    if (k == 1) ev.nplus = (int)basis.size();
+  }
+  // S and C
+  auto to_basis = [&](const double* X, std::vector<double>& out) {
+    out.assign((size_t)n * n, 0.0);
+    auto x = [&](int a, int b) { return X[a + n * b]; };
+    for (int p = 0; p < n; ++p)
+      for (int q = 0; q < n; ++q) {
+        const RealBasis r = basis[p], c = basis[q];
+        const int l = r.l, pl = ev.perm[l], m = c.l, pm = ev.perm[m];
+        double v = 0;
+        if (r.kind == 0 && c.kind == 0) v = x(l, m);
+        else if (r.kind == 0 && c.kind == 1) v = 0.5 * (x(l, m) + x(l, pm));
+        else if (r.kind == 1 && c.kind == 0) v = x(l, m) + x(pl, m);
+        else if (r.kind == 1 && c.kind == 1) v = 0.5 * (x(l, m) + x(l, pm) + x(pl, m) + x(pl, pm));
+        else if (r.kind == 2 && c.kind == 2) v = 0.5 * (x(l, m) - x(l, pm) - x(pl, m) + x(pl, pm));
+        out[(size_t)p * n + q] = v;
+      }
+  };
+  to_basis(S, ev.Sb);
+  to_basis(C, ev.Cb);
+  build_index(ev, n, basis, idx);
+  // Cholesky factors (lower) of S's blocks in the orthonormal basis
+  std::vector<double> R((size_t)n * n, 0.0);
+  ev.stoner_ok = n <= 32;
+  for (int blk = 0; blk < 2 && ev.stoner_ok; ++blk) {
+    const int i0 = blk ? ev.nplus : 0, i1 = blk ? n : ev.nplus;
+    for (int p = i0; p < i1 && ev.stoner_ok; ++p)
+      for (int q = i0; q <= p; ++q) {
+        // e_l against (e_l + e_Pl) / sqrt 2
+        const double sc = (p < ev.nself) == (q < ev.nself) ? 1.0 : (p < ev.nself ? std::sqrt(2.0) : std::sqrt(0.5));
+        double v = sc * ev.Sb[(size_t)p * n + q];
+        for (int k = i0; k < q; ++k) v -= R[(size_t)p * n + k] * R[(size_t)q * n + k];
+        if (p == q) {
+          if (!(v > 1e-10 * std::fabs(ev.Sb[(size_t)p * n + p]))) {
+            ev.stoner_ok = false;
+            break;
+          }
+          R[(size_t)p * n + p] = std::sqrt(v);
+        } else {
+          R[(size_t)p * n + q] = v / R[(size_t)q * n + q];
+        }
+      }
+  }
+  if (ev.stoner_ok) {
+    ev.d_schol.alloc(R.size());
+    ev.d_schol.upload(R.data(), R.size());
+    sync();
+  }
+  std::vector<double> si(ev.Sb), ci(ev.Cb);
+  const bool size_ok = n == 1 || n == 4 || n == 9 || n == 16 || n == 25;
+  bool sparse = ev.nself <= 8;
+  for (int p = 0; p < n; ++p)
+    for (int q = 0; q < n; ++q)
+      if (p != q && (p >= ev.nself || q >= ev.nself) && ev.Sb[(size_t)p * n + q] + ev.Cb[(size_t)p * n + q] != 0.0)
+        sparse = false;
+  ev.vertex_ok = size_ok && sparse && host_inverse(si, n) && host_inverse(ci, n);
 }
 
 __device__ __forceinline__ void max_bits(unsigned long long* out, double v) {
@@ -323,7 +358,7 @@ std::shared_ptr<Even> make_even(const Geom& g, const Pairs& p, const double* S, 
   put(ev->mem, mem);
   put(ev->memcj, cj);
   put(ev->nmem, nm);
-  if (ev->vertex_ok) {
+  if (S && C) {
     put(ev->d_vin, ev->vin);
     put(ev->d_vout, ev->vout);
   }

@@ -63,7 +63,9 @@ struct Even {
   bool vertex_ok = false;           // the real-basis vertex applies (constants in vs/vc)
   std::vector<double> Sb, Cb;       // S and C in the real basis, row-major
   std::vector<int> vin, vout;       // index tables of the real basis (see even_impl.cuh)
-  int nself = 0;
+  int nself = 0, nplus = 0;         // same-orbital pairs; pairs in the first (even) block at nu = 0
+  bool stoner_ok = false;           // S positive definite: Cholesky factors of its two blocks in d_schol
+  DBuf<double> d_schol;
   DBuf<int> d_vin, d_vout;
 };
 
@@ -100,6 +102,9 @@ void mkdelta_even(const Geom& g, const Pairs& p, const double2* F64, const cx<R>
                   const double* S, const double* C, double scale, double2* out, DeltaKernelCache<R>& cache);
 template <typename R>
 bool vertex_even(const Even& ev, cx<R>* chi, long long nmat, long long estride, int mode, bool full);
+// largest eigenvalue of chi0(q,0) S per irreducible q, into out (host, Nk)
+template <typename R>
+bool stoner_even(const Geom& g, const cx<R>* chi, std::vector<double>& out);
 // out = in between bulk types on the class representatives
 template <typename To, typename From>
 void convert_even(const Even& ev, cx<To>* out, const cx<From>* in, long long K);

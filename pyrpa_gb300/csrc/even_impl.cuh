@@ -720,6 +720,145 @@ void vertex_even_launch(const Even& ev, cx<R>* chi, long long nmat, long long es
   count_launch("vertex_even");
 }
 
+// ------------------------------------------------------------------- stoner
+// Largest eigenvalue of chi0(q, 0) S.  At nu = 0 the real-basis matrix X is
+// symmetric and splits into two blocks (the sums with the same-orbital pairs,
+// and the differences); with S = L L^T the eigenvalues of X S are those of
+// K = L^T X L.  One warp per (q, block) reduces K to tridiagonal form
+// (Householder) and finds its largest eigenvalue by 32-fold section with Sturm
+// counts, all in FP64 and without a QR iteration.  514 q points of five
+// orbitals take 0.25 ms against 7.4 ms for k_stoner's complex FP64 QR of X S and -X C.
+constexpr int kEvenStonerWarps = 4;
+__device__ __forceinline__ double wsum(double v) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  return v;
+}
+template <typename R>
+__global__ void __launch_bounds__(32 * kEvenStonerWarps) k_stoner_even(double* out, const cx<R>* chi, const int* vin,
+                                                                       const int* rep, const double* L, int Nk,
+                                                                       long long K, int n, int nself, int nplus,
+                                                                       int mx, int* err) {
+  extern __shared__ __align__(16) unsigned char smraw[];
+  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31, ld = mx + 1;
+  double* A = reinterpret_cast<double*>(smraw) + (size_t)w * (mx * ld + 3 * 32);
+  double *d = A + mx * ld, *e2 = d + 32, *v = e2 + 32;
+  const int t = blockIdx.x * kEvenStonerWarps + w;
+  if (t >= 2 * Nk) return;
+  const int k = t % Nk, blk = t / Nk, i0 = blk ? nplus : 0, m = blk ? n - nplus : nplus;
+  if (m == 0) {
+    if (lane == 0) out[t] = -1.0e300;
+    return;
+  }
+  auto part = [&](int s) {
+    const cx<R> c = chi[rep[s >> 1] * K + k];
+    return (double)((s & 1) ? c.y : c.x);
+  };
+  // row `lane` of X L, then of L^T (X L)
+  if (lane < m) {
+    for (int q = 0; q < m; ++q) {
+      const int word = vin[(i0 + q) * n + i0 + lane];
+      const int ca = ((word >> 18) & 7) - 2, cb = ((word >> 21) & 7) - 2;
+      double x = ca * part(word & 511);
+      if (cb) x += cb * part((word >> 9) & 511);
+      const bool a = i0 + lane < nself, b = i0 + q < nself;
+      if (a != b) x *= a ? 1.4142135623730951 : 0.70710678118654752;
+      A[lane * ld + q] = x;
+    }
+  }
+  __syncwarp();
+  double row[32];
+  if (lane < m)
+    for (int q = 0; q < m; ++q) {
+      double s = 0.0;
+      for (int r = q; r < m; ++r) s = fma(A[lane * ld + r], L[(i0 + r) * n + i0 + q], s);
+      row[q] = s;
+    }
+  __syncwarp();
+  if (lane < m)
+    for (int q = 0; q < m; ++q) A[lane * ld + q] = row[q];
+  __syncwarp();
+  if (lane < m)
+    for (int q = 0; q < m; ++q) {
+      double s = 0.0;
+      for (int r = lane; r < m; ++r) s = fma(L[(i0 + r) * n + i0 + lane], A[r * ld + q], s);
+      row[q] = s;
+    }
+  __syncwarp();
+  if (lane < m)
+    for (int q = 0; q < m; ++q) A[lane * ld + q] = row[q];
+  __syncwarp();
+  // tridiagonal form: A <- H A H, H = I - sc v v^T
+  for (int c = 0; c + 2 < m; ++c) {
+    const double x = (lane > c && lane < m) ? A[lane * ld + c] : 0.0;
+    const double tail = wsum(lane > c + 1 ? x * x : 0.0);
+    if (tail == 0.0) continue;
+    const double x0 = __shfl_sync(0xffffffffu, x, c + 1);
+    const double nrm = sqrt(fma(x0, x0, tail)), al = x0 > 0 ? -nrm : nrm;
+    const double vl = lane == c + 1 ? x0 - al : x;
+    v[lane] = vl;
+    __syncwarp();
+    const double sc = 2.0 / wsum(vl * vl);
+    double p = 0.0;
+    if (lane < m)
+      for (int q = c + 1; q < m; ++q) p = fma(A[lane * ld + q], v[q], p);
+    p *= sc;
+    const double h = 0.5 * sc * wsum(p * vl);
+    const double u = p - h * vl;
+    d[lane] = u;  // scratch
+    __syncwarp();
+    if (lane < m)
+      for (int q = c; q < m; ++q) {
+        const double vq = q > c ? v[q] : 0.0;
+        A[lane * ld + q] = A[lane * ld + q] - (vl * d[q] + u * vq);
+      }
+    __syncwarp();
+    if (lane > c && lane < m) A[c * ld + lane] = A[lane * ld + c];
+    __syncwarp();
+  }
+  double dl = 0.0, el = 0.0;
+  if (lane < m) dl = A[lane * ld + lane];
+  if (lane + 1 < m) el = A[lane * ld + lane + 1];
+  __syncwarp();
+  d[lane] = dl;
+  e2[lane] = el * el;
+  __syncwarp();
+  // Gershgorin interval
+  const double below = __shfl_up_sync(0xffffffffu, fabs(el), 1);
+  const double rad = fabs(el) + (lane > 0 ? below : 0.0);
+  double hi = lane < m ? dl + rad : -1e300, lo = lane < m ? dl : -1e300, ref = lane < m ? fabs(dl) + rad : 0.0;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    hi = fmax(hi, __shfl_xor_sync(0xffffffffu, hi, o));
+    lo = fmax(lo, __shfl_xor_sync(0xffffffffu, lo, o));  // the largest diagonal entry bounds it from below
+    ref = fmax(ref, __shfl_xor_sync(0xffffffffu, ref, o));
+  }
+  const double tol = 4.4e-16 * ref;
+  const bool bad = wsum(lane < m ? dl + el : 0.0) * 0.0 != 0.0;  // a NaN or an infinity in K
+  for (int it = 0; it < 64 && !bad && hi - lo > tol; ++it) {
+    // lane's point, and whether an eigenvalue lies above it: some pivot of T - x is not negative
+    const double x = lo + (hi - lo) * ((lane + 1) * (1.0 / 33.0));
+    double q = d[0] - x;
+    bool above = q > 0.0;
+    for (int i = 1; i < m; ++i) {
+      if (q == 0.0) q = -1e-300;
+      q = d[i] - x - e2[i - 1] / q;
+      above |= q > 0.0;
+    }
+    const unsigned ab = __ballot_sync(0xffffffffu, above);
+    const int na = ab ? 32 - __clz(ab) : 0;  // points 0 .. na-1 have one above
+    const double nlo = na ? __shfl_sync(0xffffffffu, x, na - 1) : lo;
+    const double nhi = na < 32 ? __shfl_sync(0xffffffffu, x, na) : hi;
+    if (!(nhi < hi || nlo > lo)) break;
+    lo = nlo;
+    hi = nhi;
+  }
+  if (lane == 0) {
+    if (bad) atomicExch(err, 2);
+    out[t] = 0.5 * (lo + hi);
+  }
+}
+
 template <typename To, typename From>
 __global__ void k_convert_el(cx<To>* out, const cx<From>* in, const int* el, long long K) {
   const long long o = (long long)el[blockIdx.y] * K;
@@ -986,12 +1125,33 @@ bool vertex_even(const Even& ev, cx<R>* chi, long long nmat, long long estride, 
   return fetch_err() == 0;
 }
 
+template <typename R>
+bool stoner_even(const Geom& g, const cx<R>* chi, std::vector<double>& out) {
+  const Even& ev = *g.even;
+  const int n = g.Nchi, mx = std::max(ev.nplus, n - ev.nplus);
+  DBuf<double> d(2 * (size_t)g.Nk);
+  reset_err();
+  const size_t smem = (size_t)kEvenStonerWarps * (mx * (mx + 1) + 3 * 32) * sizeof(double);
+  PGB_SMEM_LIMIT_ONCE(k_stoner_even<R>, 64 * 1024);
+  const unsigned blocks = (unsigned)((2LL * g.Nk + kEvenStonerWarps - 1) / kEvenStonerWarps);
+  k_stoner_even<R><<<blocks, 32 * kEvenStonerWarps, smem, ctx().stream>>>(
+      d.p, chi, ev.d_vin.p, ev.cls_el.p, ev.d_schol.p, g.Nk, g.K, n, ev.nself, ev.nplus, mx, ctx().err);
+  count_launch("stoner_even");
+  std::vector<double> h(2 * (size_t)g.Nk);
+  d.download(h.data(), h.size());
+  const bool ok = fetch_err() == 0;
+  out.resize(g.Nk);
+  for (int k = 0; k < g.Nk; ++k) out[k] = std::max(h[k], h[g.Nk + k]);
+  return ok;
+}
+
 #define PGB_EVEN_INST(R)                                                                                              \
   template void chi0_even<R>(const Geom&, const Pairs&, const double2*, double, const TailRef*, cx<R>*, bool);         \
   template void sigma_even<R>(const Geom&, const Pairs&, const double2*, const cx<R>*, const double*, const double*,   \
                               double, double2*);                                                                      \
   template void mkdelta_even<R>(const Geom&, const Pairs&, const double2*, const cx<R>*, const cx<R>*, const double*,  \
                                 const double*, double, double2*, DeltaKernelCache<R>&);                               \
-  template bool vertex_even<R>(const Even&, cx<R>*, long long, long long, int, bool);
+  template bool vertex_even<R>(const Even&, cx<R>*, long long, long long, int, bool);                                 \
+  template bool stoner_even<R>(const Geom&, const cx<R>*, std::vector<double>&);
 
 }  // namespace pgb

@@ -1029,6 +1029,17 @@ template <typename R>
 void stoner(const Geom& g, const cx<R>* chi, const double* S, const double* C, double* sdw, double* cdw,
             int* q_sdw, int* q_cdw) {
   std::vector<double> h;
+  // even models: a symmetric problem for chi0 S; the charge factor is only
+  // printed, so it is computed (below, with the other) when something prints
+  if (g.even && g.even->stoner_ok && !ctx().verbose) {
+    PGB_CHECK(stoner_even<R>(g, chi, h), "eigenvalue iteration of chi0(q,0)S did not converge");
+    const auto m = std::max_element(h.begin(), h.end());
+    *sdw = std::max(-1.0e5, *m);
+    *cdw = -1.0e5;
+    if (q_sdw) *q_sdw = (int)(m - h.begin());
+    if (q_cdw) *q_cdw = 0;
+    return;
+  }
   bool done = false;
   if constexpr (std::is_same<R, float>::value) {
     if (stoner_launch<R, float>(g, chi, S, C, h)) {
