@@ -45,33 +45,95 @@ struct Timer {
   }
 };
 
-__global__ void k_sub(double2* out, const double2* a, const double2* b, long long n) {
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
-    out[i] = a[i] - b[i];
-}
-
 struct DiisTerms {
   const double2* x[16];
   double c[16];
 };
 
-// sigma_diis = sum c_i x_i; relative change estimate; mixing (fself.f90:494-532)
+constexpr int kMaxDiis = 16, kDiisBlocks = 1024;
+
+// The history's new entry (x = sigma, residual r = sigma - sigma0) and the inner
+// products of r with the n residuals of the history (entry `self` is r itself),
+// in one pass: part[h * kDiisBlocks + block]
+__global__ void __launch_bounds__(256) k_diis_entry(double2* x, double2* r, const double2* sig, const double2* sig0,
+                                                    DiisTerms t, int n, int self, double* part, long long N) {
+  __shared__ double red[8];
+  double acc[kMaxDiis];
+#pragma unroll
+  for (int h = 0; h < kMaxDiis; ++h) acc[h] = 0.0;
+  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < N; i += (long long)gridDim.x * blockDim.x) {
+    const double2 s = sig[i], d = s - sig0[i];
+    x[i] = s;
+    r[i] = d;
+#pragma unroll
+    for (int h = 0; h < kMaxDiis; ++h)
+      if (h < n) {
+        const double2 v = h == self ? d : t.x[h][i];
+        acc[h] = fma(d.x, v.x, fma(d.y, v.y, acc[h]));
+      }
+  }
+#pragma unroll
+  for (int h = 0; h < kMaxDiis; ++h)
+    if (h < n) {
+      double v = acc[h];
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+      __syncthreads();
+      if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
+      __syncthreads();
+      if (threadIdx.x == 0) {
+        double s = 0.0;
+        for (int w = 0; w < 8; ++w) s += red[w];
+        part[h * kDiisBlocks + blockIdx.x] = s;
+      }
+    }
+}
+// out[b] = sum of part[b * n .. b * n + n)
+__global__ void k_sum_rows(double* out, const double* part, int n) {
+  __shared__ double red[256];
+  double s = 0.0;
+  for (int i = threadIdx.x; i < n; i += blockDim.x) s += part[(long long)blockIdx.x * n + i];
+  red[threadIdx.x] = s;
+  __syncthreads();
+  for (int o = blockDim.x / 2; o > 0; o >>= 1) {
+    if ((int)threadIdx.x < o) red[threadIdx.x] += red[threadIdx.x + o];
+    __syncthreads();
+  }
+  if (threadIdx.x == 0) out[blockIdx.x] = red[0];
+}
+
+// sigma_diis = sum c_i x_i; relative change estimate max |s0 - sd| / |sd| over
+// |sd| > 1e-10; mixing (fself.f90:494-532).  The largest ratio is kept as a
+// pair of squares and compared by cross products: two hypots and a division
+// per element made this pass FP64 bound (4.9 ms for 52 M elements, 1.5 ms now).
+// Squares that could leave the exponent range take the ratio itself.
 __global__ void k_diis_mix(double2* sig, const double2* sig0, DiisTerms t, int n, double pp, int use_diis,
                            double* partmax, long long N) {
   __shared__ double red[256];
-  double mx = 0.0;
+  double bn = 0.0, bd = 1.0;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < N; i += (long long)gridDim.x * blockDim.x) {
     double2 sd = mkc(0.0, 0.0);
-    for (int h = 0; h < n; ++h) sd += t.c[h] * t.x[h][i];
+    for (int h = 0; h < n; ++h) {
+      const double2 x = t.x[h][i];
+      sd = mkc(fma(t.c[h], x.x, sd.x), fma(t.c[h], x.y, sd.y));
+    }
     const double2 s0 = sig0[i];
-    const double asd = hypot(sd.x, sd.y);
-    if (asd > 1.0e-10) {
-      const double2 d = s0 - sd;
-      mx = fmax(mx, hypot(d.x, d.y) / asd);
+    const double2 d = s0 - sd;
+    double num = abs2(d), den = abs2(sd);
+    if (den > 1.0e-20) {
+      if (!(num < 1.0e70 && den < 1.0e70)) {
+        const double q = hypot(d.x, d.y) / hypot(sd.x, sd.y);
+        num = q < 1.0e70 ? q * q : 1.0e140;
+        den = 1.0;
+      }
+      if (num * bd > bn * den) {
+        bn = num;
+        bd = den;
+      }
     }
     sig[i] = use_diis ? sd : (pp * sd + (1.0 - pp) * s0);
   }
-  red[threadIdx.x] = mx;
+  red[threadIdx.x] = sqrt(bn / bd);
   __syncthreads();
   for (int s = blockDim.x / 2; s > 0; s >>= 1) {
     if ((int)threadIdx.x < s) red[threadIdx.x] = fmax(red[threadIdx.x], red[threadIdx.x + s]);
@@ -550,7 +612,7 @@ void mkself_core(Inputs& in, const FlexParams& a, double2* sig_out, double* mu_o
   } else {
     mu_old = mu * 1.2;
     sig0.zero();
-    green0(G.p, eig.p, uni.p, mu, a.temp, Nk, Nw, Norb);
+    green0(G.p, eig.p, uni.p, mu, a.temp, Nk, Nw, Norb, g.even != nullptr);
   }
   // DIIS state
   int n_hist = 0, i_hist = 0;
@@ -558,24 +620,30 @@ void mkself_core(Inputs& in, const FlexParams& a, double2* sig_out, double* mu_o
   // mu bracket cache
   bool bracket_valid = false;
   double muS_cache = 0, muL_cache = 0, cp_center = 0;
-  DBuf<double> partmax(1024), dmax(1);
+  DBuf<double> partmax(1024), dmax(1), dparts(kMaxDiis * kDiisBlocks), ddots(kMaxDiis);
 
   auto compare_sigma = [&]() {
     i_hist = i_hist % a.m_diis + 1;
     n_hist = std::min(n_hist + 1, (int)a.m_diis);
     const int slot = i_hist - 1;
-    PGB_CUDA(cudaMemcpyAsync(xout[slot].p, sig.p, KE * sizeof(double2), cudaMemcpyDeviceToDevice, st));
-    k_sub<<<nblocks(KE, 256) > 65536 ? 65536 : nblocks(KE, 256), 256, 0, st>>>(res[slot].p, sig.p, sig0.p, KE);
-    launch_check("diis_residual");
-    ctx().kernel_launches++;
     const int n = n_hist;
     std::vector<int> idx(n);
     for (int h = 1; h <= n; ++h) idx[h - 1] = (((i_hist - n + h - 1) % a.m_diis) + a.m_diis) % a.m_diis;
+    DiisTerms rt{};
+    int self = 0;
     for (int h = 0; h < n; ++h) {
-      const double v = dot_re(res[slot].p, res[idx[h]].p, KE);
-      Bc[slot * a.m_diis + idx[h]] = v;
-      Bc[idx[h] * a.m_diis + slot] = v;
+      rt.x[h] = res[idx[h]].p;
+      if (idx[h] == slot) self = h;
     }
+    k_diis_entry<<<kDiisBlocks, 256, 0, st>>>(xout[slot].p, res[slot].p, sig.p, sig0.p, rt, n, self, dparts.p, KE);
+    launch_check("diis_entry");
+    k_sum_rows<<<n, 256, 0, st>>>(ddots.p, dparts.p, kDiisBlocks);
+    launch_check("sum_rows");
+    ctx().kernel_launches += 2;
+    std::vector<double> dots(n);
+    ddots.download(dots.data(), n);
+    sync();
+    for (int h = 0; h < n; ++h) Bc[slot * a.m_diis + idx[h]] = Bc[idx[h] * a.m_diis + slot] = dots[h];
     const int nn = n + 1;
     std::vector<double> B((size_t)nn * nn, 0.0), c(nn, 0.0);
     for (int i = 0; i < n; ++i) {

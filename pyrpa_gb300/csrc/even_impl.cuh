@@ -899,7 +899,7 @@ void chi0_even(const Geom& g, const Pairs& p, const double2* G, double temp, con
   std::vector<cx<R>> hJ(ev.cls.size());
   if (tail) {
     DBuf<double2> G0((size_t)g.K * No * No);
-    green0(G0.p, tail->eig, tail->uni, tail->mu, temp, g.Nk, g.Nw, No);
+    green0(G0.p, tail->eig, tail->uni, tail->mu, temp, g.Nk, g.Nw, No, true);
     F0.alloc(ns * P);
     a.src = G0.p;
     fermi_transform<R>(ev, a, F0.p, ns, false, st);

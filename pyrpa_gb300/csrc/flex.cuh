@@ -83,9 +83,10 @@ void build_pairs_soc(Pairs& p, Geom& g, const int64_t* olist, int Norb, int Nchi
 // ------------------------------------------------------------------ stages
 // All pointers are device pointers; R is the bulk (FFT/contraction) type.
 
-// Gk = G0 (fself.f90:1-41) from eig (Norb,Nk) and uni (Norb,Norb,Nk)
+// Gk = G0 (fself.f90:1-41) from eig (Norb,Nk) and uni (Norb,Norb,Nk); sym: the
+// bands are an even model's (symmetric_bands)
 void green0(double2* G, const double* eig, const double2* uni, double mu, double temp, int Nk,
-            int Nw, int Norb);
+            int Nw, int Norb, bool sym = false);
 // Gk = (iw + mu - H - Sigma)^-1 (fself.f90:43-157); returns false if singular
 bool dyson(double2* G, const double2* sig, const double2* hamk, double mu, double temp, int Nk,
            int Nw, int Norb);
