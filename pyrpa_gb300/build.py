@@ -17,7 +17,7 @@ HERE = Path(__file__).resolve().parent
 CSRC = HERE / "csrc"
 BUILD = HERE / "_build"
 LIB = HERE / "libfmod.so"
-SOURCES = ["flex.cu", "fft.cu", "even_d.cu", "even_q.cu", "even_f.cu", "even.cu", "mu.cu", "drivers.cu", "lws.cu", "abi.cu"]
+SOURCES = ["flex.cu", "fft.cu", "even_d.cu", "even_q.cu", "even_f.cu", "even.cu", "mu.cu", "prefault.cu", "drivers.cu", "lws.cu", "abi.cu"]
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 FLAGS = ["-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC", "-Xcompiler", "-O2"]
 

@@ -456,6 +456,7 @@ double chi0_entry(double2* chi_out, const double* Smat, const double* Cmat, cons
   Pairs p;
   build_pairs(p, olist, (int)Norb, (int)Nchi, irr_chi, chi_map);
   const long long KE = g.K * Norb * Norb, KC = g.K * Nchi * Nchi;
+  HostPrefault pages(chi_out, sizeof(double2) * KC);
   DBuf<double2> G(KE);
   G.upload(Gk, KE);
   DBuf<double> e, S, C;
@@ -492,10 +493,12 @@ double chi0_entry(double2* chi_out, const double* Smat, const double* Cmat, cons
     ckchi_print(g, sdw, cdw, qs, qc);
   }
   if (std::is_same<R, double>::value) {
+    pages.join();
     chi.download(chi_out, KC);
   } else {
     DBuf<double2> w(KC);
     widen<R>(w.p, chi.p, KC);
+    pages.join();
     w.download(chi_out, KC);
   }
   sync();
@@ -787,7 +790,9 @@ void gen_green0_(double2* Gk, const double* eig, const double2* uni, const doubl
   DBuf<double2> u(no * no * nk), G(nk * nw * no * no);
   e.upload(eig, no * nk);
   u.upload(uni, no * no * nk);
+  HostPrefault pages(Gk, G.bytes());
   green0(G.p, e.p, u.p, *mu, *temp, (int)nk, (int)nw, (int)no);
+  pages.join();
   G.download(Gk, nk * nw * no * no);
   sync();
   ABI_CATCH("gen_green0_", nan_fill(Gk, (size_t)(*Nk) * (*Nw) * (*Norb) * (*Norb)))
@@ -801,9 +806,11 @@ void gen_green_inv_(double2* Gk, const double2* self, const double2* hamk, const
   PGB_CHECK(no <= kMaxOrb, "Norb above the engine limit of 8 orbitals");
   const long long KE = nk * nw * no * no;
   DBuf<double2> s(KE), h(no * no * nk), G(KE);
+  HostPrefault pages(Gk, G.bytes());
   s.upload(self, KE);
   h.upload(hamk, no * no * nk);
   green_inv_only(G.p, s.p, h.p, *mu, *temp, (int)nk, (int)nw, (int)no);
+  pages.join();
   G.download(Gk, KE);
   sync();
   ABI_CATCH("gen_green_inv_", nan_fill(Gk, (size_t)(*Nk) * (*Nw) * (*Norb) * (*Norb)))

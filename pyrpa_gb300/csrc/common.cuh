@@ -10,6 +10,7 @@
 #include <cstdio>
 #include <stdexcept>
 #include <string>
+#include <thread>
 #include <vector>
 
 namespace pgb {
@@ -324,6 +325,20 @@ void ensure_context();
 // to thread contexts
 constexpr int kErrSlots = 64;
 int* err_slot_address(int slot);
+
+// Makes the pages of a result array in the background (prefault.cu); joined
+// before the copy into it, and at the end of the scope.
+class HostPrefault {
+ public:
+  HostPrefault(void* p, size_t bytes);
+  ~HostPrefault();
+  HostPrefault(const HostPrefault&) = delete;
+  HostPrefault& operator=(const HostPrefault&) = delete;
+  void join();
+
+ private:
+  std::vector<std::thread> threads_;
+};
 
 // Device allocation through the stream-ordered pool (memory stays cached in
 // the pool between calls, so repeated calls of one shape do not re-map HBM).

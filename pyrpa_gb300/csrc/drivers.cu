@@ -791,8 +791,8 @@ void mkself_core(Inputs& in, const FlexParams& a, double2* sig_out, double* mu_o
     log("[FLEX] WARNING: Stoner factor >= 1 at the final iteration:\n");
     log("[FLEX]   max eig[chi0*S] =%10.6f -> the normal state is magnetically unstable at this T/U.\n", maxchi0s);
   }
-  std::vector<double2> hs(KE);
   if (a.sw_out) {
+    std::vector<double2> hs(KE);
     sig.download(hs.data(), KE);
     sync();
     write_sigma_bin(mu, mu_old, hs, a.temp, Nw, Norb, Nk);
@@ -815,8 +815,10 @@ void run_mkself(const MkselfArgs& a, int prec) {
                  a.sw_rescale, a.sw_tail, a.sigma_scale};
   detect_even(in, a.Smat, a.Cmat, a.hamk, a.eig, a.uni, prec == 32 ? 8 : 16);
   const long long KE = in.g.K * a.Norb * a.Norb;
+  HostPrefault pages(a.sigmak, sizeof(double2) * KE);
   DBuf<double2> sig(KE);
   mkself_core(in, prm, sig.p, a.mu_out, nullptr, 0.0, 0.0, prec);
+  pages.join();
   sig.download(a.sigmak, KE);
   sync();
 }
@@ -1193,6 +1195,7 @@ void run_lin_eliash(const LinEliashArgs& a) {
   upload_inputs(in, a.kmap, a.invk, a.olist, a.Nx, a.Ny, a.Nz, a.Nkall, a.Nk, a.Nw, a.Norb, a.Nchi, a.Smat, a.Cmat,
                 nullptr, nullptr, a.uni);
   const long long KE = in.g.K * a.Norb * a.Norb, KC = in.g.K * a.Nchi * a.Nchi;
+  HostPrefault pages(a.delta, sizeof(double2) * KE);
   DBuf<double> prt(a.Norb), init(a.Nk * a.Norb);
   prt.upload(a.prt, a.Norb);
   init.upload(a.init_delta, a.Nk * a.Norb);
@@ -1213,6 +1216,7 @@ void run_lin_eliash(const LinEliashArgs& a) {
   }
   EliashParams prm{a.temp, a.eps, a.itemax, a.gap_sym, a.arnoldi_m};
   *a.lambda_out = eliash_core<R>(in, chi.p, G.p, init.p, prt.p, prm, D.p, a.clobber_chi ? a.chi : nullptr);
+  pages.join();
   D.download(a.delta, KE);
   sync();
 }
@@ -1331,6 +1335,7 @@ void run_pipeline_impl(const PipelineArgs& a, int prec) {
   upload_inputs(in, a.kmap, a.invk, a.olist, a.Nx, a.Ny, a.Nz, a.Nkall, a.Nk, a.Nw, a.Norb, a.Nchi, a.Smat, a.Cmat,
                 a.hamk, a.eig, a.uni);
   const long long K = in.g.K, KE = K * a.Norb * a.Norb, KC = K * a.Nchi * a.Nchi;
+  HostPrefault pages_s(a.sigmak, sizeof(double2) * KE), pages_d(a.delta, sizeof(double2) * KE);
   detect_even(in, a.Smat, a.Cmat, a.hamk, a.eig, a.uni, 16);
   DBuf<double> prt(a.Norb), init(a.Nk * a.Norb);
   prt.upload(a.prt, a.Norb);
@@ -1374,6 +1379,8 @@ void run_pipeline_impl(const PipelineArgs& a, int prec) {
   }
   g_stats.iterations = iters;
   const double t_compute = t.stop();
+  pages_s.join();
+  pages_d.join();
   t.start();
   sig.download(a.sigmak, KE);
   D.download(a.delta, KE);
