@@ -445,6 +445,7 @@ int64_t make_irr_mesh(int64_t nx, int64_t ny, int64_t nz, std::vector<int64_t>& 
 
 // chi0 entry shared by get_chi0 / get_chi0_tail / get_chi0_conv_
 namespace {
+constexpr long long kEvenMinWork = 1 << 19;  // padded mesh points times pair elements
 template <typename R>
 double chi0_entry(double2* chi_out, const double* Smat, const double* Cmat, const double2* Gk, const int64_t* kmap,
                   const int64_t* invk, const int64_t* olist, double temp, int64_t Nx, int64_t Ny, int64_t Nz, int64_t Nw,
@@ -472,9 +473,16 @@ double chi0_entry(double2* chi_out, const double* Smat, const double* Cmat, cons
     tr.mu = mu;
   }
   DBuf<cx<R>> chi(KC);
-  // the even form for a symmetric G (and bands); a caller's own pair maps
-  // keep the general one
-  if (!irr_chi && !chi_map && (!tail || symmetric_bands(eig, uni, Nk, (int)Norb)) &&
+  // The even form for a symmetric G; a caller's own pair maps keep the general
+  // one, and so do
+  //  * the tail-corrected FP64 bubble: it is what lin_eliash is given, whose
+  //    fixed-size two-pass Krylov space amplifies a change of 1e-16 in chi0 to
+  //    1e-9 .. 2e-8 of the gap (twelve two-orbital models), so its bits stay;
+  //  * small calls, which launches bound: 16x16x256, one orbital, 0.27 ms
+  //    against 0.33 ms with the even form's tables and checks.
+  const bool even_call = !irr_chi && !chi_map && !(tail && std::is_same<R, double>::value) &&
+                         g.P * Nchi * Nchi >= kEvenMinWork;
+  if (even_call && (!tail || symmetric_bands(eig, uni, Nk, (int)Norb)) &&
       symmetric_blocks(G.p, g.K, (int)Norb, 1.0e-12)) {
     if (with_stoner) g.even = make_even(g, p, Smat, Cmat, (int)sizeof(cx<R>));
     if (!g.even) g.even = make_even(g, p, nullptr, nullptr, (int)sizeof(cx<R>));

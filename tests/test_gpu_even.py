@@ -85,9 +85,12 @@ def dressed(m):
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("dims", MESHES)
-@pytest.mark.parametrize("tail", [False, True])
-def test_chi0_matches_oracle_and_general_form(F, dims, tail):
+@pytest.mark.parametrize("dims", MESHES + [(2, 16, 16, 1, 64), (1, 64, 64, 1, 64), (3, 12, 10, 1, 40), (2, 6, 6, 6, 80)])
+@pytest.mark.parametrize("tail,bits", [(False, 64), (True, 64), (True, 48)])
+def test_chi0_matches_oracle_and_general_form(F, dims, tail, bits):
+    """get_chi0 takes the even form from 2^19 mesh points times pair elements on (the
+    last four meshes); the FP64 tail-corrected entry keeps the general form, the
+    double-float one does not."""
     m = model(*dims)
     G = dressed(m)
     if tail:
@@ -96,8 +99,12 @@ def test_chi0_matches_oracle_and_general_form(F, dims, tail):
     else:
         args = (m["S"], m["C"], G, m["olist"], m["kmap"], m["invk"], m["temp"], *m["mesh"])
         run, ref = F.get_chi0, O.get_chi0
-    chi, st = run(*args)
-    gchi, gst = general(lambda: run(*args))
+    F.set_precision(bits)
+    try:
+        chi, st = run(*args)
+        gchi, gst = general(lambda: run(*args))
+    finally:
+        F.set_precision(64)
     close(chi, gchi)
     assert abs(st - gst) <= 1e-9
     if chi.size * np.prod(m["mesh"]) < 4e7:
@@ -138,33 +145,51 @@ def test_mkself_converges_with_oracle(F, dims):
 @pytest.mark.parametrize("dims", [(1, 16, 16, 1, 32), (2, 32, 32, 1, 24), (3, 8, 8, 1, 30), (2, 5, 7, 1, 9),
                                   (2, 6, 6, 6, 12), (5, 4, 6, 1, 10)])
 @pytest.mark.parametrize("gap_sym", [0, 1])
-def test_pairing_vertex_and_operator_match_general_form(F, dims, gap_sym):
-    """V_Delta, and one application of the Eliashberg operator to the initial gap
-    (the power method stopped after one step): the eigenvalue itself is not
-    compared, its Krylov space amplifies rounding on weakly paired models."""
+@pytest.mark.parametrize("bits,rtol", [(64, RTOL64), (3264, 1e-4)])
+def test_fused_operator_matches_general_form(F, dims, gap_sym, bits, rtol):
+    """One FLEX iteration, then one application of the Eliashberg operator to the
+    initial gap (the power method stopped after one step) in the fused call: V_Delta,
+    the anomalous function's transforms and the contraction.  The eigenvalue itself
+    is not compared, its Krylov space amplifies rounding on weakly paired models."""
     m = model(*dims)
-    G = dressed(m)
-    chi, _ = F.get_chi0_tail(m["S"], m["C"], G, m["eig"], m["uni"], m["olist"], m["kmap"], m["invk"], m["mu"], m["temp"],
-                             *m["mesh"])
     init = F.get_initial_gap(m["klist"], m["Norb"], gap_sym) + 0.1
+    F.set_precision(bits)
+    try:
+        run = lambda: F.flex_eliash(m["S"], m["C"], m["kmap"], m["invk"], m["olist"], m["hamk"], m["eig"],  # noqa: E731
+                                    m["uni"], init, np.ones(m["Norb"]), m["mu"], m["fill"], m["temp"], m["Nw"],
+                                    *m["mesh"], gap_sym, scf_loop=1, eps=1e-12, sw_tail=True, arnoldi_m=0, itemax=1)
+        r, g = run(), general(run)
+    finally:
+        F.set_precision(64)
+    close(r["gap"], g["gap"], rtol, max(ATOL64, 1e-2 * rtol * np.abs(g["gap"]).max()))
+    assert abs(r["stoner"] - g["stoner"]) <= max(1e-9, rtol)
+
+
+@pytest.mark.gpu
+def test_fp64_pairing_input_keeps_its_bits(F):
+    """The FP64 tail-corrected chi0 and lin_eliash take the general form for every
+    model: the same bits as with the even form switched off."""
+    m = model(2, 32, 32, 1, 64)
+    G = dressed(m)
+    init = F.get_initial_gap(m["klist"], 2, 0)
 
     def run():
+        chi, st = F.get_chi0_tail(m["S"], m["C"], G, m["eig"], m["uni"], m["olist"], m["kmap"], m["invk"], m["mu"],
+                                  m["temp"], *m["mesh"])
         v = chi.copy()
-        gap, _ = F.linearized_eliashberg(v, G, m["uni"], init, m["S"], m["C"], m["olist"], np.ones(m["Norb"]),
-                                         m["kmap"], m["invk"], *m["mesh"], m["temp"], gap_sym, arnoldi_m=0, itemax=1)
-        return v, gap
+        gap, lam = F.linearized_eliashberg(v, G, m["uni"], init, m["S"], m["C"], m["olist"], np.ones(2), m["kmap"],
+                                           m["invk"], *m["mesh"], m["temp"], 0, arnoldi_m=20)
+        return chi, v, gap, lam
 
-    v, gap = run()
-    gv, ggap = general(run)
-    close(v, gv)
-    close(gap, ggap)
+    for a, b in zip(run(), general(run)):
+        assert np.array_equal(a, b)
 
 
 @pytest.mark.gpu
 def test_broken_symmetry_keeps_the_general_form(F):
-    """A G, a Sigma seed or a chi without the symmetry, and complex hoppings: the same
+    """A G or a Sigma seed without the symmetry, and complex hoppings: the same
     results as with the even form switched off, bit for bit."""
-    m = model(2, 8, 8, 1, 16)
+    m = model(2, 32, 32, 1, 24)
     G = dressed(m).copy()
     G[0, 1] *= 1.0 + 1e-6
     args = (m["S"], m["C"], G, m["olist"], m["kmap"], m["invk"], m["temp"], *m["mesh"])
@@ -172,15 +197,11 @@ def test_broken_symmetry_keeps_the_general_form(F):
     mc = model(2, 8, 8, 1, 16, complex_hop=True)
     run = lambda: F.mkself(*step_args(mc), scf_loop=2, eps=0.0, pp=0.5, sw_rescale=True)[0]  # noqa: E731
     assert np.array_equal(run(), general(run))
-    chi = F.get_chi0(m["S"], m["C"], dressed(m), m["olist"], m["kmap"], m["invk"], m["temp"], *m["mesh"])[0]
-    chi[0, 1] *= 1.0 + 1e-6
+    seed = F.mkself(*step_args(m), scf_loop=1, eps=0.0, pp=0.5, sw_rescale=True)[0]
+    seed[0, 1] *= 1.0 + 1e-6
     init = F.get_initial_gap(m["klist"], 2, 0)
-
-    def lam():
-        v = chi.copy()
-        r = F.linearized_eliashberg(v, dressed(m), m["uni"], init, m["S"], m["C"], m["olist"], np.ones(2), m["kmap"],
-                                    m["invk"], *m["mesh"], m["temp"], 0)
-        return v, r[1]
-
-    a, b = lam(), general(lam)
-    assert np.array_equal(a[0], b[0]) and a[1] == b[1]
+    fused = lambda: F.flex_eliash(m["S"], m["C"], m["kmap"], m["invk"], m["olist"], m["hamk"], m["eig"],  # noqa: E731
+                                  m["uni"], init, np.ones(2), m["mu"], m["fill"], m["temp"], m["Nw"], *m["mesh"], 0,
+                                  scf_loop=2, eps=1e-12, arnoldi_m=0, itemax=1, sigma_seed=seed, seed_mu=m["mu"],
+                                  seed_mu_old=m["mu"])["sigmak"]
+    assert np.array_equal(fused(), general(fused))
