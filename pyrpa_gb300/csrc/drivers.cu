@@ -827,14 +827,14 @@ void run_mkself(const MkselfArgs& a, int prec) {
 // pass 1 from the initial gap, exit at a Ritz value >= 0.1, else pass 2 with
 // the shift -lambda_- and that Ritz vector deflated.  apply_op/inner/norm/init
 // define the operator and the inner product of the caller's vector space of n
-// elements; the normalized Ritz vector goes to delta_out, lambda is returned.
+// elements (kw, Nkw: the weights of that inner product); the normalized Ritz vector goes to delta_out, lambda is returned.
 // With a restart tolerance set, refine(residual / |lambda|) is asked after
 // every cycle whether the operator has just been replaced by a more precise
 // one (true: the pass restarts on it from the current Ritz vector, whatever
 // the residual).
 template <class Apply, class Inner, class Norm, class Init, class Refine>
-double arnoldi_two_pass(int m, long long KE, Apply apply_op, Inner inner, Norm norm, Init init_vec,
-                        double2* delta_out, Refine refine) {
+double arnoldi_two_pass(int m, long long KE, const double* kw, int Nkw, Apply apply_op, Inner inner, Norm norm,
+                        Init init_vec, double2* delta_out, Refine refine) {
   cudaStream_t st = ctx().stream;
   double lambda_out = 0.0;
   DBuf<double2> w(KE);
@@ -847,26 +847,24 @@ double arnoldi_two_pass(int m, long long KE, Apply apply_op, Inner inner, Norm n
     m_act = m;
     for (int j = 0; j < m; ++j) {
       apply_op(w.p, V[j].p);
+      // against the deflated direction, then the basis, one coefficient after another
+      std::vector<const double2*> xs;
       if (defl) {
         axpy(w.p, make_double2(shift, 0), V[j].p, KE);
-        double2 h = inner(defl, w.p);
-        axpy(w.p, make_double2(-h.x, -h.y), defl, KE);
+        xs.push_back(defl);
       }
-      for (int ii = 0; ii <= j; ++ii) {
-        double2 h = inner(V[ii].p, w.p);
-        Hm[ii * m + j] = h;
-        axpy(w.p, make_double2(-h.x, -h.y), V[ii].p, KE);
-      }
-      const double beta = norm(w.p);
+      for (int ii = 0; ii <= j; ++ii) xs.push_back(V[ii].p);
+      std::vector<double2> h(xs.size());
+      double norm2 = 0;
+      gram_schmidt(w.p, xs.data(), (int)xs.size(), kw, Nkw, KE, h.data(), &norm2);
+      for (int ii = 0; ii <= j; ++ii) Hm[ii * m + j] = h[ii + (defl ? 1 : 0)];
+      const double beta = std::sqrt(norm2);
       Hm[(j + 1) * m + j] = make_double2(beta, 0);
       if (beta < 1.0e-14) {
         m_act = j + 1;
         break;
       }
-      if (j < m - 1) {
-        PGB_CUDA(cudaMemcpyAsync(V[j + 1].p, w.p, KE * sizeof(double2), cudaMemcpyDeviceToDevice, st));
-        scal(V[j + 1].p, 1.0 / beta, KE);
-      }
+      if (j < m - 1) scal_to(V[j + 1].p, 1.0 / beta, w.p, KE);
     }
   };
   // Ritz vector of lam into out (unit norm); returns the Ritz residual
@@ -981,9 +979,9 @@ double arnoldi_two_pass(int m, long long KE, Apply apply_op, Inner inner, Norm n
 }
 
 template <class Apply, class Inner, class Norm, class Init>
-double arnoldi_two_pass(int m, long long KE, Apply apply_op, Inner inner, Norm norm, Init init_vec,
-                        double2* delta_out) {
-  return arnoldi_two_pass(m, KE, apply_op, inner, norm, init_vec, delta_out, [](double) { return false; });
+double arnoldi_two_pass(int m, long long KE, const double* kw, int Nkw, Apply apply_op, Inner inner, Norm norm,
+                        Init init_vec, double2* delta_out) {
+  return arnoldi_two_pass(m, KE, kw, Nkw, apply_op, inner, norm, init_vec, delta_out, [](double) { return false; });
 }
 
 // FP32 start of the double-float Eliashberg stage of the mixed schedule:
@@ -1128,7 +1126,7 @@ double eliash_core(Inputs& in, cx<R>* chi, const double2* G, const double* init,
   double lambda_out = 0.0;
   const int m = (int)a.arnoldi_m;
   if (m > 0) {
-    lambda_out = arnoldi_two_pass(m, KE, apply_op, inner, norm, init_vec, delta_out, refine);
+    lambda_out = arnoldi_two_pass(m, KE, g.kweight.p, Nk, apply_op, inner, norm, init_vec, delta_out, refine);
     PGB_CHECK(!chi32, "the FP32 Arnoldi cycles did not hand over to double-float");
   } else {
     // shifted power method with deflation (feliash.f90:66-140)
@@ -1770,7 +1768,7 @@ void run_lin_eliash_soc(const LinEliashSocArgs& a) {
   };
   double lam = 0.0;
   if (a.arnoldi_m > 0) {
-    lam = arnoldi_two_pass((int)a.arnoldi_m, KF, apply_op, inner, norm, init_vec, D.p);
+    lam = arnoldi_two_pass((int)a.arnoldi_m, KF, ones.p, (int)Nkf, apply_op, inner, norm, init_vec, D.p);
   } else {
     // shifted power method of lin_eliash_soc (feliashwithsoc.f90:60-110): pass 2
     // runs with the shift |newdelta| of pass 1 and no deflation

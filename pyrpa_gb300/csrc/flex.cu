@@ -1276,29 +1276,35 @@ __device__ __forceinline__ cx<R> pick(const cx<R> (&a)[N], int k) {
 // comparison, not by dynamic indexing): a fully unrolled 25x25 elimination
 // is tens of thousands of straight-line instructions per matrix and runs
 // from the instruction cache's backing store.
+// A warp holds 32 / N matrices, one row per lane: lane i of the group that
+// starts at lane `base`; lanes past the last group (act = false) mirror the
+// first.  Every matrix takes the operations, in the order, of a warp of its own.
 template <typename R, int N>
-__device__ __forceinline__ bool warp_inverse(cx<R> (&a)[N], int* piv, int* map) {
-  const int lane = threadIdx.x & 31;
-  int label = lane;
+__device__ __forceinline__ bool warp_inverse(cx<R> (&a)[N], int* piv, int* map, int base, int i, bool act) {
+  const unsigned gmask = (N >= 32 ? 0xffffffffu : ((1u << (N & 31)) - 1u)) << base;
+  int label = i;
   bool ok = true;
 #pragma unroll 1
   for (int k = 0; k < N; ++k) {
     const cx<R> ak = pick<R, N>(a, k);
-    R v = (lane < N && label >= k) ? cabs1(ak) : (R)-1;
-    int key = (lane < N && label >= k) ? label : 1 << 20;
+    R v = (label >= k) ? cabs1(ak) : (R)-1;
+    int key = (label >= k) ? label : 1 << 20;
+    // the largest magnitude, the lowest label among equals, over windows of the
+    // group of doubling width (they may overlap: a maximum)
 #pragma unroll
-    for (int off = 16; off > 0; off >>= 1) {
-      const R ov = shfl_xor(v, off);
-      const int ok2 = __shfl_xor_sync(0xffffffffu, key, off);
+    for (int off = 1; off < N; off <<= 1) {
+      const int j = i + off, from = base + (j < N ? j : j - N);
+      const R ov = shfl_idx(v, from);
+      const int ok2 = __shfl_sync(0xffffffffu, key, from);
       if (ov > v || (ov == v && ok2 < key)) { v = ov; key = ok2; }
     }
     const int plabel = key;
     if (!(v > 0)) ok = false;
     if (label == k) label = plabel;
     else if (label == plabel) label = k;
-    if (lane == 0) piv[k] = plabel;
-    const unsigned m = __ballot_sync(0xffffffffu, label == k && lane < N);
-    const int src = __ffs(m) - 1;
+    if (act && i == 0) piv[k] = plabel;
+    const unsigned m = __ballot_sync(0xffffffffu, label == k && act) & gmask;
+    const int src = m ? __ffs(m) - 1 : base;
     const cx<R> pv = cmk<R>(shfl_idx(ak.x, src), shfl_idx(ak.y, src));
     const cx<R> ip = ok ? cdiv(cmk<R>(1, 0), pv) : cmk<R>(0, 0);
     const bool is_piv = (label == k);
@@ -1324,14 +1330,19 @@ __device__ __forceinline__ bool warp_inverse(cx<R> (&a)[N], int* piv, int* map) 
       for (int j = 0; j < N; ++j) a[j] = (j == k) ? ap : ((j == p) ? ak : a[j]);
     }
   }
-  // bring logical row i back to lane i
-  if (lane < N) map[label] = lane;
+  // bring logical row i back to lane base + i
+  if (act) map[label] = base + i;
   __syncwarp();
-  const int from = (lane < N) ? map[lane] : lane;
+  const int from = map[i];
 #pragma unroll
   for (int j = 0; j < N; ++j) a[j] = cmk<R>(shfl_idx(a[j].x, from), shfl_idx(a[j].y, from));
   __syncwarp();
   return ok;
+}
+template <typename R, int N>
+__device__ __forceinline__ bool warp_inverse(cx<R> (&a)[N], int* piv, int* map) {
+  const int lane = threadIdx.x & 31;
+  return warp_inverse<R, N>(a, piv, map, 0, lane < N ? lane : 0, lane < N);
 }
 
 // Pivot magnitude |Re| + |Im| as a float, for the pivot key of
@@ -1450,22 +1461,29 @@ __device__ __forceinline__ bool warp_inverse_rot(cx<R> (&a)[N], cx<R>* prow, int
 }
 
 // Matrices of consecutive (q,iv) are staged through shared memory in tiles of
-// 2W: the loads and stores of the Fortran (Nk,Nw,Nchi,Nchi) layout are then
-// runs of 2W consecutive elements instead of one element per cache sector.
+// T: the loads and stores of the Fortran (Nk,Nw,Nchi,Nchi) layout are then
+// runs of T consecutive elements instead of one element per cache sector.
+// A warp works on G = 32 / N matrices at a time (one to a warp left 28 of 32
+// lanes idle at N = 4 and 31 at N = 1): two orbitals 15x21x300 FP64 2.34 -> 0.37 ms,
+// three orbitals 32x32x512 FP32 2.03 -> 0.94 ms.
+template <int N, int W> __host__ __device__ constexpr int vertex_reg_tile() {
+  return (N == 4 || N == 16 || N == 25 ? 2 : 1) * W * (32 / N);
+}
 template <typename R, int N, int W>
 __global__ void __launch_bounds__(32 * W) k_vertex_reg(cx<R>* chi, long long nmat, long long estride,
                                                        const R* consts, int mode, int* err) {
-  constexpr int T = 2 * W;          // matrices per tile
-  constexpr int TP = T + 1;         // padded tile row
+  constexpr int G = 32 / N;
+  constexpr int T = vertex_reg_tile<N, W>();  // matrices per tile
+  constexpr int TP = T + 1;                   // padded tile row
   extern __shared__ __align__(16) unsigned char smraw[];
   // constants in the compute precision: an FP64->FP32 conversion per use
   // would run on the FP64 pipe
   R* cs = reinterpret_cast<R*>(smraw);                                 // Si, Ci, S+C, S, C
   constexpr size_t cs_bytes = (5 * N * N * sizeof(R) + 15) / 16 * 16;  // keep the tile 16-byte aligned
   cx<R>* tile = reinterpret_cast<cx<R>*>(smraw + cs_bytes);            // [N*N][TP]
-  cx<R>* tb = tile + (size_t)N * N * TP;                               // [W][N*N]
-  int* pv = reinterpret_cast<int*>(tb + (size_t)W * N * N);            // [W][N+1]
-  int* mp = pv + W * (N + 1);                                          // [W][32]
+  cx<R>* tb = tile + (size_t)N * N * TP;                               // [W G][N*N]
+  int* pv = reinterpret_cast<int*>(tb + (size_t)W * G * N * N);        // [W G][N]
+  int* mp = pv + W * G * N;                                            // [W G][N]
   for (int e = threadIdx.x; e < 5 * N * N; e += blockDim.x) cs[e] = consts[e];
   const R* Si = cs;
   const R* Ci = cs + N * N;
@@ -1473,8 +1491,11 @@ __global__ void __launch_bounds__(32 * W) k_vertex_reg(cx<R>* chi, long long nma
   const R* Sm = cs + 3 * N * N;
   const R* Cm = cs + 4 * N * N;
   const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int i = lane < N ? lane : 0;
-  cx<R>* tbw = tb + (size_t)w * N * N;
+  const bool act = lane < G * N;
+  const int g = act ? lane / N : 0, i = act ? lane - g * N : 0, base = g * N;
+  const int slot = w * G + g;
+  cx<R>* tbw = tb + (size_t)slot * N * N;
+  int *pvw = pv + slot * N, *mpw = mp + slot * N;
   const R c1 = mode == 2 ? (R)-0.5 : (R)1.5;
   const R c2 = mode == 0 ? (R)-0.5 : (R)0.5;
   for (long long m0 = (long long)blockIdx.x * T; m0 < nmat; m0 += (long long)gridDim.x * T) {
@@ -1485,35 +1506,39 @@ __global__ void __launch_bounds__(32 * W) k_vertex_reg(cx<R>* chi, long long nma
       if (t < nt) tile[e * TP + t] = chi[m0 + t + estride * e];
     }
     __syncthreads();
-    for (int t = w; t < nt; t += W) {
+    for (int r = 0; r < T / (W * G); ++r) {
+      const int mine = r * W * G + slot;
+      if (r * W * G + w * G >= nt) break;       // the whole warp is past the end
+      const int t = mine < nt ? mine : nt - 1;  // groups past the end repeat the last matrix
+      const bool keep = act && mine < nt;
       // x(i, j) = tile[(i + N j) * TP + t]
       cx<R> a[N], v[N];
 #pragma unroll
       for (int j = 0; j < N; ++j) a[j] = cmk<R>((R)Si[i * N + j], (R)0) - tile[(i + N * j) * TP + t];
-      bool ok = warp_inverse<R, N>(a, pv + w * (N + 1), mp + w * 32);
+      bool ok = warp_inverse<R, N>(a, pvw, mpw, base, i, act);
 #pragma unroll
       for (int j = 0; j < N; ++j) {
-        R base = 0;
-        if (mode == 1) base = (R)-Sm[i * N + j];
-        else if (mode == 2) base = (R)(Sm[i * N + j] - Cm[i * N + j]);
-        v[j] = cmk<R>(base, (R)0) + c1 * a[j];
+        R bs = (R)0;
+        if (mode == 1) bs = (R)-Sm[i * N + j];
+        else if (mode == 2) bs = (R)(Sm[i * N + j] - Cm[i * N + j]);
+        v[j] = cmk<R>(bs, (R)0) + c1 * a[j];
       }
 #pragma unroll
       for (int j = 0; j < N; ++j) a[j] = cmk<R>((R)Ci[i * N + j], (R)0) + tile[(i + N * j) * TP + t];
-      ok &= warp_inverse<R, N>(a, pv + w * (N + 1), mp + w * 32);
+      ok &= warp_inverse<R, N>(a, pvw, mpw, base, i, act);
 #pragma unroll
       for (int j = 0; j < N; ++j) v[j] += c2 * a[j];
       if (mode == 0) {
         // -0.25 (S+C) X (S+C): t = X (S+C) row-local, then (S+C) t through smem
 #pragma unroll
-        for (int j = 0; j < N; ++j) a[j] = cmk<R>(0, 0);
+        for (int j = 0; j < N; ++j) a[j] = cmk<R>((R)0, (R)0);
 #pragma unroll 1
         for (int k = 0; k < N; ++k) {
           const cx<R> xk = tile[(i + N * k) * TP + t];
 #pragma unroll
           for (int j = 0; j < N; ++j) a[j] += SC[k * N + j] * xk;
         }
-        if (lane < N) {
+        if (act) {
 #pragma unroll
           for (int j = 0; j < N; ++j) tbw[i * N + j] = a[j];
         }
@@ -1525,9 +1550,9 @@ __global__ void __launch_bounds__(32 * W) k_vertex_reg(cx<R>* chi, long long nma
           for (int j = 0; j < N; ++j) v[j] += sk * tbw[k * N + j];
         }
       }
-      if (!ok && lane == 0) atomicExch(err, 3);
+      if (!ok && keep) atomicExch(err, 3);
       __syncwarp();
-      if (lane < N) {
+      if (keep) {
 #pragma unroll
         for (int j = 0; j < N; ++j) tile[(i + N * j) * TP + t] = v[j];
       }
@@ -1670,8 +1695,10 @@ template <typename R, int N, int W> size_t vertex_vs_smem() {
 }
 
 template <typename R, int N, int W> size_t vertex_reg_smem() {
-  return (sizeof(R) * 5 * N * N + 15) / 16 * 16 + sizeof(cx<R>) * ((size_t)N * N * (2 * W + 1) + (size_t)W * N * N) +
-         sizeof(int) * (W * (N + 1) + W * 32);
+  constexpr int G = 32 / N;
+  return (sizeof(R) * 5 * N * N + 15) / 16 * 16 +
+         sizeof(cx<R>) * ((size_t)N * N * (vertex_reg_tile<N, W>() + 1) + (size_t)W * G * N * N) +
+         sizeof(int) * 2 * W * G * N;
 }
 
 template <typename R, int N>
@@ -1679,7 +1706,8 @@ bool vertex_reg_launch(cx<R>* chi, long long nmat, long long estride, const R* d
   constexpr int warps = (N >= 16) ? 4 : 8;
   const size_t smem = vertex_reg_smem<R, N, warps>();
   PGB_SMEM_LIMIT_ONCE((k_vertex_reg<R, N, warps>), smem);
-  const long long tiles = (nmat + 2 * warps - 1) / (2 * warps);
+  constexpr int T = vertex_reg_tile<N, warps>();
+  const long long tiles = (nmat + T - 1) / T;
   const long long blocks = std::min<long long>(tiles, (long long)ctx().num_sms * 8);
   k_vertex_reg<R, N, warps><<<(unsigned)std::max(1LL, blocks), 32 * warps, smem, ctx().stream>>>(
       chi, nmat, estride, dconsts, mode, ctx().err);
@@ -1748,8 +1776,8 @@ bool vertex(cx<R>* chi, long long nmat, long long stride, int Nchi, const double
       reset_err();
       if constexpr (std::is_same<R, dfl>::value) {
         switch (n) {
-          case 1: vertex_vs_launch<R, 1>(chi, nmat, estride, dc.p, mode); break;
-          case 4: vertex_vs_launch<R, 4>(chi, nmat, estride, dc.p, mode); break;
+          case 1: vertex_reg_launch<R, 1>(chi, nmat, estride, dc.p, mode); break;
+          case 4: vertex_reg_launch<R, 4>(chi, nmat, estride, dc.p, mode); break;
           case 9: vertex_vs_launch<R, 9>(chi, nmat, estride, dc.p, mode); break;
           case 16: vertex_vs_launch<R, 16>(chi, nmat, estride, dc.p, mode); break;
           case 25: vertex_vs_launch<R, 25>(chi, nmat, estride, dc.p, mode); break;
@@ -2956,6 +2984,62 @@ __global__ void k_scal(double2* y, double a, long long n) {
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
     y[i] = a * y[i];
 }
+// One step of the modified Gram-Schmidt orthogonalization of y against a Krylov
+// basis, device resident: h = 2 sum_i of the previous step's partial sums (every
+// block adds them up itself, in k_sum_parts' order), y -= h xp, and the partial
+// sums of the next inner product sum kw conj(xn) y (xn null: of y with itself).
+// The element order and arithmetic are those of inner_w, axpy and inner_w called
+// one after the other, which waited for the host at every coefficient.
+__global__ void __launch_bounds__(kRedThreads) k_gs_step(double2* y, const double2* xp, const double2* part_in,
+                                                         double2* h_out, const double2* xn, double2* part_out,
+                                                         const double* kw, unsigned Nk, unsigned n) {
+  __shared__ double2 red[kRedThreads];
+  double2 a = mkc(0.0, 0.0);
+  if (xp) {
+    double2 acc = mkc(0.0, 0.0);
+    for (int i = threadIdx.x; i < kRedBlocks; i += blockDim.x) acc += part_in[i];
+    red[threadIdx.x] = acc;
+    __syncthreads();
+    for (int s = blockDim.x / 2; s > 0; s >>= 1) {
+      if ((int)threadIdx.x < s) red[threadIdx.x] += red[threadIdx.x + s];
+      __syncthreads();
+    }
+    const double2 s = red[0];
+    __syncthreads();
+    const double2 h = mkc(2.0 * s.x, 2.0 * s.y);
+    if (blockIdx.x == 0 && threadIdx.x == 0) *h_out = h;
+    a = mkc(-h.x, -h.y);
+  }
+  double2 acc = mkc(0.0, 0.0);
+  for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+    // the roundings of k_axpy and k_inner_w (which product of each pair is fused
+    // is the compiler's choice there; written out, because the Krylov space
+    // amplifies a different one)
+    double2 v = y[i];
+    if (xp) {
+      const double2 x = xp[i];
+      v.x = __dadd_rn(v.x, fma(a.x, x.x, -__dmul_rn(a.y, x.y)));
+      v.y = __dadd_rn(v.y, fma(a.y, x.x, __dmul_rn(a.x, x.y)));
+      y[i] = v;
+    }
+    const double2 u = xn ? xn[i] : v;
+    const double k = kw[i % Nk];
+    acc.x = fma(k, fma(u.x, v.x, __dmul_rn(u.y, v.y)), acc.x);
+    acc.y = fma(k, fma(u.x, v.y, -__dmul_rn(u.y, v.x)), acc.y);
+  }
+  red[threadIdx.x] = acc;
+  __syncthreads();
+  for (int s = blockDim.x / 2; s > 0; s >>= 1) {
+    if ((int)threadIdx.x < s) red[threadIdx.x] += red[threadIdx.x + s];
+    __syncthreads();
+  }
+  if (threadIdx.x == 0) part_out[blockIdx.x] = red[0];
+}
+__global__ void k_scal_to(double2* y, double a, const double2* x, long long n) {
+  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
+    y[i] = a * x[i];
+}
+
 struct LinComb {
   const double2* x[64];
   double2 c[64];
@@ -2966,6 +3050,29 @@ __global__ void k_lincomb(double2* y, LinComb lc, int m, long long n) {
     for (int t = 0; t < m; ++t) acc += lc.c[t] * lc.x[t][i];
     y[i] = acc;
   }
+}
+void gram_schmidt(double2* y, const double2* const* xs, int m, const double* kw, int Nk, long long n, double2* h,
+                  double* norm2) {
+  PGB_CHECK(n < (1LL << 32) - (long long)kRedBlocks * kRedThreads, "vector too long for the orthogonalization");
+  cudaStream_t st = ctx().stream;
+  DBuf<double2> part(2 * kRedBlocks), out(m + 1);
+  for (int i = 0; i <= m; ++i) {
+    k_gs_step<<<kRedBlocks, kRedThreads, 0, st>>>(y, i ? xs[i - 1] : nullptr, part.p + (i & 1) * kRedBlocks,
+                                                  i ? out.p + i - 1 : nullptr, i < m ? xs[i] : nullptr,
+                                                  part.p + ((i + 1) & 1) * kRedBlocks, kw, (unsigned)Nk, (unsigned)n);
+    count_launch("gs_step");
+  }
+  k_sum_parts<<<1, kRedThreads, 0, st>>>(out.p + m, part.p + ((m + 1) & 1) * kRedBlocks, kRedBlocks);
+  count_launch("sum_parts");
+  std::vector<double2> hh(m + 1);
+  out.download(hh.data(), m + 1);
+  sync();
+  for (int i = 0; i < m; ++i) h[i] = hh[i];
+  *norm2 = 2.0 * hh[m].x;
+}
+void scal_to(double2* y, double a, const double2* x, long long n) {
+  k_scal_to<<<grid_1d(n, 256, 65536), 256, 0, ctx().stream>>>(y, a, x, n);
+  count_launch("scal_to");
 }
 void axpy(double2* y, double2 a, const double2* x, long long n) {
   k_axpy<<<grid_1d(n, 256, 65536), 256, 0, ctx().stream>>>(y, a, x, n);

@@ -184,6 +184,12 @@ bool mkfk_df(cdf* F, const cdf* G, const double2* D, long long K, int Norb);
 void hermitize(double2* D, long long K, int Norb);
 void initial_delta(double2* D, const double* init, const double2* uni, int Nk, int Nw, int Norb,
                    int gap_sym);
+// modified Gram-Schmidt of y against xs[0..m) with the inner product
+// 2 sum_i kw[i mod Nk] conj(a_i) b_i: coefficients into h[0..m), the squared
+// norm of what is left into norm2; one wait for all of them
+void gram_schmidt(double2* y, const double2* const* xs, int m, const double* kw, int Nk, long long n, double2* h,
+                  double* norm2);
+void scal_to(double2* y, double a, const double2* x, long long n);       // y = a x
 void axpy(double2* y, double2 a, const double2* x, long long n);         // y += a x
 void scal(double2* y, double a, long long n);
 void lincomb(double2* y, const double2* const* xs, const double2* cs, int m, long long n);
