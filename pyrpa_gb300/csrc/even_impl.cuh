@@ -460,16 +460,46 @@ __global__ void k_even_contract(cx<R>* out, const cx<R>* W, const cx<R>* F, cons
 // element; word = a | b << 9 | (ca + 2) << 18 | (cb + 2) << 21.  vout, per class two
 // words (real, imaginary part): value = cf (sa v[a] + sb v[b]) over the result
 // v[q N + p]; word = a | b << 10 | (sa + 1) << 20 | (sb + 1) << 22 | (cf = 1/2) << 24.
-template <typename R> __device__ __forceinline__ R small_coef(int c) {  // -2 .. 2, exact
-  return c == 0 ? (R)0.f : (c == 1 ? (R)1.f : (c == 2 ? (R)2.f : (c == -1 ? (R)-1.f : (R)-2.f)));
-}
-
 __device__ __forceinline__ float real_mag(float a) { return fabsf(a); }
 __device__ __forceinline__ float real_mag(double a) { return (float)fabs(a); }
 __device__ __forceinline__ float real_mag(dfl a) { return fabsf(a.hi); }
 
 template <typename R> __host__ __device__ constexpr int rrow_pad() { return sizeof(R) == 4 ? 4 : 2; }
 template <typename R> __host__ __device__ constexpr int rrow_len(int n) { return (n + rrow_pad<R>() + 2) & ~3; }
+
+// entries 1 .. N-1 of a row in 16-byte words (d aligned), and two of them back
+template <typename R, int N> __device__ __forceinline__ void row_put(R* d, const R (&a)[N]) {
+  if constexpr (sizeof(R) == 4) {
+    float4* d4 = reinterpret_cast<float4*>(d);
+#pragma unroll
+    for (int s = 1; s < N; s += 4)
+      d4[(s - 1) >> 2] = make_float4(a[s], s + 1 < N ? a[s + 1 < N ? s + 1 : 0] : 0.f,
+                                     s + 2 < N ? a[s + 2 < N ? s + 2 : 0] : 0.f,
+                                     s + 3 < N ? a[s + 3 < N ? s + 3 : 0] : 0.f);
+  } else if constexpr (std::is_same<R, dfl>::value) {
+    float4* d4 = reinterpret_cast<float4*>(d);
+#pragma unroll
+    for (int s = 1; s < N; s += 2) {
+      const dfl b = s + 1 < N ? a[s + 1 < N ? s + 1 : 0] : dfl(0.f);
+      d4[(s - 1) >> 1] = make_float4(a[s].hi, a[s].lo, b.hi, b.lo);
+    }
+  } else {
+    double2* d2 = reinterpret_cast<double2*>(d);
+#pragma unroll
+    for (int s = 1; s < N; s += 2) d2[(s - 1) >> 1] = make_double2(a[s], s + 1 < N ? a[s + 1 < N ? s + 1 : 0] : 0.0);
+  }
+}
+__device__ __forceinline__ void row_get(const double* d, double& a, double& b) {
+  const double2 v = *reinterpret_cast<const double2*>(d);
+  a = v.x;
+  b = v.y;
+}
+__device__ __forceinline__ void row_get(const dfl* d, dfl& a, dfl& b) {
+  const float4 v = *reinterpret_cast<const float4*>(d);
+  a = dfl(v.x, v.y);
+  b = dfl(v.z, v.w);
+}
+__device__ __forceinline__ void row_get(const float*, float&, float&) {}  // float rows go in fours
 
 // Real warp_inverse_rot (flex.cu) of the group's matrix: lane i of a group of N
 // lanes holds row i.  The pivot row goes through shared memory with entry s at
@@ -507,8 +537,8 @@ __device__ __forceinline__ bool real_inverse_rot(R (&a)[N], R* prow, int* piv, i
     if (act && i == 0) piv[k] = plabel;
     R* buf = prow + (k & 1) * PL;
     if (is_piv) {
-#pragma unroll
-      for (int s = 0; s < N; ++s) buf[s + PAD - 1] = a[s];
+      buf[PAD - 1] = a[0];
+      row_put<R, N>(buf + PAD, a);
     }
     __syncwarp();
     const R p = buf[PAD - 1];
@@ -527,7 +557,12 @@ __device__ __forceinline__ bool real_inverse_rot(R (&a)[N], R* prow, int* piv, i
       }
     } else {
 #pragma unroll
-      for (int s = 1; s < N; ++s) a[s - 1] = mad(f, buf[s + PAD - 1], a[s]);
+      for (int s = 1; s < N; s += 2) {
+        R q0, q1;
+        row_get(buf + PAD + s - 1, q0, q1);
+        a[s - 1] = mad(f, q0, a[s]);
+        if (s + 1 < N) a[s] = mad(f, q1, a[s + 1]);
+      }
     }
     a[N - 1] = is_piv ? (R)1 : f;
   }
@@ -555,7 +590,10 @@ struct EvenVertexTabs {
 // lane), a CTA stages a tile of them through shared memory; the accumulator of
 // V is real.  consts: Si, Ci (inverses of S and C), D = S + C, S, C in the
 // basis, row-major; D is dense on the nself same-orbital pairs and diagonal
-// elsewhere.
+// elsewhere.  FP64: bound by its pipe (91 % at N = 25, 33 ms for 263,168
+// matrices; general form 122 ms).  FP32: issue bound; predecoded source offsets,
+// the pivot row in 16-byte stores and D's row in registers took 2.1 M matrices from
+// 24.0 to 20.4 ms (general form 45 ms).
 template <typename R, int N, int W>
 __global__ void __launch_bounds__(32 * W, sizeof(R) == 4 ? 4 : 2)
     k_vertex_even(cx<R>* chi, long long nmat, long long estride, const R* consts, EvenVertexTabs tb, int mode,
@@ -566,15 +604,22 @@ __global__ void __launch_bounds__(32 * W, sizeof(R) == 4 ? 4 : 2)
   cx<R>* tile = reinterpret_cast<cx<R>*>(prow + (size_t)T * 2 * PL);  // [ncls][TP]
   R* vb = reinterpret_cast<R*>(tile + (size_t)tb.ncls * TP);  // [T][N*N], entry (p, q) at q N + p
   R* cs = vb + (size_t)T * N * N;                            // Si, Ci (column-major), then D row-major
-  int* vin = reinterpret_cast<int*>(cs + 3 * N * N);         // [N*N]
-  int* pv = vin + N * N;                                     // [T][N]
+  int2* vin = reinterpret_cast<int2*>(cs + 3 * N * N + (N & 1));  // [N*N]
+  int* pv = reinterpret_cast<int*>(vin + N * N);             // [T][N]
   int* ps = pv + T * N;                                      // [T][N]
   for (int e = threadIdx.x; e < N * N; e += blockDim.x) {
     const int p = e % N, q = e / N;  // stored column-major for the row-per-lane reads
     cs[e] = consts[p * N + q];
     cs[N * N + e] = consts[N * N + p * N + q];
     cs[2 * N * N + e] = consts[2 * N * N + e];
-    vin[e] = tb.vin[e];
+    // the two sources as offsets into the tile, with the signs in bit 31 and
+    // "twice" in bit 30 of the first, "absent" in bit 30 of the second
+    const int word = tb.vin[e];
+    const int ia = word & 511, ib = (word >> 9) & 511;
+    const int ca = ((word >> 18) & 7) - 2, cb = ((word >> 21) & 7) - 2;
+    const unsigned oa = (unsigned)((ia >> 1) * TP * 2 + (ia & 1)), ob = (unsigned)((ib >> 1) * TP * 2 + (ib & 1));
+    vin[e] = make_int2((int)(oa | (ca < 0 ? 1u << 31 : 0u) | (ca == 2 || ca == -2 ? 1u << 30 : 0u)),
+                       (int)(ob | (cb < 0 ? 1u << 31 : 0u) | (cb == 0 ? 1u << 30 : 0u)));
   }
   const R* Sm = consts + 3 * N * N;
   const R* Cm = consts + 4 * N * N;
@@ -600,17 +645,15 @@ __global__ void __launch_bounds__(32 * W, sizeof(R) == 4 ? 4 : 2)
     }
     __syncthreads();
     R a[N];
+    const R* mine = tr + 2 * t;
     auto entry = [&](int q) {
-      const int word = vin[q * N + i];
-      const int ia = word & 511, ib = (word >> 9) & 511;
-      const int ca = ((word >> 18) & 7) - 2, cb = ((word >> 21) & 7) - 2;
-      R v = tr[((ia >> 1) * TP + t) * 2 + (ia & 1)];
-      if (ca == -1) v = -v;
-      else if (ca == 2) v = v + v;
-      else if (ca == -2) v = -(v + v);
-      if (cb) {
-        const R u = tr[((ib >> 1) * TP + t) * 2 + (ib & 1)];
-        v = v + (cb > 0 ? u : -u);
+      const int2 word = vin[q * N + i];
+      R v = mine[word.x & 0x3fffffff];
+      if (word.x < 0) v = -v;
+      if (word.x & (1 << 30)) v = v + v;
+      if (!(word.y & (1 << 30))) {
+        const R u = mine[word.y & 0x3fffffff];
+        v = v + (word.y < 0 ? -u : u);
       }
       return v;
     };
@@ -668,15 +711,18 @@ __global__ void __launch_bounds__(32 * W, sizeof(R) == 4 ? 4 : 2)
       }
       const R m4 = (R)-0.25f;
       const R dl = m4 * D[i * N + i];
+      constexpr int NH = N < 8 ? N : 8;
+      R dh[NH];
+#pragma unroll
+      for (int r = 0; r < NH; ++r) dh[r] = r < ns ? m4 * D[i * N + r] : (R)0;
+      const bool head = i < ns;
 #pragma unroll
       for (int q = 0; q < N; ++q) {
-        R v = dl * a[q];
         R sum = (R)0;
-        for (int r = 0; r < ns; ++r) {
-          const R o = shfl_idx(a[q], g * N + r);
-          sum = mad(m4 * D[i * N + r], o, sum);
-        }
-        if (i < ns) v = sum;
+#pragma unroll
+        for (int r = 0; r < NH; ++r)
+          if (r < ns) sum = mad(dh[r], shfl_idx(a[q], g * N + r), sum);
+        const R v = head ? sum : dl * a[q];
         if (act) vw[q * N + i] = vw[q * N + i] + v;
       }
     }
@@ -710,7 +756,7 @@ void vertex_even_launch(const Even& ev, cx<R>* chi, long long nmat, long long es
   constexpr int W = 8, T = W * (32 / N);
   const int nc = (int)ev.cls.size();
   const size_t smem = sizeof(R) * ((size_t)T * 2 * rrow_len<R>(N) + (size_t)T * N * N + 3 * N * N) +
-                      sizeof(cx<R>) * (size_t)nc * (T + 1) + sizeof(int) * (N * N + 2 * T * N);
+                      sizeof(cx<R>) * (size_t)nc * (T + 1) + sizeof(R) + sizeof(int) * (2 * N * N + 2 * T * N);
   PGB_SMEM_LIMIT_ONCE((k_vertex_even<R, N, W>), 220 * 1024);
   EvenVertexTabs tb{ev.d_vin.p, ev.d_vout.p, ev.cls_el.p, ev.mem.p, ev.memcj.p, ev.nmem.p, nc, ev.nself, full ? 1 : 0};
   const long long tiles = (nmat + T - 1) / T;
