@@ -23,7 +23,7 @@
 // same scalar decisions from the same total.  A host-driven search paid two
 // launches, a copy and a wait for each of its 30 to 40 evaluations.
 // Measured, search with its coefficients (two searches of one FLEX iteration):
-// one orbital 32x32x1024 2.6 -> 1.4 ms; five orbitals 64x64x1024 26 -> 5.9 ms (9.8
+// one orbital 32x32x1024 2.6 -> 0.8 ms; five orbitals 64x64x1024 26 -> 5.5 ms (9.8
 // with a Householder reduction).
 #include <algorithm>
 
@@ -147,35 +147,30 @@ __device__ double im_digamma(double a, double y) {
   return s + atan2(y, a) - 0.5 * r.y - t.y;
 }
 
-constexpr int kMuThreads = 512;
+constexpr int kMuThreads = 256;
 constexpr long long kMuWaitCycles = 4000000000LL;  // about 2 s
 
 // Sum over the grid of v, the same in every thread.  Blocks meet at a counter
 // that only grows; every wait is bounded, and a block that gives up tells the
 // caller through `dead`.  The launch is cooperative, so all blocks are resident.
 __device__ double grid_sum(double v, double* part, unsigned* bar, unsigned round, bool& dead) {
-  __shared__ double red[32];
+  __shared__ double red[kMuThreads / 32];
   __shared__ double total;
   __shared__ int gave_up;
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  auto block_sum = [&](double x) {
+  auto warp_sum = [](double x) {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
-    if (lane == 0) red[w] = x;
-    __syncthreads();
-    if (w == 0) {
-      x = lane < nw ? red[lane] : 0.0;
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
-      if (lane == 0) total = x;
-    }
-    __syncthreads();
-    return total;
+    return x;
   };
-  const double mine = block_sum(v);
+  v = warp_sum(v);
+  if (lane == 0) red[w] = v;
+  __syncthreads();
   double* p = part + (round & 1) * gridDim.x;
   if (threadIdx.x == 0) {
     gave_up = 0;
+    double mine = red[0];
+    for (int i = 1; i < nw; ++i) mine += red[i];
     __stcg(p + blockIdx.x, mine);
     __threadfence();
     atomicAdd(bar, 1u);
@@ -190,9 +185,16 @@ __device__ double grid_sum(double v, double* part, unsigned* bar, unsigned round
   }
   __syncthreads();
   dead = dead || gave_up;
-  double s = 0.0;
-  for (int b = threadIdx.x; b < (int)gridDim.x; b += blockDim.x) s += __ldcg(p + b);
-  return block_sum(s);
+  // the blocks' sums by one warp: an FP64 add of every warp would cost as much as
+  // a trial point of every thread
+  if (w == 0) {
+    double s = 0.0;
+    for (int b = lane; b < (int)gridDim.x; b += 32) s += __ldcg(p + b);
+    s = warp_sum(s);
+    if (lane == 0) total = s;
+  }
+  __syncthreads();
+  return total;
 }
 
 template <int N>
@@ -210,6 +212,10 @@ __global__ void __launch_bounds__(kMuThreads) k_mu_search(MuState* io, const dou
   auto get_rn = [&](double rmu) {
     const double x = rmu - center;
     double acc = 0.0, tail = 0.0;
+    // dealt out block by block: one digamma costs as much FP64 as a few points, and
+    // the first blocks would hold all others up
+    for (long long t = threadIdx.x * (long long)gridDim.x + blockIdx.x; t < (long long)Nk * N; t += S)
+      tail += im_digamma(Nw + 0.5, (rmu - eig[t]) / (2.0 * kPi * temp));
     for (long long i = first; i < K; i += G * S) {
       double num[G], den[G];
 #pragma unroll
@@ -218,15 +224,15 @@ __global__ void __launch_bounds__(kMuThreads) k_mu_search(MuState* io, const dou
         den[g] = 1.0;
         const long long at = i + g * S;
         if (at < K) {
-          double2 p = cp[(N - 1) * K + at], dp = mkc(1.0, 0.0);
+          double2 p = cp[(N - 1) * K + at], dp;
           p.x += x;
 #pragma unroll
           for (int d = N - 2; d >= 0; --d) {
             const double2 c = cp[d * K + at];
-            dp = mkc(fma(dp.x, x, p.x), fma(dp.y, x, p.y));
+            dp = d == N - 2 ? mkc(x + p.x, p.y) : mkc(fma(dp.x, x, p.x), fma(dp.y, x, p.y));
             p = mkc(fma(p.x, x, c.x), fma(p.y, x, c.y));
           }
-          num[g] = fma(dp.x, p.x, dp.y * p.y);
+          num[g] = N == 1 ? p.x : fma(dp.x, p.x, dp.y * p.y);
           den[g] = fma(p.x, p.x, p.y * p.y);
         }
       }
@@ -239,8 +245,6 @@ __global__ void __launch_bounds__(kMuThreads) k_mu_search(MuState* io, const dou
         }
       acc += num[0] / den[0];
     }
-    for (long long t = first; t < (long long)Nk * N; t += S)
-      tail += im_digamma(Nw + 0.5, (rmu - eig[t]) / (2.0 * kPi * temp));
     const double s = grid_sum(fma(2.0 * temp, acc, tail / kPi), part, bar, round, dead);
     ++round;
     return 0.5 * N + s / Nk;
@@ -344,9 +348,9 @@ __global__ void __launch_bounds__(kMuThreads) k_mu_search(MuState* io, const dou
 
 template <int N>
 void mu_launch(MuState* io, const double2* cp, double center, const double* eig, double fill, double esterr, double temp,
-               int Nk, int Nw, double* part, unsigned* bar, unsigned blocks) {
+               int Nk, int Nw, double* part, unsigned* bar, unsigned blocks, unsigned threads) {
   void* args[] = {&io, &cp, &center, &eig, &fill, &esterr, &temp, &Nk, &Nw, &part, &bar};
-  PGB_CUDA(cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(&k_mu_search<N>), dim3(blocks), dim3(kMuThreads),
+  PGB_CUDA(cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(&k_mu_search<N>), dim3(blocks), dim3(threads),
                                        args, 0, ctx().stream));
 }
 
@@ -369,16 +373,22 @@ void mu_search(MuState& s, const double2* cp, double center, const double* eig, 
                int Nk, int Nw, int Norb) {
   cudaStream_t st = ctx().stream;
   const long long K = (long long)Nk * Nw;
-  // one block per SM at most (co-residency with other contexts' kernels), and
-  // no more blocks than give each thread a few points
-  const unsigned blocks = (unsigned)std::max(1LL, std::min<long long>(ctx().num_sms, (K + 4 * kMuThreads - 1) / (4 * kMuThreads)));
+  // One block per SM at most (co-residency with other contexts' kernels).  A
+  // trial is bound by the FP64 pipe, which a few warps per SM keep busy, so a small
+  // problem spreads over the SMs (two warps at least) before a block gets more:
+  // 16640 points at five orbitals on 9 blocks of 16 warps took 31 us a trial,
+  // 12 us on 130 of two; 526336 at one orbital on 152 of 16 27 us, 21 us on 152 of 8.
+  const long long per = 64 * 2;
+  const unsigned blocks = (unsigned)std::max(1LL, std::min<long long>(ctx().num_sms, (K + per - 1) / per));
+  const long long want = (K + 2LL * blocks - 1) / (2LL * blocks);
+  const unsigned threads = (unsigned)std::max(64LL, std::min<long long>(kMuThreads, (want + 31) / 32 * 32));
   DBuf<MuState> io(1);
   DBuf<double> part(2 * blocks);
   DBuf<unsigned> bar(1);
   bar.zero();
   io.upload(&s, 1);
   switch (Norb) {
-#define PGB_MU(n_) case n_: mu_launch<n_>(io.p, cp, center, eig, fill, esterr, temp, Nk, Nw, part.p, bar.p, blocks); break;
+#define PGB_MU(n_) case n_: mu_launch<n_>(io.p, cp, center, eig, fill, esterr, temp, Nk, Nw, part.p, bar.p, blocks, threads); break;
     PGB_MU(1) PGB_MU(2) PGB_MU(3) PGB_MU(4) PGB_MU(5) PGB_MU(6) PGB_MU(7) PGB_MU(8)
 #undef PGB_MU
     default: throw Error("Norb above the engine limit of 8 orbitals");
