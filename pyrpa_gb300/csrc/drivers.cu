@@ -25,22 +25,66 @@ namespace {
 // the statistics of the last solve called from this thread
 thread_local LastStats g_stats;
 
+// Laps of the stage timers of one call, read together at its end: a lap read when it
+// closes makes the host wait for the device between any two stages, and the device
+// then waits for the host (0.3 of 2.3 ms per iteration at one orbital, 32x32
+// points and 1024 frequencies).
+struct TimerScope {
+  struct Lap {
+    cudaEvent_t a, b;
+    double* into;
+  };
+  static constexpr size_t kMaxOpen = 256;
+  std::vector<Lap> open;
+  TimerScope* outer;
+  TimerScope();
+  ~TimerScope();
+  void flush() {
+    for (const Lap& l : open) {
+      float ms = 0;
+      if (cudaEventSynchronize(l.b) == cudaSuccess && cudaEventElapsedTime(&ms, l.a, l.b) == cudaSuccess) *l.into += ms;
+      cudaEventDestroy(l.a);
+      cudaEventDestroy(l.b);
+    }
+    open.clear();
+  }
+};
+thread_local TimerScope* t_laps = nullptr;
+TimerScope::TimerScope() : outer(t_laps) { t_laps = this; }
+TimerScope::~TimerScope() {
+  flush();
+  t_laps = outer;
+}
+
 struct Timer {
-  cudaEvent_t a, b;
-  Timer() {
-    cudaEventCreate(&a);
-    cudaEventCreate(&b);
-  }
+  cudaEvent_t a = nullptr;
   ~Timer() {
-    cudaEventDestroy(a);
-    cudaEventDestroy(b);
+    if (a) cudaEventDestroy(a);
   }
-  void start() { cudaEventRecord(a, ctx().stream); }
+  void start() {
+    if (!a) cudaEventCreate(&a);
+    cudaEventRecord(a, ctx().stream);
+  }
+  // adds the time since start() to `into`, at the end of the innermost TimerScope
+  // of the thread or, outside of one, now
+  void stop(double& into) {
+    cudaEvent_t b = nullptr;
+    cudaEventCreate(&b);
+    cudaEventRecord(b, ctx().stream);
+    TimerScope now;
+    TimerScope& s = now.outer ? *now.outer : now;
+    s.open.push_back({a, b, &into});
+    a = nullptr;
+    if (s.open.size() >= TimerScope::kMaxOpen) s.flush();
+  }
   double stop() {
+    cudaEvent_t b = nullptr;
+    cudaEventCreate(&b);
     cudaEventRecord(b, ctx().stream);
     cudaEventSynchronize(b);
     float ms = 0;
     cudaEventElapsedTime(&ms, a, b);
+    cudaEventDestroy(b);
     return ms;
   }
 };
@@ -358,7 +402,7 @@ double stage_chi0(Inputs& in, const FlexParams& a, const double2* G, double mu, 
   tm.start();
   TailRef tail{in.eig.p, in.uni.p, mu};
   chi0<R>(g, in.p, G, a.temp, a.sw_tail ? &tail : nullptr, chi, !compact_chi(in));
-  g_stats.t_chi0 += tm.stop();
+  tm.stop(g_stats.t_chi0);
   double sdw = 0, cdw = 0;
   int qs = 0, qc = 0;
   tm.start();
@@ -374,7 +418,7 @@ double stage_chi0(Inputs& in, const FlexParams& a, const double2* G, double mu, 
     log("[FLEX] Stoner factor=%10.6f >= 1: rescaling chi0 to%7.4f\n", sdw, rt);
     scale_chi<R>(chi, g.K * in.Nchi * in.Nchi, rt / sdw);
   }
-  g_stats.t_stoner += tm.stop();
+  tm.stop(g_stats.t_stoner);
   return sdw;
 }
 // the vertex of nmat matrices (element stride nmat): in the real basis of an
@@ -394,7 +438,7 @@ void stage_vertex(Inputs& in, cx<R>* chi) {
   } else {
     PGB_CHECK(vertex_of<R>(in, chi, in.g.K, 0, false), "zgesv failed in V_sigma");
   }
-  g_stats.t_vertex += tm.stop();
+  tm.stop(g_stats.t_vertex);
 }
 template <typename R>
 void stage_sigma(Inputs& in, const FlexParams& a, const double2* G, const cx<R>* chi, double2* sig) {
@@ -402,7 +446,7 @@ void stage_sigma(Inputs& in, const FlexParams& a, const double2* G, const cx<R>*
   tm.start();
   if (in.soc) sigma<R>(in.g, in.p, G, chi, in.Vneg.p, nullptr, a.temp, sig);  // static slot -V
   else sigma<R>(in.g, in.p, G, chi, in.S.p, in.C.p, a.temp, sig);
-  g_stats.t_sigma += tm.stop();
+  tm.stop(g_stats.t_sigma);
 }
 
 // the chi buffer of each bulk type, allocated on first use
@@ -471,7 +515,7 @@ double flex_bulk(Inputs& in, const FlexParams& a, const double2* G, double mu, c
     PGB_CUDA(cudaMemcpy2DAsync(low.p, nlow * sizeof(cdf), c0, K * sizeof(cdf), nlow * sizeof(cdf), nel,
                                cudaMemcpyDeviceToDevice, ctx().stream));
     PGB_CHECK(vertex_of<dfl>(in, low.p, nlow, 0, false), "zgesv failed in V_sigma");
-    g_stats.t_vertex += tl.stop();
+    tl.stop(g_stats.t_vertex);
   }
   void* cv = b.get(sp.vertex, KC);
   convert_chi(in, cv, sp.vertex, c0, sp.chi0);
@@ -571,6 +615,7 @@ int fp32_stage_mask() {
 // mix_judge_prec); convergence is only declared in the judging phase.
 void mkself_core(Inputs& in, const FlexParams& a, double2* sig_out, double* mu_out, const double2* seed,
                  double seed_mu, double seed_mu_old, int prec) {
+  TimerScope laps;
   cudaStream_t st = ctx().stream;
   const Geom& g = in.g;
   const Pairs& p = in.p;
@@ -725,7 +770,7 @@ void mkself_core(Inputs& in, const FlexParams& a, double2* sig_out, double* mu_o
     tm.start();
     if (a.sub_sigma > 0) hf_subtract(sig.p, Nk, Nw, Norb, (int)a.sub_sigma);
     compare_sigma();
-    g_stats.t_diis += tm.stop();
+    tm.stop(g_stats.t_diis);
     g_stats.esterr = esterr;
     g_stats.iterations = it;
     g_stats.stoner = maxchi0s;
@@ -765,21 +810,21 @@ void mkself_core(Inputs& in, const FlexParams& a, double2* sig_out, double* mu_o
     }
     tm.start();
     renew_mu();
-    g_stats.t_mu += tm.stop();
+    tm.stop(g_stats.t_mu);
     tm.start();
     PGB_CHECK(dyson(G.p, sig.p, H.p, mu, a.temp, Nk, Nw, Norb), "singular G^-1 in the Dyson step");
     PGB_CUDA(cudaMemcpyAsync(sig0.p, sig.p, KE * sizeof(double2), cudaMemcpyDeviceToDevice, st));
-    g_stats.t_dyson += tm.stop();
+    tm.stop(g_stats.t_dyson);
   }
   if (prec == kPrecMixed && phase == 2 && esterr < a.eps) {
     // full steps of the judging map from the converged Sigma, without DIIS
     for (int k = 0; k < judge_r.polish; ++k) {
       tm.start();
       renew_mu();
-      g_stats.t_mu += tm.stop();
+      tm.stop(g_stats.t_mu);
       tm.start();
       PGB_CHECK(dyson(G.p, sig.p, H.p, mu, a.temp, Nk, Nw, Norb), "singular G^-1 in the Dyson step");
-      g_stats.t_dyson += tm.stop();
+      tm.stop(g_stats.t_dyson);
       cp_current = false;
       maxchi0s = flex_bulk(in, a, G.p, mu, prec_of(2), bufs, sig.p);
       if (a.sub_sigma > 0) hf_subtract(sig.p, Nk, Nw, Norb, (int)a.sub_sigma);
@@ -799,7 +844,7 @@ void mkself_core(Inputs& in, const FlexParams& a, double2* sig_out, double* mu_o
   }
   tm.start();
   renew_mu();
-  g_stats.t_mu += tm.stop();
+  tm.stop(g_stats.t_mu);
   PGB_CUDA(cudaMemcpyAsync(sig_out, sig.p, KE * sizeof(double2), cudaMemcpyDeviceToDevice, st));
   sync();
   *mu_out = mu;
@@ -827,14 +872,17 @@ void run_mkself(const MkselfArgs& a, int prec) {
 // pass 1 from the initial gap, exit at a Ritz value >= 0.1, else pass 2 with
 // the shift -lambda_- and that Ritz vector deflated.  apply_op/inner/norm/init
 // define the operator and the inner product of the caller's vector space of n
-// elements (kw, Nkw: the weights of that inner product); the normalized Ritz vector goes to delta_out, lambda is returned.
+// elements (kw, Nkw: the weights of that inner product).  Nherm > 0: the vectors
+// are Nherm x Nherm matrices (a + Nherm b slowest), Hermitian for the initial gap
+// and after every application, so the coefficients are real and the space
+// stays Hermitian, as long as its Ritz vectors are real ones.  The normalized Ritz vector goes to delta_out, lambda is returned.
 // With a restart tolerance set, refine(residual / |lambda|) is asked after
 // every cycle whether the operator has just been replaced by a more precise
 // one (true: the pass restarts on it from the current Ritz vector, whatever
 // the residual).
 template <class Apply, class Inner, class Norm, class Init, class Refine>
-double arnoldi_two_pass(int m, long long KE, const double* kw, int Nkw, Apply apply_op, Inner inner, Norm norm,
-                        Init init_vec, double2* delta_out, Refine refine) {
+double arnoldi_two_pass(int m, long long KE, int Nherm, const double* kw, int Nkw, Apply apply_op, Inner inner,
+                        Norm norm, Init init_vec, double2* delta_out, Refine refine) {
   cudaStream_t st = ctx().stream;
   double lambda_out = 0.0;
   DBuf<double2> w(KE);
@@ -842,6 +890,7 @@ double arnoldi_two_pass(int m, long long KE, const double* kw, int Nkw, Apply ap
   std::vector<DBuf<double2>> V(m);
   for (auto& v : V) v.alloc(KE);
   DBuf<double2> D(KE);
+  bool herm = Nherm > 0;
   auto arnoldi = [&](double shift, const double2* defl, std::vector<double2>& Hm, int& m_act) {
     Hm.assign((size_t)(m + 1) * m, make_double2(0, 0));
     m_act = m;
@@ -856,7 +905,13 @@ double arnoldi_two_pass(int m, long long KE, const double* kw, int Nkw, Apply ap
       for (int ii = 0; ii <= j; ++ii) xs.push_back(V[ii].p);
       std::vector<double2> h(xs.size());
       double norm2 = 0;
-      gram_schmidt(w.p, xs.data(), (int)xs.size(), kw, Nkw, KE, h.data(), &norm2);
+      if (herm) {
+        std::vector<double> hr(xs.size());
+        gram_schmidt_herm(w.p, xs.data(), (int)xs.size(), kw, Nkw, KE / (Nherm * Nherm), Nherm, hr.data(), &norm2);
+        for (size_t i = 0; i < h.size(); ++i) h[i] = make_double2(hr[i], 0.0);
+      } else {
+        gram_schmidt(w.p, xs.data(), (int)xs.size(), kw, Nkw, KE, h.data(), &norm2);
+      }
       for (int ii = 0; ii <= j; ++ii) Hm[ii * m + j] = h[ii + (defl ? 1 : 0)];
       const double beta = std::sqrt(norm2);
       Hm[(j + 1) * m + j] = make_double2(beta, 0);
@@ -864,7 +919,9 @@ double arnoldi_two_pass(int m, long long KE, const double* kw, int Nkw, Apply ap
         m_act = j + 1;
         break;
       }
-      if (j < m - 1) scal_to(V[j + 1].p, 1.0 / beta, w.p, KE);
+      if (j >= m - 1) continue;
+      if (herm) scal_herm(V[j + 1].p, 1.0 / beta, w.p, KE / (Nherm * Nherm), Nherm);
+      else scal_to(V[j + 1].p, 1.0 / beta, w.p, KE);
     }
   };
   // Ritz vector of lam into out (unit norm); returns the Ritz residual
@@ -874,6 +931,17 @@ double arnoldi_two_pass(int m, long long KE, const double* kw, int Nkw, Apply ap
     for (int i = 0; i < m_act; ++i)
       for (int j = 0; j < m_act; ++j) Hs[i * m_act + j] = Hm[i * m + j];
     std::vector<double2> y = eigvec(Hs, m_act, lam);
+    if (herm) {
+      // of a pair of complex eigenvalues: the restart leaves the Hermitian vectors
+      double re = 0, im = 0;
+      for (const auto& v : y) {
+        re = std::max(re, std::fabs(v.x));
+        im = std::max(im, std::fabs(v.y));
+      }
+      if (im <= 1.0e-9 * re)
+        for (auto& v : y) v.y = 0;
+      else herm = false;
+    }
     std::vector<const double2*> xs(m_act);
     for (int i = 0; i < m_act; ++i) xs[i] = V[i].p;
     lincomb(out, xs.data(), y.data(), m_act, KE);
@@ -950,7 +1018,7 @@ double arnoldi_two_pass(int m, long long KE, const double* kw, int Nkw, Apply ap
     const double shift = -lambda1;
     init_vec(V[0].p);
     double2 h = inner(delta1.p, V[0].p);
-    axpy(V[0].p, make_double2(-h.x, -h.y), delta1.p, KE);
+    axpy(V[0].p, make_double2(-h.x, herm ? 0.0 : -h.y), delta1.p, KE);
     const double b0 = norm(V[0].p);
     if (!(b0 >= 1.0e-14)) {
       // the operator has no component outside the pass-1 direction
@@ -981,7 +1049,7 @@ double arnoldi_two_pass(int m, long long KE, const double* kw, int Nkw, Apply ap
 template <class Apply, class Inner, class Norm, class Init>
 double arnoldi_two_pass(int m, long long KE, const double* kw, int Nkw, Apply apply_op, Inner inner, Norm norm,
                         Init init_vec, double2* delta_out) {
-  return arnoldi_two_pass(m, KE, kw, Nkw, apply_op, inner, norm, init_vec, delta_out, [](double) { return false; });
+  return arnoldi_two_pass(m, KE, 0, kw, Nkw, apply_op, inner, norm, init_vec, delta_out, [](double) { return false; });
 }
 
 // FP32 start of the double-float Eliashberg stage of the mixed schedule:
@@ -1012,12 +1080,18 @@ bool vertex_delta(const Inputs& in, cx<R>* chi, int mode, bool full) {
   }
 }
 
+// The gap's Krylov space with real coefficients.  Not in FP64: the two passes of a
+// fixed size amplify another rounding of the coefficients to 1e-9 .. 2e-8 of the gap
+// there, which is above that operator's own error; below the others'.
+template <typename R> constexpr bool hermitian_basis() { return !std::is_same<R, double>::value; }
+
 // ============================================================ lin_eliash ==
 // chi (device, cx<R>) is overwritten with the pairing vertex V_Delta; if
 // chi_host is given, V_Delta is also copied back there (feliash.f90:61).
 template <typename R>
 double eliash_core(Inputs& in, cx<R>* chi, const double2* G, const double* init, const double* prt,
                    const EliashParams& a, double2* delta_out, double2* chi_host) {
+  TimerScope laps;
   cudaStream_t st = ctx().stream;
   const Geom& g = in.g;
   const Pairs& p = in.p;
@@ -1038,7 +1112,7 @@ double eliash_core(Inputs& in, cx<R>* chi, const double2* G, const double* init,
     Timer tv;
     tv.start();
     PGB_CHECK(vertex_delta<R>(in, chi, singlet ? 1 : 2, chi_host || !even_delta), "zgesv failed in V_delta");
-    g_stats.t_vertex += tv.stop();
+    tv.stop(g_stats.t_vertex);
     if (chi_host) {
       DBuf<double2> tmp(KC);
       if (std::is_same<R, double>::value)
@@ -1100,7 +1174,7 @@ double eliash_core(Inputs& in, cx<R>* chi, const double2* G, const double* init,
       mkfk(F.p, G, v, K, Norb);
       mkdelta<R>(g, p, F.p, chi, S.p, C.p, prt, singlet, scale, out, &cache, nullptr, even_delta);
     }
-    g_stats.t_apply += ta.stop();
+    ta.stop(g_stats.t_apply);
     g_stats.applies += 1;
   };
   auto refine = [&](double rel) {
@@ -1126,7 +1200,8 @@ double eliash_core(Inputs& in, cx<R>* chi, const double2* G, const double* init,
   double lambda_out = 0.0;
   const int m = (int)a.arnoldi_m;
   if (m > 0) {
-    lambda_out = arnoldi_two_pass(m, KE, g.kweight.p, Nk, apply_op, inner, norm, init_vec, delta_out, refine);
+    lambda_out = arnoldi_two_pass(m, KE, hermitian_basis<R>() ? Norb : 0, g.kweight.p, Nk, apply_op, inner, norm,
+                                  init_vec, delta_out, refine);
     PGB_CHECK(!chi32, "the FP32 Arnoldi cycles did not hand over to double-float");
   } else {
     // shifted power method with deflation (feliash.f90:66-140)
@@ -1732,7 +1807,7 @@ void run_lin_eliash_soc(const LinEliashSocArgs& a) {
     Timer tv;
     tv.start();
     PGB_CHECK(vertex_soc(chi.p, g.K, Nchi, in.V.p), "zgesv failed in V_delta");  // chi -> V_Delta
-    g_stats.t_vertex += tv.stop();
+    tv.stop(g_stats.t_vertex);
   }
   chi.download(a.chi, KC);
   G.upload(a.Gk, KE);
@@ -1751,7 +1826,7 @@ void run_lin_eliash_soc(const LinEliashSocArgs& a) {
     ta.start();
     mkfk_soc(F.p, G.p, v, fm, g, gap_sym);
     mkdelta_soc(g, in.p, fm, F.p, chi.p, hV, invschi, gap_sym, scale, out);
-    g_stats.t_apply += ta.stop();
+    ta.stop(g_stats.t_apply);
     g_stats.applies += 1;
   };
   const int Nkf = (int)fm.Nkall;

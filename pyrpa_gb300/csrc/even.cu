@@ -367,6 +367,31 @@ std::shared_ptr<Even> make_even(const Geom& g, const Pairs& p, const double* S, 
   put(ev->mem, mem);
   put(ev->memcj, cj);
   put(ev->nmem, nm);
+  std::vector<int> elt;
+  for (int x : ev->sym_el) elt.push_back(x / No + No * (x % No));
+  put(ev->d_sym_el, ev->sym_el);
+  put(ev->d_sym_elt, elt);
+  std::vector<EvenPair> hp;
+  for (const EvenClass& c : ev->cls) {
+    const int a13 = p.o1[c.l], b13 = p.o1[c.m], a42 = p.o2[c.m], b42 = p.o2[c.l];
+    hp.push_back(EvenPair{ev->sym_of[a13 + No * b13], ev->sym_of[a42 + No * b42], a13, b13, a42, b42});
+  }
+  ev->pairs.alloc(hp.size());
+  ev->pairs.upload(hp.data(), hp.size());
+  std::vector<EvenTerm> terms;
+  std::vector<int> tb(1, 0);
+  if (p.sigma.size() == (size_t)No * No) {
+    for (int e : ev->sym_el) {
+      for (const Term& t : p.sigma[e]) {
+        const int x = t.m + n * t.l;
+        terms.push_back(EvenTerm{ev->cls_of[x], ev->sym_of[t.ef], ev->cj_of[x]});
+      }
+      tb.push_back((int)terms.size());
+    }
+    ev->sig_terms.alloc(std::max<size_t>(1, terms.size()));
+    ev->sig_terms.upload(terms.data(), terms.size());
+    put(ev->sig_tb, tb);
+  }
   if (S && C) {
     put(ev->d_vin, ev->vin);
     put(ev->d_vout, ev->vout);

@@ -46,6 +46,15 @@ struct EvenClass {
   int mem[4], cj[4];
 };
 
+struct EvenPair {
+  int f13, f42;  // a <= b copies of G13 and G42
+  int a13, b13, a42, b42;  // their orbitals
+};
+struct EvenTerm {
+  int c, f;  // class of the vertex element, fermionic copy
+  int rev;   // bit 0: the vertex at the reversed tau, bit 1: the fermionic copy (antiperiodic)
+};
+
 struct Even {
   int nx = 1, ny = 1, nz = 1, Nw = 1, H = 1, nsym = 1;
   bool three_d = false;
@@ -60,6 +69,10 @@ struct Even {
   int nzp = 0;
   DBuf<int> cls_el;                 // device: el of each class
   DBuf<int> mem, memcj, nmem;       // device: members (4 per class)
+  DBuf<int> d_sym_el, d_sym_elt;    // device: sym_el, and the transposed elements
+  DBuf<EvenPair> pairs;             // device: per class
+  DBuf<EvenTerm> sig_terms;         // device: the terms of Sigma, by a <= b output
+  DBuf<int> sig_tb;                 // and the first of each output
   bool vertex_ok = false;           // the real-basis vertex applies (constants in vs/vc)
   std::vector<double> Sb, Cb;       // S and C in the real basis, row-major
   std::vector<int> vin, vout;       // index tables of the real basis (see even_impl.cuh)
@@ -91,9 +104,9 @@ bool even_chi(const Geom& g, const Even& ev, const double2* chi, double tol);
 // chi0, Sigma, V and Delta of an even model.  full: every element is written;
 // otherwise the class representatives, and every element at nu = 0.
 template <typename R>
-void chi0_even(const Geom& g, const Pairs& p, const double2* G, double temp, const TailRef* tail, cx<R>* chi, bool full);
+void chi0_even(const Geom& g, const double2* G, double temp, const TailRef* tail, cx<R>* chi, bool full);
 template <typename R>
-void sigma_even(const Geom& g, const Pairs& p, const double2* G, const cx<R>* V, const double* S, const double* C,
+void sigma_even(const Geom& g, const double2* G, const cx<R>* V, const double* S, const double* C,
                 double temp, double2* sig);
 // Delta = scale sum_kq V_Delta F (singlet, orbitals of one parity) from F in
 // FP64 or, when given, in the bulk type

@@ -351,38 +351,50 @@ void fermi_transform(const Even& ev, SpaceArgs<R> a, cx<R>* F, int narr, bool bu
   count_launch("even_phase");
 }
 
-// The reference bubble's tau kernels on the half grid (k_ref_tau): element
-// (a <= b) at slots 2s and 2s+1 as the two parts of one number
+// The reference bubble's tau kernel on the half grid (k_ref_tau's A): element
+// (a <= b) at slots 2s and 2s+1 as the two parts of one number.  Its B is
+// B(tau) = -A(beta - tau), read off A by k_even_product.
 template <typename R, typename T>
-__global__ void k_even_ref_tau(cx<R>* A, cx<R>* B, const T* gp, const T* gm, const cx<T>* cf, const int* h_irr,
-                               const int* sym_el, int H, int Nk, int No, int Nw) {
+__global__ void k_even_ref_tau(cx<R>* A, const T* gp, const cx<T>* cf, const int* h_irr, const int* sym_el, int H, int Nk,
+                               int No, int Nw) {
   MeshTau q;
   if (!mesh_tau(H, Nw, q)) return;
   const int k = h_irr[q.r];
   const cx<T>* c = cf + ((long long)k * No * No + sym_el[blockIdx.y]) * No;
   const long long o = (long long)blockIdx.y * H * Nw + q.r;
   for (int s = q.t0; s < q.t1; ++s) {
-    T a[2] = {(T)0, (T)0}, b[2] = {(T)0, (T)0};
+    T a[2] = {(T)0, (T)0};
 #pragma unroll
     for (int h = 0; h < 2; ++h)
-      for (int n = 0; n < No; ++n) {
-        const long long g = ((long long)(2 * s + h) * No + n) * Nk + k;
-        a[h] += gp[g] * c[n].x;
-        b[h] += gm[g] * c[n].x;
-      }
+      for (int n = 0; n < No; ++n) a[h] += gp[((long long)(2 * s + h) * No + n) * Nk + k] * c[n].x;
     A[o + (long long)H * s] = cmk<R>((R)a[0], (R)a[1]);
-    B[o + (long long)H * s] = cmk<R>((R)b[0], (R)b[1]);
   }
 }
 
-struct EvenPair {
-  int f13, f42;  // a <= b copies of G13 and G42
-};
+// tau = 0 jump of the classes (tail_jump) from the band sums rb, in the bulk type
+template <typename R>
+__global__ void k_even_jump(cx<R>* J, const EvenPair* pairs, const double2* rb, int No, int nc) {
+  const int c = blockIdx.x * blockDim.x + threadIdx.x;
+  if (c >= nc) return;
+  const EvenPair p = pairs[c];
+  double2 v = make_double2(0, 0);
+  if (p.a13 == p.b13) v = v + rb[p.a42 + No * p.b42];
+  if (p.a42 == p.b42) v = v - rb[p.a13 + No * p.b13];
+  J[c] = cmk<R>((R)v.x, (R)v.y);
+}
+
+// static slots a S + b C of the classes' vertex
+template <typename R>
+__global__ void k_even_static(R* out, const double* S, const double* C, const int* cls_el, double a, double b, int nc) {
+  const int c = blockIdx.x * blockDim.x + threadIdx.x;
+  if (c < nc) out[c] = (R)(__dmul_rn(a, S[cls_el[c]]) + __dmul_rn(b, C[cls_el[c]]));
+}
+
 // chi0(r, tau) of the classes: G13(tau) G42(-tau) (both fermionic phases gone:
 // their product is -1, except at tau = 0), minus G0's, minus the analytic bubble
 template <typename R>
-__global__ void k_even_product(cx<R>* out, const cx<R>* F, const cx<R>* F0, const cx<R>* A, const cx<R>* B,
-                               const EvenPair* pairs, int H, int Nw, const int* pos, const int* lt, R sc, R sr) {
+__global__ void k_even_product(cx<R>* out, const cx<R>* F, const cx<R>* F0, const cx<R>* A,
+                               const EvenPair* pairs, int H, int Nw, const int* pos, const int* lt, R sc, R sr, R n0) {
   const EvenPair pr = pairs[blockIdx.y];
   const long long P = (long long)H * Nw;
   const cx<R>*a13 = F + pr.f13 * P, *b42 = F + pr.f42 * P;
@@ -404,19 +416,18 @@ __global__ void k_even_product(cx<R>* out, const cx<R>* F, const cx<R>* F0, cons
     vx = sc * vx;
     vy = sc * vy;
     if (A) {
-      const long long is = q.r + (long long)H * s;
-      const cx<R> ta = A[pr.f13 * P + is], tb = B[pr.f42 * P + is];
-      vx = vx - sr * (ta.x * tb.x);
-      vy = vy - sr * (ta.y * tb.y);
+      // B at slots 2s, 2s+1: minus A at slots 2(Nw-s), 2(Nw-1-s)+1; at tau = 0
+      // the projectors' completeness, A(beta) = -delta_ab N delta_r0 - A(0)
+      const cx<R> ta = A[pr.f13 * P + q.r + (long long)H * s], *u = A + pr.f42 * P + q.r;
+      R bx = -u[(long long)H * (s ? Nw - s : 0)].x;
+      if (s == 0) bx = (pr.a42 == pr.b42 && q.r == 0 ? n0 : (R)0) - bx;
+      vx = vx - sr * (ta.x * bx);
+      vy = vy + sr * (ta.y * u[(long long)H * (Nw - 1 - s)].y);
     }
     o[i] = cmk<R>(vx, vy);
   }
 }
 
-struct EvenTerm {
-  int c, f;  // class of the vertex element, fermionic copy
-  int rev;   // bit 0: the vertex at the reversed tau, bit 1: the fermionic copy (antiperiodic)
-};
 // Fermionic outputs sum_t w_t(r, tau) g_t(r, tau) of real factors, with the
 // half-integer phase of the backward transform; the output runs fastest over the blocks, so
 // that the outputs of one tile of points share its w and g in L2
@@ -929,20 +940,18 @@ template <typename R> int even_batch(const Even& ev) {
 }
 
 template <typename R>
-void chi0_even(const Geom& g, const Pairs& p, const double2* G, double temp, const TailRef* tail, cx<R>* chi, bool full) {
+void chi0_even(const Geom& g, const double2* G, double temp, const TailRef* tail, cx<R>* chi, bool full) {
   const Even& ev = *g.even;
   cudaStream_t st = ctx().stream;
   const int ns = ev.nsym, No = g.Norb, H = ev.H, Nw = ev.Nw;
   const size_t P = (size_t)H * Nw;
-  DBuf<int> sel(ns);
-  sel.upload(ev.sym_el.data(), ns);
-  DBuf<cx<R>> F(ns * P), F0, A, B, sawc, dJ;
+  DBuf<cx<R>> F(ns * P), F0, A, sawc, dJ;
   SpaceArgs<R> a{};
   a.Nk = g.Nk;
   a.src = G;
-  a.el = sel.p;
+  a.el = ev.d_sym_el.p;
   fermi_transform<R>(ev, a, F.p, ns, false, st);
-  std::vector<cx<R>> hJ(ev.cls.size());
+  const int nc = (int)ev.cls.size();
   if (tail) {
     DBuf<double2> G0((size_t)g.K * No * No);
     green0(G0.p, tail->eig, tail->uni, tail->mu, temp, g.Nk, g.Nw, No, true);
@@ -952,36 +961,23 @@ void chi0_even(const Geom& g, const Pairs& p, const double2* G, double temp, con
     G0.release();
     using T = typename std::conditional<std::is_same<R, float>::value, float, double>::type;
     TailTables<T> tt;
-    tail_tables<T>(g, *tail, temp, tt);
+    tail_tables<T>(g, *tail, temp, tt, false);
     A.alloc(ns * P);
-    B.alloc(ns * P);
-    k_even_ref_tau<R, T><<<mesh_tau_grid(H, Nw, ns), 256, 0, st>>>(A.p, B.p, tt.gp.p, tt.gm.p, tt.projectors(),
-                                                                  ev.h_irr.p, sel.p, H, g.Nk, No, Nw);
+    k_even_ref_tau<R, T><<<mesh_tau_grid(H, Nw, ns), 256, 0, st>>>(A.p, tt.gp.p, tt.projectors(), ev.h_irr.p,
+                                                                  ev.d_sym_el.p, H, g.Nk, No, Nw);
     count_launch("even_ref_tau");
     SpaceArgs<R> r{};
     r.Nk = g.Nk;
-    for (DBuf<cx<R>>* x : {&A, &B}) {
-      r.src = x->p;
-      even_forward<R, kInPlain>(ev, r, x->p, ns, false, st);
-    }
-    const std::vector<double2> rb = tail_rhobar(g, *tail, tt.ff.p);
-    for (size_t c = 0; c < ev.cls.size(); ++c) {
-      const double2 J = tail_jump(p, rb, No, ev.cls[c].l, ev.cls[c].m);
-      hJ[c] = cmk<R>((R)J.x, (R)J.y);
-    }
-    dJ.alloc(hJ.size());
-    dJ.upload(hJ.data(), hJ.size());
+    r.src = A.p;
+    even_forward<R, kInPlain>(ev, r, A.p, ns, false, st);
+    DBuf<double2> rb(No * No);
+    tail_rhobar(g, *tail, tt.ff.p, rb.p);
+    dJ.alloc(nc);
+    k_even_jump<R><<<(nc + 127) / 128, 128, 0, st>>>(dJ.p, ev.pairs.p, rb.p, No, nc);
+    count_launch("even_jump");
     sawc.alloc(g.Nw);
     narrow<R>(sawc.p, tail_sawtooth(g, temp), g.Nw);
   }
-  std::vector<EvenPair> hp(ev.cls.size());
-  for (size_t c = 0; c < hp.size(); ++c) {
-    const int l = ev.cls[c].l, m = ev.cls[c].m;
-    hp[c] = EvenPair{ev.sym_of[p.o1[l] + No * p.o1[m]], ev.sym_of[p.o2[m] + No * p.o2[l]]};
-  }
-  DBuf<EvenPair> dp(hp.size());
-  dp.upload(hp.data(), hp.size());
-  const int nc = (int)ev.cls.size();
   const int ch = std::min(nc, even_batch<R>(ev));
   DBuf<cx<R>> T(ch * P), T2;
   if (ev.three_d) T2.alloc(ch * P);
@@ -995,8 +991,8 @@ void chi0_even(const Geom& g, const Pairs& p, const double2* G, double temp, con
   o.full = full ? 1 : 0;
   for (int c0 = 0; c0 < nc; c0 += ch) {
     const int n = std::min(ch, nc - c0);
-    k_even_product<R><<<mesh_tau_grid(H, Nw, n), 256, 0, st>>>(T.p, F.p, F0.p, A.p, B.p, dp.p + c0, H, Nw, ft.d_pos(3),
-                                                               ft.d_logical(3), sc, sr);
+    k_even_product<R><<<mesh_tau_grid(H, Nw, n), 256, 0, st>>>(T.p, F.p, F0.p, A.p, ev.pairs.p + c0, H, Nw, ft.d_pos(3),
+                                                               ft.d_logical(3), sc, sr, (R)(double)g.Nkall);
     count_launch("even_product");
     o.mem = ev.mem.p + 4 * c0;
     o.memcj = ev.memcj.p + 4 * c0;
@@ -1004,17 +1000,18 @@ void chi0_even(const Geom& g, const Pairs& p, const double2* G, double temp, con
     o.J = tail ? dJ.p + c0 : nullptr;
     even_backward<R, kInPostBoson, kOutChi>(ev, o, T.p, T2.p, n, st);
   }
-  sync();  // the host-built tables above go out of scope
 }
 
-// transforms of the classes' vertex elements V, static slots stat (host, per class)
+// transforms of the classes' vertex elements V, static slots a S + b C
 template <typename R>
-void vertex_transforms(const Geom& g, const cx<R>* V, const std::vector<R>& stat, cx<R>* W, cudaStream_t st) {
+void vertex_transforms(const Geom& g, const cx<R>* V, const double* S, const double* C, double wS, double wC, cx<R>* W,
+                       cudaStream_t st) {
   const Even& ev = *g.even;
   const int nc = (int)ev.cls.size(), ch = even_batch<R>(ev);
   const size_t P = (size_t)ev.H * ev.Nw;
   DBuf<R> dstat(nc);
-  dstat.upload(stat.data(), nc);
+  k_even_static<R><<<(nc + 127) / 128, 128, 0, st>>>(dstat.p, S, C, ev.cls_el.p, wS, wC, nc);
+  count_launch("even_static");
   SpaceArgs<R> b{};
   b.Nk = g.Nk;
   b.src = V;
@@ -1026,57 +1023,34 @@ void vertex_transforms(const Geom& g, const cx<R>* V, const std::vector<R>& stat
 }
 
 template <typename R>
-void sigma_even(const Geom& g, const Pairs& p, const double2* G, const cx<R>* V, const double* S, const double* C,
+void sigma_even(const Geom& g, const double2* G, const cx<R>* V, const double* S, const double* C,
                 double temp, double2* sig) {
   const Even& ev = *g.even;
   cudaStream_t st = ctx().stream;
-  const int ns = ev.nsym, No = g.Norb, Nchi = g.Nchi, H = ev.H, Nw = ev.Nw, nc = (int)ev.cls.size();
+  const int ns = ev.nsym, H = ev.H, Nw = ev.Nw, nc = (int)ev.cls.size();
   const size_t P = (size_t)H * Nw;
-  std::vector<double> hS(Nchi * Nchi), hC(Nchi * Nchi);
-  PGB_CUDA(cudaMemcpyAsync(hS.data(), S, sizeof(double) * hS.size(), cudaMemcpyDeviceToHost, st));
-  PGB_CUDA(cudaMemcpyAsync(hC.data(), C, sizeof(double) * hC.size(), cudaMemcpyDeviceToHost, st));
-  sync();
-  std::vector<R> stat(nc);
-  for (int c = 0; c < nc; ++c) stat[c] = (R)(1.5 * hS[ev.cls[c].el] - 0.5 * hC[ev.cls[c].el]);
-  std::vector<int> elt(ns), tb(1, 0);
-  std::vector<EvenTerm> terms;
-  for (int e = 0; e < ns; ++e) {
-    const int el = ev.sym_el[e];
-    elt[e] = el / No + No * (el % No);
-    for (const Term& t : p.sigma[el]) {
-      const int x = t.m + Nchi * t.l;
-      terms.push_back(EvenTerm{ev.cls_of[x], ev.sym_of[t.ef], ev.cj_of[x]});
-    }
-    tb.push_back((int)terms.size());
-  }
-  DBuf<int> sel(ns), delt(ns), dtb(tb.size());
-  DBuf<EvenTerm> dt(terms.size());
-  sel.upload(ev.sym_el.data(), ns);
-  delt.upload(elt.data(), ns);
-  dtb.upload(tb.data(), tb.size());
-  dt.upload(terms.data(), terms.size());
+  PGB_CHECK(ev.sig_tb.n == (size_t)ns + 1, "the even form's pair list has no Sigma terms");
   DBuf<cx<R>> F(ns * P), W((size_t)nc * P), T(ns * P), T2;
   if (ev.three_d) T2.alloc(ns * P);
   SpaceArgs<R> a{};
   a.Nk = g.Nk;
   a.src = G;
-  a.el = sel.p;
+  a.el = ev.d_sym_el.p;
   fermi_transform<R>(ev, a, F.p, ns, false, st);
-  vertex_transforms<R>(g, V, stat, W.p, st);
+  vertex_transforms<R>(g, V, S, C, 1.5, -0.5, W.p, st);
   const FFT4D& ft = fft_plan_t(H, Nw, (int)sizeof(cx<R>));
   const unsigned tiles = (unsigned)(((H + 255) / 256) * Nw);
-  k_even_contract<R><<<tiles * ns, 256, 0, st>>>(T.p, W.p, F.p, dt.p, dtb.p, fft_roots<R>(2 * Nw), H, Nw, ft.d_pos(3),
+  k_even_contract<R><<<tiles * ns, 256, 0, st>>>(T.p, W.p, F.p, ev.sig_terms.p, ev.sig_tb.p, fft_roots<R>(2 * Nw), H, Nw, ft.d_pos(3),
                                                 ft.d_logical(3), ns);
   count_launch("even_contract");
   SpaceArgs<R> o{};
   o.Nk = g.Nk;
   o.dst = sig;
-  o.el = sel.p;
-  o.elt = delt.p;
+  o.el = ev.d_sym_el.p;
+  o.elt = ev.d_sym_elt.p;
   o.scale = temp / (double)g.Nkall / (double)g.P;
   o.thresh = 1;
   even_backward<R, kInPostFermi, kOutSigma>(ev, o, T.p, T2.p, ns, st);
-  sync();
 }
 
 template <typename R>
@@ -1088,14 +1062,8 @@ void mkdelta_even(const Geom& g, const Pairs& p, const double2* F64, const cx<R>
   const size_t P = (size_t)H * Nw;
   if (!cache.built) {
     cache.built = true;
-    std::vector<double> hS(Nchi * Nchi), hC(Nchi * Nchi);
-    PGB_CUDA(cudaMemcpyAsync(hS.data(), S, sizeof(double) * hS.size(), cudaMemcpyDeviceToHost, st));
-    PGB_CUDA(cudaMemcpyAsync(hC.data(), C, sizeof(double) * hC.size(), cudaMemcpyDeviceToHost, st));
-    sync();
-    std::vector<R> stat(nc);
-    for (int c = 0; c < nc; ++c) stat[c] = (R)(0.5 * (hS[ev.cls[c].el] + hC[ev.cls[c].el]));
     cache.W.alloc((size_t)nc * P);
-    vertex_transforms<R>(g, Vd, stat, cache.W.p, st);
+    vertex_transforms<R>(g, Vd, S, C, 0.5, 0.5, cache.W.p, st);
     std::vector<EvenTerm> terms;
     std::vector<int> tb(1, 0), el;
     for (int e = 0; e < No * No; ++e) {
@@ -1192,8 +1160,8 @@ bool stoner_even(const Geom& g, const cx<R>* chi, std::vector<double>& out) {
 }
 
 #define PGB_EVEN_INST(R)                                                                                              \
-  template void chi0_even<R>(const Geom&, const Pairs&, const double2*, double, const TailRef*, cx<R>*, bool);         \
-  template void sigma_even<R>(const Geom&, const Pairs&, const double2*, const cx<R>*, const double*, const double*,   \
+  template void chi0_even<R>(const Geom&, const double2*, double, const TailRef*, cx<R>*, bool);         \
+  template void sigma_even<R>(const Geom&, const double2*, const cx<R>*, const double*, const double*,   \
                               double, double2*);                                                                      \
   template void mkdelta_even<R>(const Geom&, const Pairs&, const double2*, const cx<R>*, const cx<R>*, const double*,  \
                                 const double*, double, double2*, DeltaKernelCache<R>&);                               \

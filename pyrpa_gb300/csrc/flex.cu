@@ -665,7 +665,10 @@ __global__ void k_chi0_scatter(cx<R>* chi, const cx<R>* tmp, const ChiDev* pairs
 
 // tau kernels of the analytic reference bubble (fchi.f90:703-729), laid out
 // [(s*Norb + n)*Nk + k]
-template <typename T>
+//
+// BOTH false leaves gm out, half of the exponentials: at one orbital, 1024 points
+// and M = 2048 in FP64 (bound by the FP64 pipe) 300 -> 181 us.
+template <typename T, bool BOTH>
 __global__ void k_gpm(T* gp, T* gm, double* ff, const double* eig, double mu, double temp,
                       int Nk, int No, int M) {
   const double beta = 1.0 / temp, dtau = beta / M;
@@ -684,27 +687,27 @@ __global__ void k_gpm(T* gp, T* gm, double* ff, const double* eig, double mu, do
       const float rd = 1.0f / (1.0f + e);
       const float lo = expf((float)(-fabs(xi) * tau)), hi = expf((float)(-fabs(xi) * (beta - tau)));
       gp[idx] = xi >= 0 ? -lo * rd : -hi * rd;
-      gm[idx] = xi >= 0 ? hi * rd : lo * rd;
+      if (BOTH) gm[idx] = xi >= 0 ? hi * rd : lo * rd;
       if (s == 0) {
         const double d = 1.0 + exp(-beta * fabs(xi));
         ff[n + (long long)No * k] = xi >= 0 ? exp(-beta * xi) / d : 1.0 / d;
       }
       continue;
     }
-    double p, q;
+    double p, q = 0.0;
     if (xi >= 0) {
       const double d = 1.0 + exp(-beta * xi);
       p = -exp(-xi * tau) / d;
-      q = exp(-xi * (beta - tau)) / d;
+      if (BOTH) q = exp(-xi * (beta - tau)) / d;
       if (s == 0) ff[n + (long long)No * k] = exp(-beta * xi) / d;
     } else {
       const double d = 1.0 + exp(beta * xi);
       p = -exp(xi * (beta - tau)) / d;
-      q = exp(xi * tau) / d;
+      if (BOTH) q = exp(xi * tau) / d;
       if (s == 0) ff[n + (long long)No * k] = 1.0 / d;
     }
     gp[idx] = (T)p;
-    gm[idx] = (T)q;
+    if (BOTH) gm[idx] = (T)q;
   }
 }
 
@@ -763,30 +766,46 @@ __global__ void k_rhobar(double2* rhobar, const double2* uni, const double* ff, 
 }
 
 // sawtooth correction: exact -1/(i nu) minus its rectangle-rule DFT (fchi.f90:757-772)
-__global__ void k_sawc(double2* sawc, int Nw, int M, double temp) {
+// the roots and weights it needs, once per s instead of once per (j, s)
+__global__ void k_sawc_table(double2* root, double* wt, int M, double temp) {
+  const int s = blockIdx.x * blockDim.x + threadIdx.x;
+  if (s >= M) return;
+  double sn, cs;
+  sincospi(2.0 * (double)s / (double)M, &sn, &cs);
+  root[s] = mkc(cs, sn);
+  const double dtau = 1.0 / temp / M;
+  wt[s] = dtau * (0.5 - (double)s / (double)M);
+}
+// A chain of M sums per j, so one warp per block, with the loads of eight steps in
+// flight; with a sine and cosine of its own in every step and 128 threads per
+// block it took 4.8 ms at Nw = 1024, now 0.22 ms.
+__global__ void k_sawc(double2* sawc, const double2* root, const double* wt, int Nw, int M, double temp) {
   const int j = blockIdx.x * blockDim.x + threadIdx.x;
   if (j >= Nw) return;
-  const double dtau = 1.0 / temp / M;
   double2 v = mkc(0.0, 0.0);
   if (j > 0) v = mkc(0.0, 1.0 / (2.0 * kPi * j * temp));
+  int r = 0;
+#pragma unroll 8
   for (int s = 0; s < M; ++s) {
-    double sn, cs;
-    sincospi(2.0 * (double)(((long long)j * s) % M) / (double)M, &sn, &cs);
-    const double w = dtau * (0.5 - (double)s / (double)M);
-    v.x -= w * cs;
-    v.y -= w * sn;
+    const double w = wt[s];
+    const double2 c = root[r];
+    v.x -= w * c.x;
+    v.y -= w * c.y;
+    r += j;
+    if (r >= M) r -= M;
   }
   sawc[j] = v;
 }
 
 // ---- parts of the analytic reference bubble shared with the even-model form
-template <typename T> void tail_tables(const Geom& g, const TailRef& tail, double temp, TailTables<T>& tt) {
+template <typename T> void tail_tables(const Geom& g, const TailRef& tail, double temp, TailTables<T>& tt, bool both) {
   const int No2 = g.Norb * g.Norb;
   const size_t nt = (size_t)g.Nk * g.Norb * g.M, ncf = (size_t)g.Nk * g.Norb * No2;
   tt.gp.alloc(nt);
-  tt.gm.alloc(nt);
+  if (both) tt.gm.alloc(nt);
   tt.ff.alloc((size_t)g.Nk * g.Norb);
-  k_gpm<T><<<mesh_tau_grid((long long)g.Nk * g.Norb, g.M, 1), 256, 0, ctx().stream>>>(
+  const auto gpm = both ? &k_gpm<T, true> : &k_gpm<T, false>;
+  gpm<<<mesh_tau_grid((long long)g.Nk * g.Norb, g.M, 1), 256, 0, ctx().stream>>>(
       tt.gp.p, tt.gm.p, tt.ff.p, tail.eig, tail.mu, temp, g.Nk, g.Norb, (int)g.M);
   count_launch("gpm");
   tt.cf64.alloc(ncf);
@@ -796,18 +815,12 @@ template <typename T> void tail_tables(const Geom& g, const TailRef& tail, doubl
     convert<float, double>(tt.cf32.p, tt.cf64.p, (long long)ncf);
   }
 }
-template void tail_tables<float>(const Geom&, const TailRef&, double, TailTables<float>&);
-template void tail_tables<double>(const Geom&, const TailRef&, double, TailTables<double>&);
+template void tail_tables<float>(const Geom&, const TailRef&, double, TailTables<float>&, bool);
+template void tail_tables<double>(const Geom&, const TailRef&, double, TailTables<double>&, bool);
 
-std::vector<double2> tail_rhobar(const Geom& g, const TailRef& tail, const double* ff) {
-  const int No2 = g.Norb * g.Norb;
-  DBuf<double2> rb(No2);
-  k_rhobar<<<No2, 256, 0, ctx().stream>>>(rb.p, tail.uni, ff, g.grid_irr.p, g.grid_flag.p, g.Nkall, g.Norb);
+void tail_rhobar(const Geom& g, const TailRef& tail, const double* ff, double2* rb) {
+  k_rhobar<<<g.Norb * g.Norb, 256, 0, ctx().stream>>>(rb, tail.uni, ff, g.grid_irr.p, g.grid_flag.p, g.Nkall, g.Norb);
   count_launch("rhobar");
-  std::vector<double2> h(No2);
-  rb.download(h.data(), No2);
-  sync();
-  return h;
 }
 
 // tau = 0 jump coefficient of pair (l,m) (fchi.f90:836-844)
@@ -828,7 +841,11 @@ const double2* tail_sawtooth(const Geom& g, double temp) {
   DBuf<double2>*& e = cache[std::make_pair(g.Nw, temp)];
   if (!e) {
     e = new DBuf<double2>(g.Nw);
-    k_sawc<<<grid_1d(g.Nw, 128), 128, 0, st>>>(e->p, g.Nw, (int)g.M, temp);
+    DBuf<double2> root(g.M);
+    DBuf<double> wt(g.M);
+    k_sawc_table<<<grid_1d(g.M, 64), 64, 0, st>>>(root.p, wt.p, (int)g.M, temp);
+    count_launch("sawc_table");
+    k_sawc<<<grid_1d(g.Nw, 32), 32, 0, st>>>(e->p, root.p, wt.p, g.Nw, (int)g.M, temp);
     count_launch("sawc");
     // complete before another thread's stream reads the cached entry
     PGB_CUDA(cudaStreamSynchronize(st));
@@ -842,10 +859,14 @@ bool chi0_swap_enabled() {
   return !(s && std::string(s) == "0");
 }
 
+// scratch below this is taken without a look at the free memory: with the look a
+// 16x16x256 chi0 of one orbital takes 0.267 ms, without 0.239
+constexpr long long kSmallScratch = 16LL << 20;
+
 template <typename R>
 void chi0(const Geom& g, const Pairs& p, const double2* G, double temp, const TailRef* tail, cx<R>* chi, bool full) {
   if (g.even) {
-    chi0_even<R>(g, p, G, temp, tail, chi, full);
+    chi0_even<R>(g, G, temp, tail, chi, full);
     return;
   }
   cudaStream_t st = ctx().stream;
@@ -900,7 +921,7 @@ void chi0(const Geom& g, const Pairs& p, const double2* G, double temp, const Ta
     // FP32 transforms'), in FP64 for the wider types
     using T = typename std::conditional<std::is_same<R, float>::value, float, double>::type;
     TailTables<T> tt;
-    tail_tables<T>(g, *tail, temp, tt);
+    tail_tables<T>(g, *tail, temp, tt, true);
     A.alloc((size_t)No2 * g.P);
     B.alloc((size_t)No2 * g.P);
     k_ref_tau<R, T><<<mesh_tau_grid(g.Nkall, g.M, No2), 256, 0, st>>>(A.p, B.p, tt.gp.p, tt.gm.p, tt.projectors(), g.grid_irr.p, g.grid_flag.p, g.Nkall,
@@ -908,7 +929,11 @@ void chi0(const Geom& g, const Pairs& p, const double2* G, double temp, const Ta
     count_launch("ref_tau");
     fft.forward_space<R>(A.p, No2, st);
     fft.forward_space<R>(B.p, No2, st);
-    const std::vector<double2> hrb = tail_rhobar(g, *tail, tt.ff.p);
+    DBuf<double2> rb(No2);
+    tail_rhobar(g, *tail, tt.ff.p, rb.p);
+    std::vector<double2> hrb(No2);
+    rb.download(hrb.data(), No2);
+    sync();
     auto Jof = [&](int l, int m) { return tail_jump(p, hrb, g.Norb, l, m); };
     for (auto& c : hp) {
       c.J = Jof(c.l, c.m);
@@ -926,12 +951,14 @@ void chi0(const Geom& g, const Pairs& p, const double2* G, double temp, const Ta
   DBuf<ChiDev> dp(hp.size());
   dp.upload(hp.data(), hp.size());
   PGB_CUDA(cudaMemsetAsync(chi, 0, sizeof(cx<R>) * (size_t)g.K * g.Nchi * g.Nchi, st));
-  // chunk of pairs per backward batch: bounded by free memory
+  // chunk of pairs per backward batch: bounded by free memory, which is asked for
+  // only where the chunk is not small (the question waits for the device)
   sync();
-  const size_t freeb = device_bytes_available();
-  long long ch = (long long)((freeb / 3) / (sizeof(cx<R>) * (size_t)g.P));
-  ch = std::max(1LL, std::min<long long>(ch, (long long)hp.size()));
-  ch = std::min(ch, 64LL);
+  long long ch = std::max(1LL, std::min(64LL, (long long)hp.size()));
+  if (ch * g.P * (long long)sizeof(cx<R>) > kSmallScratch) {
+    const long long fit = (long long)((device_bytes_available() / 3) / (sizeof(cx<R>) * (size_t)g.P));
+    ch = std::max(1LL, std::min(ch, fit));
+  }
   DBuf<cx<R>> T((size_t)ch * g.P);
   const double sc = temp / (double)g.Nkall / (double)g.P;
   const double sr = 1.0 / (temp * (double)g.Nkall) / (double)g.P;
@@ -2518,7 +2545,7 @@ template <typename R>
 void sigma(const Geom& g, const Pairs& p, const double2* G, const cx<R>* V, const double* S, const double* C,
            double temp, double2* sig) {
   if (g.even) {
-    sigma_even<R>(g, p, G, V, S, C, temp, sig);
+    sigma_even<R>(g, G, V, S, C, temp, sig);
     return;
   }
   cudaStream_t st = ctx().stream;
@@ -2984,32 +3011,50 @@ __global__ void k_scal(double2* y, double a, long long n) {
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
     y[i] = a * y[i];
 }
+// Sum of v over the block's kRedThreads threads in the order of the tree
+// red[t] += red[t + s], s = 128 ... 1; in thread 0
+__device__ __forceinline__ double2 tree_sum(double2 v, double2* red) {
+  red[threadIdx.x] = v;
+  __syncthreads();
+  for (int s = kRedThreads / 2; s >= 32; s >>= 1) {
+    if ((int)threadIdx.x < s) red[threadIdx.x] = v = v + red[threadIdx.x + s];
+    __syncthreads();
+  }
+  if (threadIdx.x < 32) {
+#pragma unroll
+    for (int s = 16; s > 0; s >>= 1)
+      v = v + mkc(__shfl_down_sync(0xffffffffu, v.x, s), __shfl_down_sync(0xffffffffu, v.y, s));
+  }
+  return v;
+}
+// true in every thread of the block that arrives last of the grid, whose
+// predecessors' partial sums are then visible
+__device__ __forceinline__ bool last_block(unsigned* ticket) {
+  __shared__ bool last;
+  if (threadIdx.x == 0) {
+    __threadfence();
+    last = atomicAdd(ticket, 1u) == gridDim.x - 1;
+    if (last) *ticket = 0;
+    __threadfence();
+  }
+  __syncthreads();
+  return last;
+}
+
 // One step of the modified Gram-Schmidt orthogonalization of y against a Krylov
-// basis, device resident: h = 2 sum_i of the previous step's partial sums (every
-// block adds them up itself, in k_sum_parts' order), y -= h xp, and the partial
-// sums of the next inner product sum kw conj(xn) y (xn null: of y with itself).
+// basis, device resident: y -= h xp with the previous step's coefficient, and the
+// next one, twice the sum of kw conj(xn) y (xn null: of y with itself).
 // The element order and arithmetic are those of inner_w, axpy and inner_w called
-// one after the other, which waited for the host at every coefficient.
-__global__ void __launch_bounds__(kRedThreads) k_gs_step(double2* y, const double2* xp, const double2* part_in,
-                                                         double2* h_out, const double2* xn, double2* part_out,
-                                                         const double* kw, unsigned Nk, unsigned n) {
+// one after the other, which waited for the host at every coefficient.  The last
+// block adds up the partial sums, in k_sum_parts' order (every block of the next
+// step doing it for itself cost 1024 times the FP64 adds: 36 us a step at
+// two orbitals, 32x32x256, 24 now).
+__global__ void __launch_bounds__(kRedThreads) k_gs_step(double2* y, const double2* xp, const double2* h_in,
+                                                         const double2* xn, double2* part, unsigned* ticket,
+                                                         double2* h_out, const double* kw, unsigned Nk, unsigned n) {
   __shared__ double2 red[kRedThreads];
   double2 a = mkc(0.0, 0.0);
-  if (xp) {
-    double2 acc = mkc(0.0, 0.0);
-    for (int i = threadIdx.x; i < kRedBlocks; i += blockDim.x) acc += part_in[i];
-    red[threadIdx.x] = acc;
-    __syncthreads();
-    for (int s = blockDim.x / 2; s > 0; s >>= 1) {
-      if ((int)threadIdx.x < s) red[threadIdx.x] += red[threadIdx.x + s];
-      __syncthreads();
-    }
-    const double2 s = red[0];
-    __syncthreads();
-    const double2 h = mkc(2.0 * s.x, 2.0 * s.y);
-    if (blockIdx.x == 0 && threadIdx.x == 0) *h_out = h;
-    a = mkc(-h.x, -h.y);
-  }
+  if (xp) a = mkc(-h_in->x, -h_in->y);
   double2 acc = mkc(0.0, 0.0);
   for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
     // the roundings of k_axpy and k_inner_w (which product of each pair is fused
@@ -3027,13 +3072,81 @@ __global__ void __launch_bounds__(kRedThreads) k_gs_step(double2* y, const doubl
     acc.x = fma(k, fma(u.x, v.x, __dmul_rn(u.y, v.y)), acc.x);
     acc.y = fma(k, fma(u.x, v.y, -__dmul_rn(u.y, v.x)), acc.y);
   }
-  red[threadIdx.x] = acc;
-  __syncthreads();
-  for (int s = blockDim.x / 2; s > 0; s >>= 1) {
-    if ((int)threadIdx.x < s) red[threadIdx.x] += red[threadIdx.x + s];
-    __syncthreads();
+  acc = tree_sum(acc, red);
+  if (threadIdx.x == 0) part[blockIdx.x] = acc;
+  if (!last_block(ticket)) return;
+  acc = mkc(0.0, 0.0);
+  for (int i = threadIdx.x; i < kRedBlocks; i += kRedThreads) acc += __ldcg(part + i);
+  acc = tree_sum(acc, red);
+  if (threadIdx.x == 0) *h_out = mkc(2.0 * acc.x, 2.0 * acc.y);
+}
+
+// The same step for vectors whose (a, b) matrices are Hermitian at every point:
+// real coefficients, and only the elements a >= b of y are kept.  A thread takes a
+// point, so that the weights cost one product per point: 4 FP64 instructions for
+// each of N (N + 1) / 2 elements instead of 12 for each of N^2.  At five orbitals,
+// 32x32x256, k_gs_step takes 98 us a step (FP64 pipe), this 32 us.
+template <int N>
+__global__ void __launch_bounds__(128) k_gs_herm(double2* y, const double2* __restrict__ xp, const double* h_in,
+                                                 const double2* __restrict__ xn, double* part, unsigned* ticket,
+                                                 double* h_out, const double* __restrict__ kw, int Nk, long long K) {
+  __shared__ double red[4];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const double a = xp ? -*h_in : 0.0;
+  double acc = 0.0;
+  for (long long i = blockIdx.x * 128LL + threadIdx.x; i < K; i += gridDim.x * 128LL) {
+    double dg = 0.0, od = 0.0;
+#pragma unroll
+    for (int c = 0; c < N; ++c) {
+      double2 v[N], x[N], u[N];
+#pragma unroll
+      for (int r = c; r < N; ++r) {
+        const long long e = i + K * (r + N * c);
+        v[r] = y[e];
+        if (xp) x[r] = xp[e];
+        if (xn) u[r] = xn[e];
+      }
+#pragma unroll
+      for (int r = c; r < N; ++r) {
+        if (xp) {
+          v[r].x = fma(a, x[r].x, v[r].x);
+          if (r > c) v[r].y = fma(a, x[r].y, v[r].y);
+          y[i + K * (r + N * c)] = v[r];
+        }
+        const double2 z = xn ? u[r] : v[r];
+        if (r == c) dg = fma(z.x, v[r].x, dg);
+        else od = fma(z.y, v[r].y, fma(z.x, v[r].x, od));
+      }
+    }
+    acc = fma(kw[i % Nk], fma(2.0, od, dg), acc);
   }
-  if (threadIdx.x == 0) part_out[blockIdx.x] = red[0];
+  auto block_sum = [&](double v) {
+    v = warp_sum(v);
+    if (lane == 0) red[w] = v;
+    __syncthreads();
+    return (red[0] + red[1]) + (red[2] + red[3]);
+  };
+  acc = block_sum(acc);
+  if (threadIdx.x == 0) part[blockIdx.x] = acc;
+  if (!last_block(ticket)) return;
+  acc = 0.0;
+  for (int i = threadIdx.x; i < (int)gridDim.x; i += 128) acc += __ldcg(part + i);
+  acc = block_sum(acc);
+  if (threadIdx.x == 0) *h_out = 2.0 * acc;
+}
+// y = a x from the elements a >= b of x, the others conjugate
+template <int N>
+__global__ void k_scal_herm(double2* y, double a, const double2* __restrict__ x, long long K) {
+  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < K; i += (long long)gridDim.x * blockDim.x)
+#pragma unroll
+    for (int c = 0; c < N; ++c)
+#pragma unroll
+      for (int r = c; r < N; ++r) {
+        double2 v = x[i + K * (r + N * c)];
+        v = mkc(a * v.x, r == c ? 0.0 : a * v.y);
+        y[i + K * (r + N * c)] = v;
+        if (r > c) y[i + K * (c + N * r)] = conj(v);
+      }
 }
 __global__ void k_scal_to(double2* y, double a, const double2* x, long long n) {
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
@@ -3055,20 +3168,54 @@ void gram_schmidt(double2* y, const double2* const* xs, int m, const double* kw,
                   double* norm2) {
   PGB_CHECK(n < (1LL << 32) - (long long)kRedBlocks * kRedThreads, "vector too long for the orthogonalization");
   cudaStream_t st = ctx().stream;
-  DBuf<double2> part(2 * kRedBlocks), out(m + 1);
+  DBuf<double2> part(kRedBlocks), out(m + 1);
+  DBuf<unsigned> ticket(1);
+  ticket.zero();
   for (int i = 0; i <= m; ++i) {
-    k_gs_step<<<kRedBlocks, kRedThreads, 0, st>>>(y, i ? xs[i - 1] : nullptr, part.p + (i & 1) * kRedBlocks,
-                                                  i ? out.p + i - 1 : nullptr, i < m ? xs[i] : nullptr,
-                                                  part.p + ((i + 1) & 1) * kRedBlocks, kw, (unsigned)Nk, (unsigned)n);
+    k_gs_step<<<kRedBlocks, kRedThreads, 0, st>>>(y, i ? xs[i - 1] : nullptr, i ? out.p + i - 1 : nullptr,
+                                                  i < m ? xs[i] : nullptr, part.p, ticket.p, out.p + i, kw,
+                                                  (unsigned)Nk, (unsigned)n);
     count_launch("gs_step");
   }
-  k_sum_parts<<<1, kRedThreads, 0, st>>>(out.p + m, part.p + ((m + 1) & 1) * kRedBlocks, kRedBlocks);
-  count_launch("sum_parts");
   std::vector<double2> hh(m + 1);
   out.download(hh.data(), m + 1);
   sync();
   for (int i = 0; i < m; ++i) h[i] = hh[i];
-  *norm2 = 2.0 * hh[m].x;
+  *norm2 = hh[m].x;
+}
+void gram_schmidt_herm(double2* y, const double2* const* xs, int m, const double* kw, int Nk, long long K, int Norb,
+                       double* h, double* norm2) {
+  cudaStream_t st = ctx().stream;
+  const unsigned nb = (unsigned)std::min<long long>((K + 127) / 128, 8LL * ctx().num_sms);
+  DBuf<double> part(nb), out(m + 1);
+  DBuf<unsigned> ticket(1);
+  ticket.zero();
+  for (int i = 0; i <= m; ++i) {
+    const double2 *xp = i ? xs[i - 1] : nullptr, *xn = i < m ? xs[i] : nullptr;
+    const double* hi = i ? out.p + i - 1 : nullptr;
+    switch (Norb) {
+#define PGB_GH(n_) case n_: k_gs_herm<n_><<<nb, 128, 0, st>>>(y, xp, hi, xn, part.p, ticket.p, out.p + i, kw, Nk, K); break;
+      PGB_GH(1) PGB_GH(2) PGB_GH(3) PGB_GH(4) PGB_GH(5) PGB_GH(6) PGB_GH(7) PGB_GH(8)
+#undef PGB_GH
+      default: throw Error("Norb above the engine limit of 8 orbitals");
+    }
+    count_launch("gs_herm");
+  }
+  std::vector<double> hh(m + 1);
+  out.download(hh.data(), m + 1);
+  sync();
+  for (int i = 0; i < m; ++i) h[i] = hh[i];
+  *norm2 = hh[m];
+}
+void scal_herm(double2* y, double a, const double2* x, long long K, int Norb) {
+  const unsigned grid = grid_1d(K, 256, 65536);
+  switch (Norb) {
+#define PGB_SH(n_) case n_: k_scal_herm<n_><<<grid, 256, 0, ctx().stream>>>(y, a, x, K); break;
+    PGB_SH(1) PGB_SH(2) PGB_SH(3) PGB_SH(4) PGB_SH(5) PGB_SH(6) PGB_SH(7) PGB_SH(8)
+#undef PGB_SH
+    default: throw Error("Norb above the engine limit of 8 orbitals");
+  }
+  count_launch("scal_herm");
 }
 void scal_to(double2* y, double a, const double2* x, long long n) {
   k_scal_to<<<grid_1d(n, 256, 65536), 256, 0, ctx().stream>>>(y, a, x, n);

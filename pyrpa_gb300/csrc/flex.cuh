@@ -119,8 +119,9 @@ template <typename T> struct TailTables {
     else return cf64.p;
   }
 };
-template <typename T> void tail_tables(const Geom& g, const TailRef& tail, double temp, TailTables<T>& tt);
-std::vector<double2> tail_rhobar(const Geom& g, const TailRef& tail, const double* ff);
+// both: gm as well as gp (gm(tau) = -gp(beta - tau))
+template <typename T> void tail_tables(const Geom& g, const TailRef& tail, double temp, TailTables<T>& tt, bool both);
+void tail_rhobar(const Geom& g, const TailRef& tail, const double* ff, double2* rb);
 double2 tail_jump(const Pairs& p, const std::vector<double2>& rb, int Norb, int l, int m);
 const double2* tail_sawtooth(const Geom& g, double temp);
 // Stoner factors: max Re eig(chi0(q,0) S) and of -chi0(q,0) C (fchi.f90:352-399)
@@ -189,6 +190,11 @@ void initial_delta(double2* D, const double* init, const double2* uni, int Nk, i
 // norm of what is left into norm2; one wait for all of them
 void gram_schmidt(double2* y, const double2* const* xs, int m, const double* kw, int Nk, long long n, double2* h,
                   double* norm2);
+// the same with real coefficients for vectors of Hermitian matrices (K points of
+// Norb x Norb); the elements a < b of y are left as they are
+void gram_schmidt_herm(double2* y, const double2* const* xs, int m, const double* kw, int Nk, long long K, int Norb,
+                       double* h, double* norm2);
+void scal_herm(double2* y, double a, const double2* x, long long K, int Norb);
 void scal_to(double2* y, double a, const double2* x, long long n);       // y = a x
 void axpy(double2* y, double2 a, const double2* x, long long n);         // y += a x
 void scal(double2* y, double a, long long n);
