@@ -167,7 +167,7 @@ __global__ void k_diis_mix(double2* sig, const double2* sig0, DiisTerms t, int n
     if (den > 1.0e-20) {
       if (!(num < 1.0e70 && den < 1.0e70)) {
         const double q = hypot(d.x, d.y) / hypot(sd.x, sd.y);
-        num = q < 1.0e70 ? q * q : 1.0e140;
+        num = q < 1.0e70 ? q * q : (q >= 1.0e70 ? 1.0e140 : 0.0);  // a NaN counts as nothing
         den = 1.0;
       }
       if (num * bd > bn * den) {
