@@ -335,6 +335,8 @@ class HostPrefault {
   HostPrefault(const HostPrefault&) = delete;
   HostPrefault& operator=(const HostPrefault&) = delete;
   void join();
+  // whether a result of this size may be started on before its last stage
+  static bool early(size_t bytes) { return bytes <= (1u << 30); }
 
  private:
   std::vector<std::thread> threads_;

@@ -860,10 +860,13 @@ void run_mkself(const MkselfArgs& a, int prec) {
                  a.sw_rescale, a.sw_tail, a.sigma_scale};
   detect_even(in, a.Smat, a.Cmat, a.hamk, a.eig, a.uni, prec == 32 ? 8 : 16);
   const long long KE = in.g.K * a.Norb * a.Norb;
-  HostPrefault pages(a.sigmak, sizeof(double2) * KE);
   DBuf<double2> sig(KE);
+  const size_t bytes = sizeof(double2) * KE;
+  std::unique_ptr<HostPrefault> pages;
+  if (a.scf_loop <= 4 && HostPrefault::early(bytes)) pages.reset(new HostPrefault(a.sigmak, bytes));
   mkself_core(in, prm, sig.p, a.mu_out, nullptr, 0.0, 0.0, prec);
-  pages.join();
+  if (!pages) pages.reset(new HostPrefault(a.sigmak, bytes));
+  pages->join();
   sig.download(a.sigmak, KE);
   sync();
 }
@@ -1268,7 +1271,6 @@ void run_lin_eliash(const LinEliashArgs& a) {
   upload_inputs(in, a.kmap, a.invk, a.olist, a.Nx, a.Ny, a.Nz, a.Nkall, a.Nk, a.Nw, a.Norb, a.Nchi, a.Smat, a.Cmat,
                 nullptr, nullptr, a.uni);
   const long long KE = in.g.K * a.Norb * a.Norb, KC = in.g.K * a.Nchi * a.Nchi;
-  HostPrefault pages(a.delta, sizeof(double2) * KE);
   DBuf<double> prt(a.Norb), init(a.Nk * a.Norb);
   prt.upload(a.prt, a.Norb);
   init.upload(a.init_delta, a.Nk * a.Norb);
@@ -1291,7 +1293,7 @@ void run_lin_eliash(const LinEliashArgs& a) {
   }
   EliashParams prm{a.temp, a.eps, a.itemax, a.gap_sym, a.arnoldi_m};
   *a.lambda_out = eliash_core<R>(in, chi.p, G.p, init.p, prt.p, prm, D.p, a.clobber_chi ? a.chi : nullptr);
-  pages.join();
+  HostPrefault(a.delta, sizeof(double2) * KE).join();
   D.download(a.delta, KE);
   sync();
 }
@@ -1410,7 +1412,6 @@ void run_pipeline_impl(const PipelineArgs& a, int prec) {
   upload_inputs(in, a.kmap, a.invk, a.olist, a.Nx, a.Ny, a.Nz, a.Nkall, a.Nk, a.Nw, a.Norb, a.Nchi, a.Smat, a.Cmat,
                 a.hamk, a.eig, a.uni);
   const long long K = in.g.K, KE = K * a.Norb * a.Norb, KC = K * a.Nchi * a.Nchi;
-  HostPrefault pages_s(a.sigmak, sizeof(double2) * KE), pages_d(a.delta, sizeof(double2) * KE);
   detect_even(in, a.Smat, a.Cmat, a.hamk, a.eig, a.uni, 16);
   DBuf<double> prt(a.Norb), init(a.Nk * a.Norb);
   prt.upload(a.prt, a.Norb);
@@ -1441,6 +1442,13 @@ void run_pipeline_impl(const PipelineArgs& a, int prec) {
   seed.release();
   PGB_CHECK(dyson(G.p, sig.p, in.H.p, mu, a.temp, in.Nk, in.Nw, in.Norb), "singular G^-1 in the Dyson step");
   double stoner_v = 0;
+  const size_t bytes = sizeof(double2) * KE;
+  std::unique_ptr<HostPrefault> pages_s, pages_d;
+  auto prefault = [&]() {
+    pages_s.reset(new HostPrefault(a.sigmak, bytes));
+    pages_d.reset(new HostPrefault(a.delta, bytes));
+  };
+  if (HostPrefault::early(bytes)) prefault();
   {
     DBuf<cx<R>> chi(KC);
     TailRef tr{in.eig.p, in.uni.p, mu};
@@ -1454,8 +1462,9 @@ void run_pipeline_impl(const PipelineArgs& a, int prec) {
   }
   g_stats.iterations = iters;
   const double t_compute = t.stop();
-  pages_s.join();
-  pages_d.join();
+  if (!pages_s) prefault();
+  pages_s->join();
+  pages_d->join();
   t.start();
   sig.download(a.sigmak, KE);
   D.download(a.delta, KE);

@@ -6,7 +6,10 @@
 // with large results start a few threads here that make the pages
 // (MADV_POPULATE_WRITE, which leaves the contents as they are) while the solve
 // runs, and join them before the copy: one FLEX iteration of five orbitals,
-// 64x64x1024 (840 MB of Sigma) 86 -> 76 ms.
+// 64x64x1024 (840 MB of Sigma) 83 -> 58 ms.  Large sets of pages that wait for their copy
+// take longer to copy into than none, the longer they wait (2 x 1.7 GB made a second
+// before the copy 200 to 660 ms, without 122): results above 1 GB, and those of a loop
+// of many iterations, are started at the solve's end.
 #include <sys/mman.h>
 #include <unistd.h>
 
@@ -23,7 +26,7 @@
 namespace pgb {
 
 namespace {
-constexpr size_t kPrefaultMin = 4u << 20;       // below this the faults cost less than a thread
+constexpr size_t kPrefaultMin = 32u << 20;  // 36 MB 8.9 -> 8.4 ms a call, 28 MB 2.00 -> 2.05
 constexpr size_t kPerThread = 64u << 20;
 constexpr size_t kMaxThreads = 4;
 constexpr size_t kPiece = 1u << 20;
