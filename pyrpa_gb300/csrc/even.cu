@@ -123,6 +123,39 @@ void build_index(Even& ev, int n, const std::vector<RealBasis>& basis, const std
   }
 }
 
+// The symmetric form of the real basis.  An element (l,m) and (m,l) are the same
+// function, so with h = 1 (same orbital), 2 (sums), -2 (differences) the matrix
+// M_pq = A_pq h_q is symmetric and A^-1 = diag(h) M^-1.  A symmetric matrix is kept
+// as its cyclic diagonals: entry (p, (p + d) mod n), d <= n/2, at d n + p.
+// sin: entry of M from the class representatives; sout: part of a class's result
+// A = diag(h) W from W, every coefficient +-1.
+int sym_at(int n, int p, int q) {
+  const int d = (q - p + n) % n;
+  return 2 * d < n || (2 * d == n && p < q) ? d * n + p : (n - d) * n + q;
+}
+void build_sym(Even& ev, int n, const std::vector<RealBasis>& basis) {
+  ev.hsc.clear();
+  for (const RealBasis& b : basis) ev.hsc.push_back(b.kind == 0 ? 1.0 : (b.kind == 1 ? 2.0 : -2.0));
+  ev.sin.clear();
+  for (int d = 0; d <= n / 2; ++d)
+    for (int p = 0; p < n; ++p) {
+      const int q = (p + d) % n, w = ev.vin[(size_t)q * n + p];
+      const int ca = (((w >> 18) & 7) - 2) * (int)ev.hsc[q], cb = (((w >> 21) & 7) - 2) * (int)ev.hsc[q];
+      ev.sin.push_back((w & 511) | ((w >> 9) & 511) << 9 | (ca < 0) << 18 | (cb < 0) << 19 | (cb != 0) << 20 |
+                       (std::abs(ca) == 2) << 21);
+    }
+  ev.sout.clear();
+  for (int w : ev.vout) {
+    const int at[2] = {w & 1023, (w >> 10) & 1023}, sg[2] = {((w >> 20) & 3) - 1, ((w >> 22) & 3) - 1};
+    int word = 0;
+    for (int x = 0; x < 2; ++x) {
+      const int p = at[x] % n, q = at[x] / n, neg = sg[x] * (ev.hsc[p] < 0 ? -1 : 1);
+      word |= sym_at(n, p, q) << (10 * x) | (neg + 1) << (20 + 2 * x);
+    }
+    ev.sout.push_back(word);
+  }
+}
+
 // The real basis: same-orbital pairs, then the sums, then i times the
 // differences, of the pairs (a,b), (b,a) with the smaller index first.  With
 // rows e_l, e_l + e_Pl, i (e_l - e_Pl) and the inverse's columns e_l,
@@ -162,6 +195,7 @@ void build_vertex(Even& ev, int n, const double* S, const double* C) {
   to_basis(S, ev.Sb);
   to_basis(C, ev.Cb);
   build_index(ev, n, basis, idx);
+  build_sym(ev, n, basis);
   // Cholesky factors (lower) of S's blocks in the orthonormal basis
   std::vector<double> R((size_t)n * n, 0.0);
   ev.stoner_ok = n <= 32;
@@ -395,6 +429,8 @@ std::shared_ptr<Even> make_even(const Geom& g, const Pairs& p, const double* S, 
   if (S && C) {
     put(ev->d_vin, ev->vin);
     put(ev->d_vout, ev->vout);
+    put(ev->d_sin, ev->sin);
+    put(ev->d_sout, ev->sout);
   }
   sync();
   return ev;

@@ -24,8 +24,8 @@
 //
 // Measured on one FLEX iteration of five orbitals, general form -> this one:
 // 32x32 points and 512 frequencies in FP64, where both are bound by the FP64
-// pipe, chi0 44 -> 9.4 ms, Sigma 62 -> 10.1 ms, vertex 122 -> 33 ms; 64x64 and
-// 1024 in FP32 chi0 40 -> 9.3 ms, Sigma 51 -> 10.2 ms, vertex 45 -> 24 ms.
+// pipe, chi0 44 -> 9.4 ms, Sigma 62 -> 10.1 ms, vertex 122 -> 22 ms; 64x64 and
+// 1024 in FP32 chi0 40 -> 9.3 ms, Sigma 51 -> 10.2 ms, vertex 45 -> 19 ms.
 // Without the symmetry (complex or s-p like hoppings), for planes that do not
 // fit in shared memory and for spin-orbit models the general form remains.
 //
@@ -76,10 +76,12 @@ struct Even {
   bool vertex_ok = false;           // the real-basis vertex applies (constants in vs/vc)
   std::vector<double> Sb, Cb;       // S and C in the real basis, row-major
   std::vector<int> vin, vout;       // index tables of the real basis (see even_impl.cuh)
+  std::vector<int> sin, sout;       // the same for its symmetric form (k_vertex_sym)
+  std::vector<double> hsc;          // and the scaling h of its rows (even.cu, build_sym)
   int nself = 0, nplus = 0;         // same-orbital pairs; pairs in the first (even) block at nu = 0
   bool stoner_ok = false;           // S positive definite: Cholesky factors of its two blocks in d_schol
   DBuf<double> d_schol;
-  DBuf<int> d_vin, d_vout;
+  DBuf<int> d_vin, d_vout, d_sin, d_sout;
 };
 
 // The even-model tables of a mesh and pair list, or null where they do not

@@ -30,7 +30,7 @@ template <typename R> struct SpaceArgs {
   const int *h_irr, *irr_h;
   const int *korder, *koff;    // irreducible k by plane of the half grid
   const int* el;               // boson in: element per array; fermion in / Sigma out: orbital element
-  const R* stat;               // boson in: static slot per array
+  const R* stat;               // boson in: static part per array
   // chi out
   const int *mem, *memcj, *nmem;
   const cx<R>* J;              // per array; null without the tail
@@ -38,6 +38,7 @@ template <typename R> struct SpaceArgs {
   int full;
   // Sigma out
   const int* elt;              // transposed element
+  const double* c0;            // constant per array
   double scale;
   int thresh;
 };
@@ -74,8 +75,13 @@ __device__ __forceinline__ cx<R> space_load(const SpaceArgs<R>& a, int h, int j,
     }
   } else if constexpr (IN == kInBoson) {
     const cx<R>* v = static_cast<const cx<R>*>(a.src) + (long long)a.el[arr] * a.Nk * a.Nw + a.h_irr[h];
-    const cx<R> p = v[(long long)a.Nk * j];
-    const cx<R> q = j ? conj(v[(long long)a.Nk * (a.Nw - j)]) : cmk<R>(stat, (R)0);
+    // without the static part, which is a constant in the result (k_even_const)
+    cx<R> p = v[(long long)a.Nk * j], q = cmk<R>((R)0, (R)0);
+    p.x = p.x - stat;
+    if (j) {
+      q = conj(v[(long long)a.Nk * (a.Nw - j)]);
+      q.x = q.x - stat;
+    }
     return pre_mix<R>(p, q, w);
   } else if constexpr (IN == kInFermi64) {
     const double2* v = static_cast<const double2*>(a.src) + (long long)a.el[arr] * a.Nk * a.Nw + a.h_irr[h];
@@ -111,6 +117,7 @@ __device__ __forceinline__ void space_store(const SpaceArgs<R>& a, int out, cx<R
     double2* s = static_cast<double2*>(a.dst);
     double2 d = mkc((double)v.x, (double)v.y);
     d = a.scale * d;
+    d.x += a.c0[arr];
     if (a.thresh) d = thresh(d);
     s[a.el[arr] * K + at] = d;
     if (a.elt[arr] != a.el[arr]) s[a.elt[arr] * K + at] = d;
@@ -383,7 +390,7 @@ __global__ void k_even_jump(cx<R>* J, const EvenPair* pairs, const double2* rb, 
   J[c] = cmk<R>((R)v.x, (R)v.y);
 }
 
-// static slots a S + b C of the classes' vertex
+// static parts a S + b C of the classes' vertex
 template <typename R>
 __global__ void k_even_static(R* out, const double* S, const double* C, const int* cls_el, double a, double b, int nc) {
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
@@ -463,6 +470,21 @@ __global__ void k_even_contract(cx<R>* out, const cx<R>* W, const cx<R>* F, cons
     }
   }
   out[o * P + i] = cmk<R>(x, y) * twid<R>(root, s, 1);
+}
+
+// What the static part of W gives an output: its transform is one spike at r = tau = 0,
+// so a constant in (k, i omega).  The spike is as large as all frequencies together, and
+// its rounding in the transforms was what FP32 Sigma's error came from: one orbital
+// 16x16x256 1.06e-6 of its norm in this stage (general form 6.5e-7).
+template <typename R>
+__global__ void k_even_const(double* c0, const R* stat, const cx<R>* F, const EvenTerm* terms, const int* tb, long long P,
+                             const int* pos, int H, double scale, int no) {
+  const int o = blockIdx.x * blockDim.x + threadIdx.x;
+  if (o >= no) return;
+  const long long at = (long long)H * pos[0];
+  double s = 0.0;
+  for (int t = tb[o]; t < tb[o + 1]; ++t) s += (double)stat[terms[t].c] * (double)F[terms[t].f * P + at].x;
+  c0[o] = scale * s;
 }
 
 // ------------------------------------------------------------------- vertex
@@ -594,7 +616,9 @@ __device__ __forceinline__ bool real_inverse_rot(R (&a)[N], R* prow, int* piv, i
 
 struct EvenVertexTabs {
   const int *vin, *vout, *rep, *mem, *memcj, *nmem;
-  int ncls, nself, full;
+  int ncls, nself, nplus, full;
+  // the matrices to take, and their number; null: all of them
+  const unsigned *list, *count;
 };
 
 // The FLEX vertex in the real basis.  A warp holds 32 / N matrices (one row per
@@ -602,14 +626,18 @@ struct EvenVertexTabs {
 // V is real.  consts: Si, Ci (inverses of S and C), D = S + C, S, C in the
 // basis, row-major; D is dense on the nself same-orbital pairs and diagonal
 // elsewhere.  FP64: bound by its pipe (91 % at N = 25, 33 ms for 263,168
-// matrices; general form 122 ms).  FP32: issue bound; predecoded source offsets,
+// matrices; general form 122 ms, k_vertex_sym 22).  FP32: issue bound; predecoded source offsets,
 // the pivot row in 16-byte stores and D's row in registers took 2.1 M matrices from
-// 24.0 to 20.4 ms (general form 45 ms).
-template <typename R, int N, int W>
+// 24.0 to 20.4 ms (general form 45 ms), D's product from the left through the transposed
+// entries instead of five shuffles a column to 19.0.
+template <typename R, int N, int W, int mode>
 __global__ void __launch_bounds__(32 * W, sizeof(R) == 4 ? 4 : 2)
-    k_vertex_even(cx<R>* chi, long long nmat, long long estride, const R* consts, EvenVertexTabs tb, int mode,
-                  int* err) {
+    k_vertex_even(cx<R>* chi, long long nmat, long long estride, const R* consts, EvenVertexTabs tb, int* err) {
   constexpr int G = 32 / N, T = W * G, TP = T + 1, PL = rrow_len<R>(N);
+  if (tb.list) {
+    nmat = *tb.count;
+    if (nmat == 0) return;
+  }
   extern __shared__ __align__(16) unsigned char smraw[];
   R* prow = reinterpret_cast<R*>(smraw);                    // [T][2][PL]
   cx<R>* tile = reinterpret_cast<cx<R>*>(prow + (size_t)T * 2 * PL);  // [ncls][TP]
@@ -652,7 +680,8 @@ __global__ void __launch_bounds__(32 * W, sizeof(R) == 4 ? 4 : 2)
     for (int idx = threadIdx.x; idx < tb.ncls * T; idx += blockDim.x) {
       const int tt = idx % T, e = idx / T;
       // matrices past the end repeat the last one: every group has a regular matrix
-      tile[e * TP + tt] = chi[m0 + min(tt, nt - 1) + estride * tb.rep[e]];
+      const long long m = m0 + min(tt, nt - 1);
+      tile[e * TP + tt] = chi[(tb.list ? tb.list[m] : m) + estride * tb.rep[e]];
     }
     __syncthreads();
     R a[N];
@@ -723,18 +752,30 @@ __global__ void __launch_bounds__(32 * W, sizeof(R) == 4 ? 4 : 2)
       const R m4 = (R)-0.25f;
       const R dl = m4 * D[i * N + i];
       constexpr int NH = N < 8 ? N : 8;
+      const bool head = i < ns;
+      // D from the left mixes the ns same-orbital rows only.  Outside of their block
+      // they are the columns of the others, row i entry q / row q entry i = h_q / h_i
+      // with h = 1, 2, -2 for the three kinds of rows
+      const R hi = (R)(i < tb.nplus ? 0.5f : -0.5f);
+#pragma unroll
+      for (int q = 0; q < N; ++q) {
+        const R v = dl * a[q];
+        if (act && !head) {
+          vw[q * N + i] = vw[q * N + i] + v;
+          if (q < NH && q < ns) vw[i * N + q] = vw[i * N + q] + hi * v;
+        }
+      }
       R dh[NH];
 #pragma unroll
       for (int r = 0; r < NH; ++r) dh[r] = r < ns ? m4 * D[i * N + r] : (R)0;
-      const bool head = i < ns;
 #pragma unroll
-      for (int q = 0; q < N; ++q) {
+      for (int q = 0; q < NH; ++q) {
+        if (q >= ns) continue;
         R sum = (R)0;
 #pragma unroll
         for (int r = 0; r < NH; ++r)
           if (r < ns) sum = mad(dh[r], shfl_idx(a[q], g * N + r), sum);
-        const R v = head ? sum : dl * a[q];
-        if (act) vw[q * N + i] = vw[q * N + i] + v;
+        if (act && head) vw[q * N + i] = vw[q * N + i] + sum;
       }
     }
     if (!ok && act && t < nt) atomicExch(err, 3);
@@ -762,19 +803,413 @@ __global__ void __launch_bounds__(32 * W, sizeof(R) == 4 ? 4 : 2)
   }
 }
 
+// The vertex of FP64 with the spin inverse (S^-1 - X)^-1 from the symmetric form of the
+// real basis (even.cu, build_sym).  Row-per-lane elimination (k_vertex_even) spends N
+// FMAs a row and step, and 7 of 32 lanes idle at N = 25; here
+//  * a row keeps its N / 2 + 1 cyclic diagonals, in registers: half of the FMAs.
+//    Row i needs entries i + d of the pivot column, which lies in shared memory twice
+//    over, so that the offsets are constants;
+//  * a warp works on G matrices, their rows dealt out over four register rows per lane:
+//    125 of 128 at N = 25;
+//  * the inverse is swept in place, M -> -M^-1 after every diagonal entry has been
+//    the pivot once, the largest that is left each time: no interchanges.  A pivot
+//    below an eighth of its column (an indefinite M, which no chi0 below its
+//    instability gives) or not finite sends the matrix to k_vertex_even through `list`.
+// The charge inverse keeps the row pivots: C's same-orbital block is indefinite (an
+// eigenvalue -J among 2 U' - J + ...), and a sweep of C^-1 + X doubled the error of
+// Sigma (four orbitals, 16x16x128: 1.5e-15 with row pivots, 3.5e-15 swept, of its norm).
+// Bound by the FP64 pipe (75 % busy with both inverses swept).  Eight warps, two to a
+// scheduler, are what shared memory holds at N = 25 if X is staged twice, in halves of the
+// tile: 15.9 ms against 17.4 with six and X kept (263,168 matrices, both inverses swept).
+constexpr int kSymRows = 4;
+template <int N> __host__ __device__ constexpr int sym_group() { return 32 * kSymRows / N; }
+template <int N> __host__ __device__ constexpr int sym_half() { return (N / 2 + 1) * N; }
+template <int N> __host__ __device__ constexpr int sym_keys() { return (N + 3) & ~3; }
+// place of entry (p, q); at even N the diagonal d = N / 2 holds its pairs twice, the
+// first half is read
+template <int N> __device__ __forceinline__ int sym_at(int p, int q) {
+  const int d = q >= p ? q - p : q - p + N;
+  return 2 * d < N || (2 * d == N && p < q) ? d * N + p : (N - d) * N + q;
+}
+
+// magnitude as an ordered integer; kSymExpo is a factor of two
+__device__ __forceinline__ unsigned sym_mag(double a) { return (unsigned)__double2hiint(a) & 0x7fffffffu; }
+constexpr unsigned kSymExpo = 1u << 20;
+
+struct SymTabs {
+  const int *sin, *sout, *rep, *mem, *memcj, *nmem;
+  int ncls, nself, full;
+  unsigned *list, *count;  // out: the matrices left to k_vertex_even
+};
+
+template <typename R, int N, int W> struct SymSmem {
+  static constexpr int G = sym_group<N>(), T = W * G, TH = T / 2, HL = sym_half<N>(), KP = sym_keys<N>();
+  static_assert(T % 2 == 0, "the tile is staged in two halves");
+  static __host__ __device__ size_t tile(int ncls) { return sizeof(cx<R>) * (size_t)ncls * (TH + 1); }
+  static constexpr int CS = (2 * HL + N * N + N + 65) & ~1;  // constants, an even number
+  static __host__ __device__ size_t bytes(int ncls) {
+    return tile(ncls) + sizeof(R) * ((size_t)T * HL + CS + T * (3 * N + 1)) +
+           sizeof(int) * ((size_t)T * KP + HL + 3 * T + 64 * W);
+  }
+};
+
+// consts: Si (as M) and the coefficients of the sandwich, HL entries each; Ci
+// column-major, N^2; 1 / h, N; the nself x nself block of S + C, 64; then the W forms
+// of S and C, HL each
+template <typename R, int N, int W>
+__global__ void __launch_bounds__(32 * W, N == 9 ? 2 : 1)
+    k_vertex_sym(cx<R>* chi, long long nmat, long long estride, const R* consts, SymTabs tb, int mode, int* err) {
+  using L = SymSmem<R, N, W>;
+  constexpr int G = L::G, T = L::T, TH = L::TH, TP = TH + 1, HL = L::HL, KP = L::KP, DG = N / 2 + 1, SL = kSymRows;
+  constexpr int DK = (N & 1) ? DG : DG - 1;  // diagonals that the pivot row publishes
+  extern __shared__ __align__(16) unsigned char smraw[];
+  cx<R>* tile = reinterpret_cast<cx<R>*>(smraw);  // [ncls][TP]: half of the matrices at a time
+  unsigned* keys = reinterpret_cast<unsigned*>(smraw + L::tile(tb.ncls));  // [T][KP]
+  R* xb = reinterpret_cast<R*>(keys + T * KP);                             // [T][HL]: X, then the result
+  R* cst = xb + T * HL;
+  const R *K = cst + HL, *Ci = cst + 2 * HL, *hinv = Ci + N * N, *qh = hinv + N;
+  R* cbuf = cst + L::CS;       // [T][2N]
+  R* diag = cbuf + T * 2 * N;  // [T][N]
+  R* ipb = diag + T * N;       // [T]
+  int* sin = reinterpret_cast<int*>(ipb + T);  // [HL]
+  int* pvb = sin + HL;                         // [T]
+  unsigned* pkb = reinterpret_cast<unsigned*>(pvb + T);  // [T]
+  int* badb = reinterpret_cast<int*>(pkb + T);           // [T]
+  int* perm = badb + T;                                  // [W][64]
+  const int ns = tb.nself;
+  for (int e = threadIdx.x; e < L::CS; e += blockDim.x) cst[e] = consts[e];
+  for (int e = threadIdx.x; e < HL; e += blockDim.x) sin[e] = tb.sin[e];
+  for (int e = threadIdx.x; e < T * KP; e += blockDim.x) keys[e] = 0u;
+  const R *WS = consts + L::CS, *WC = WS + HL;
+  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const R c1 = mode == 2 ? (R)0.5f : (R)-1.5f;  // of the swept -M^-1
+  const R c2 = mode == 0 ? (R)-0.5f : (R)0.5f;
+  // the lane's rows: matrix t (of the CTA's tile) and row i; rows past the last one
+  // mirror it without writing
+  int rt[SL], ri[SL];
+  bool act[SL];
+#pragma unroll
+  for (int s = 0; s < SL; ++s) {
+    const int r = s * 32 + lane, rr = min(r, G * N - 1);
+    act[s] = r < G * N;
+    rt[s] = w * G + rr / N;
+    ri[s] = rr % N;
+  }
+  R a[SL][DG];
+  // half h of the tile; matrices past the end repeat the last one, so that every row
+  // belongs to a regular matrix
+  auto stage = [&](long long m0, int nt, int h) {
+    for (int idx = threadIdx.x; idx < tb.ncls * TH; idx += blockDim.x) {
+      const int tt = idx % TH, e = idx / TH;
+      tile[e * TP + tt] = chi[m0 + min(h * TH + tt, nt - 1) + estride * tb.rep[e]];
+    }
+    __syncthreads();
+  };
+  // entry e of the symmetric form of X, of matrix tt of the staged half
+  auto entry = [&](int e, int tt) {
+    const R* tr = reinterpret_cast<const R*>(tile) + 2 * tt;
+    const int word = sin[e], ia = word & 511, ib = (word >> 9) & 511;
+    R v = tr[2 * (ia >> 1) * TP + (ia & 1)];
+    if (word >> 18 & 1) v = -v;
+    if (word >> 20 & 1) {
+      const R u = tr[2 * (ib >> 1) * TP + (ib & 1)];
+      v = v + ((word >> 19 & 1) ? -u : u);
+    }
+    if (word >> 21 & 1) v = v + v;
+    return v;
+  };
+  for (long long m0 = (long long)blockIdx.x * T; m0 < nmat; m0 += (long long)gridDim.x * T) {
+    const int nt = (int)min((long long)T, nmat - m0);
+    __syncthreads();
+    if (threadIdx.x < T) badb[threadIdx.x] = 0;
+    for (int h = 0; h < 2; ++h) {
+      stage(m0, nt, h);
+      for (int idx = threadIdx.x; idx < HL * TH; idx += blockDim.x) {
+        const int tt = idx % TH, e = idx / TH;
+        xb[(h * TH + tt) * HL + e] = entry(e, tt);
+      }
+      __syncthreads();
+    }
+    // (Si - X)^-1 by sweeps, into registers
+#pragma unroll
+    for (int s = 0; s < SL; ++s)
+#pragma unroll
+      for (int d = 0; d < DG; ++d) a[s][d] = cst[d * N + ri[s]] - xb[rt[s] * HL + d * N + ri[s]];
+    unsigned done = 0u;
+#pragma unroll
+    for (int s = 0; s < SL; ++s)
+      if (act[s]) {
+        diag[rt[s] * N + ri[s]] = a[s][0];
+        keys[rt[s] * KP + ri[s]] = (sym_mag(a[s][0]) & ~31u) | (unsigned)(31 - ri[s]);
+      }
+    __syncwarp();
+#pragma unroll 1
+    for (int step = 0; step < N; ++step) {
+      if (lane < G) {
+        const int t = w * G + lane;
+        const uint4* k4 = reinterpret_cast<const uint4*>(keys + t * KP);
+        unsigned best = 0u;
+#pragma unroll
+        for (int x = 0; x < KP / 4; ++x) {
+          const uint4 v = k4[x];
+          best = max(best, max(max(v.x, v.y), max(v.z, v.w)));
+        }
+        const int k = 31 - (int)(best & 31u);
+        const unsigned ex = best / kSymExpo;
+        if (ex == 0u || ex == 0x7fffffffu / kSymExpo) badb[t] = 1;  // zero, tiny or not finite
+        pvb[t] = k;
+        pkb[t] = best;
+        ipb[t] = (R)1 / diag[t * N + k];
+      }
+      __syncwarp();
+      int dd[SL];
+#pragma unroll
+      for (int s = 0; s < SL; ++s) {
+        const int i = ri[s], x = pvb[rt[s]] - i;
+        dd[s] = x < 0 ? x + N : x;
+        if (!act[s]) continue;
+        R* cb = cbuf + rt[s] * 2 * N;
+        R c = a[s][0];
+#pragma unroll
+        for (int d = 1; d < DG; ++d) {
+          const R x = a[s][d];
+          c = d == dd[s] ? x : c;
+        }
+        if (dd[s] < DG) cb[i] = cb[i + N] = c;
+        if (dd[s] == 0) {
+#pragma unroll
+          for (int d = 1; d < DK; ++d) {
+            const int j = i + d < N ? i + d : i + d - N;
+            cb[j] = cb[j + N] = a[s][d];
+          }
+        }
+      }
+      __syncwarp();
+#pragma unroll
+      for (int s = 0; s < SL; ++s) {
+        const R* cb = cbuf + rt[s] * 2 * N + ri[s];
+        const bool piv = dd[s] == 0;
+        const R c = cb[0], ip = ipb[rt[s]];
+        if (act[s] && !piv && !(done >> s & 1u) && sym_mag(c) > pkb[rt[s]] + 3u * kSymExpo) badb[rt[s]] = 1;
+        const R f = piv ? ip : -(c * ip);
+#pragma unroll
+        for (int d = 0; d < DG; ++d) {
+          const R v = mad(f, cb[d], piv ? (R)0 : a[s][d]);
+          a[s][d] = d == dd[s] ? -f : v;
+        }
+        if (piv) done |= 1u << s;
+        if (act[s]) {
+          diag[rt[s] * N + ri[s]] = a[s][0];
+          keys[rt[s] * KP + ri[s]] =
+              (done >> s & 1u) ? 0u : ((sym_mag(a[s][0]) & ~31u) | (unsigned)(31 - ri[s]));
+        }
+      }
+      __syncwarp();
+    }
+    // (Ci + X)^-1 with row pivots, 32 / N matrices of the warp at a time, over X
+    constexpr int GP = 32 / N, PL = rrow_len<R>(N);
+    const int gp = lane / N < GP ? lane / N : 0;
+    const bool actp = lane < GP * N;
+    const int ip = actp ? lane - gp * N : 0;
+#pragma unroll 1
+    for (int m = 0; m < G; m += GP) {
+      const int t = w * G + min(m + gp, G - 1);
+      const bool keep = actp && m + gp < G;
+      R b[N];
+#pragma unroll
+      for (int q = 0; q < N; ++q) b[q] = mad(xb[t * HL + sym_at<N>(ip, q)], hinv[q], Ci[q * N + ip]);
+      int lab;
+      R sc;
+      int* pp = perm + w * 64 + gp * 2 * N;
+      const bool ok = real_inverse_rot<R, N>(b, cbuf + w * G * 2 * N + gp * 2 * PL, pp, pp + N, lab, sc, gp * N, ip, actp);
+      if (!ok && keep && t < nt) atomicExch(err, 3);
+      const R f = c2 * (sc * hinv[lab]);
+      if (keep) {
+#pragma unroll
+        for (int q = 0; q < N; ++q) {
+          const int c = pp[N + q], d = c >= lab ? c - lab : c - lab + N;
+          if (2 * d < N || (2 * d == N && lab < c)) xb[t * HL + d * N + lab] = f * b[q];
+        }
+      }
+      __syncwarp();
+    }
+#pragma unroll
+    for (int s = 0; s < SL; ++s)
+#pragma unroll
+      for (int d = 0; d < DG; ++d) {
+        const int e = d * N + ri[s];
+        R* v = xb + rt[s] * HL + e;
+        if (!act[s] || (2 * d == N && 2 * ri[s] >= N)) continue;
+        R c = mad(c1, a[s][d], *v);
+        if (mode == 1) c = c - WS[e];
+        else if (mode == 2) c = c + (WS[e] - WC[e]);
+        *v = c;
+      }
+    for (int h = 0; mode == 0 && h < 2; ++h) {
+      // -1/4 (S + C) X (S + C), X staged once more (keeping it would take the shared
+      // memory of two warps): S + C is dense on the ns same-orbital pairs, diagonal
+      // elsewhere.  K: -1/4 and the products with the diagonal ones
+      __syncthreads();
+      stage(m0, nt, h);
+      for (int idx = threadIdx.x; idx < HL * TH; idx += blockDim.x) {
+        const int tt = idx % TH, e = idx / TH, p = e % N, q = p + e / N < N ? p + e / N : p + e / N - N;
+        if (p < ns || q < ns) continue;
+        R* v = xb + (h * TH + tt) * HL + e;
+        *v = mad(K[e], entry(e, tt), *v);
+      }
+      auto add = [&](int t, int p, int q, R v) {
+        const int e = sym_at<N>(p, q);
+        xb[t * HL + e] = mad(K[e], v, xb[t * HL + e]);
+      };
+      // the dense block's rows, column j; its own columns go to z for the other side
+      constexpr int NH = N < 8 ? N : 8;
+      for (int idx = threadIdx.x; idx < TH * N; idx += blockDim.x) {
+        const int tt = idx % TH, j = idx / TH, t = h * TH + tt;
+        R* z = cbuf + t * 2 * N;
+        R in[NH];
+#pragma unroll
+        for (int r = 0; r < NH; ++r) in[r] = r < ns ? entry(sym_at<N>(r, j), tt) : (R)0;
+        for (int r = 0; r < ns; ++r) {
+          R sum = (R)0;
+#pragma unroll
+          for (int q = 0; q < NH; ++q)
+            if (q < ns) sum = mad(qh[r * ns + q], in[q], sum);
+          if (j >= ns) add(t, r, j, sum);
+          else z[j * ns + r] = sum;
+        }
+      }
+      __syncthreads();
+      for (int idx = threadIdx.x; idx < TH * ns * ns; idx += blockDim.x) {
+        const int t = h * TH + idx % TH, p = idx / TH / ns, q = idx / TH % ns;
+        if (p > q) continue;
+        const R* z = cbuf + t * 2 * N;
+        R sum = (R)0;
+        for (int s = 0; s < ns; ++s) sum = mad(z[s * ns + p], qh[s * ns + q], sum);
+        add(t, p, q, sum);
+      }
+    }
+    __syncthreads();
+    for (int idx = threadIdx.x; idx < tb.ncls * T; idx += blockDim.x) {
+      const int tt = idx % T, e = idx / T;
+      if (tt >= nt || badb[tt]) continue;
+      const R* v = xb + (size_t)tt * HL;
+      R part[2];
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const int word = tb.sout[2 * e + h], sa = word >> 20 & 3, sb = word >> 22 & 3;
+        R r = sa == 1 ? (R)0 : v[word & 1023];
+        if (sa == 0) r = -r;
+        if (sb != 1) {
+          const R y = v[(word >> 10) & 1023];
+          r = r + (sb == 0 ? -y : y);
+        }
+        part[h] = r;
+      }
+      const cx<R> z = cmk<R>(part[0], part[1]);
+      const int n = tb.full ? tb.nmem[e] : 1;
+      for (int m = 0; m < n; ++m)
+        chi[m0 + tt + estride * tb.mem[4 * e + m]] = tb.memcj[4 * e + m] ? conj(z) : z;
+    }
+    if (threadIdx.x < nt && badb[threadIdx.x]) tb.list[atomicAdd(tb.count, 1u)] = (unsigned)(m0 + threadIdx.x);
+  }
+}
+
+// A^-1 of a real matrix that host_inverse accepts, in the arithmetic of the kernels:
+// their elimination of S^-1 -+ X then undoes these roundings.  The rounding of an exact
+// C^-1 does not cancel like that; C^-1's same-orbital block has entries of 30 times its
+// smallest eigenvalue, and the error is the same in every matrix, so that it adds up in
+// Sigma.
+template <typename R> std::vector<R> inverse_as(const std::vector<double>& X, int n) {
+  std::vector<R> A((size_t)n * n);
+  for (size_t e = 0; e < A.size(); ++e) A[e] = (R)X[e];
+  std::vector<int> piv(n);
+  for (int k = 0; k < n; ++k) {
+    int p = k;
+    for (int r = k + 1; r < n; ++r)
+      if (std::fabs((double)A[r * n + k]) > std::fabs((double)A[p * n + k])) p = r;
+    piv[k] = p;
+    if (p != k)
+      for (int j = 0; j < n; ++j) std::swap(A[k * n + j], A[p * n + j]);
+    const R d = (R)1 / A[k * n + k];
+    A[k * n + k] = (R)1;
+    for (int j = 0; j < n; ++j) A[k * n + j] = A[k * n + j] * d;
+    for (int r = 0; r < n; ++r) {
+      if (r == k) continue;
+      const R f = A[r * n + k];
+      A[r * n + k] = (R)0;
+      for (int j = 0; j < n; ++j) A[r * n + j] = A[r * n + j] - f * A[k * n + j];
+    }
+  }
+  for (int k = n - 1; k >= 0; --k)
+    if (piv[k] != k)
+      for (int r = 0; r < n; ++r) std::swap(A[r * n + k], A[r * n + piv[k]]);
+  return A;
+}
+
 template <typename R, int N>
-void vertex_even_launch(const Even& ev, cx<R>* chi, long long nmat, long long estride, const R* dc, int mode, bool full) {
+void vertex_even_launch(const Even& ev, cx<R>* chi, long long nmat, long long estride, const R* dc, int mode, bool full,
+                        const unsigned* list = nullptr, const unsigned* count = nullptr) {
   constexpr int W = 8, T = W * (32 / N);
   const int nc = (int)ev.cls.size();
   const size_t smem = sizeof(R) * ((size_t)T * 2 * rrow_len<R>(N) + (size_t)T * N * N + 3 * N * N) +
                       sizeof(cx<R>) * (size_t)nc * (T + 1) + sizeof(R) + sizeof(int) * (2 * N * N + 2 * T * N);
-  PGB_SMEM_LIMIT_ONCE((k_vertex_even<R, N, W>), 220 * 1024);
-  EvenVertexTabs tb{ev.d_vin.p, ev.d_vout.p, ev.cls_el.p, ev.mem.p, ev.memcj.p, ev.nmem.p, nc, ev.nself, full ? 1 : 0};
+  EvenVertexTabs tb{ev.d_vin.p, ev.d_vout.p, ev.cls_el.p, ev.mem.p, ev.memcj.p, ev.nmem.p, nc, ev.nself, ev.nplus, full ? 1 : 0,
+                    list, count};
   const long long tiles = (nmat + T - 1) / T;
   const long long blocks = std::min<long long>(tiles, (long long)ctx().num_sms * 16);
-  k_vertex_even<R, N, W><<<(unsigned)std::max(1LL, blocks), 32 * W, smem, ctx().stream>>>(chi, nmat, estride, dc, tb,
-                                                                                         mode, ctx().err);
+#define PGB_VE(m_)                                                                                                      \
+  do {                                                                                                                 \
+    PGB_SMEM_LIMIT_ONCE((k_vertex_even<R, N, W, m_>), 220 * 1024);                                                     \
+    k_vertex_even<R, N, W, m_><<<(unsigned)std::max(1LL, blocks), 32 * W, smem, ctx().stream>>>(chi, nmat, estride, dc, \
+                                                                                               tb, ctx().err);         \
+  } while (0)
+  if (mode == 0) PGB_VE(0);
+  else if (mode == 1) PGB_VE(1);
+  else PGB_VE(2);
+#undef PGB_VE
   count_launch("vertex_even");
+}
+
+// k_vertex_sym, then k_vertex_even on the matrices that it has left; false where a
+// pair list's same-orbital block or classes do not fit its buffers
+template <typename R, int N, int W>
+bool vertex_sym_launch(const Even& ev, cx<R>* chi, long long nmat, long long estride, const R* dc, int mode, bool full) {
+  using L = SymSmem<R, N, W>;
+  constexpr int HL = L::HL;
+  const int nc = (int)ev.cls.size(), ns = ev.nself;
+  if (ns * ns > 2 * N || ns * ns > 64 || L::bytes(nc) > 220 * 1024 || nmat >= (1LL << 32)) return false;
+  std::vector<R> c(L::CS + 2 * HL);
+  std::vector<double> Si(ev.Sb), Ci(ev.Cb), Q((size_t)N * N);
+  PGB_CHECK(host_inverse(Si, N) && host_inverse(Ci, N), "singular interaction matrix in the real-basis vertex");
+  for (int e = 0; e < N * N; ++e) Q[e] = ev.Sb[e] + ev.Cb[e];
+  for (int p = 0; p < N; ++p) {
+    for (int d = 0; d <= N / 2; ++d) {
+      const int q = (p + d) % N, e = d * N + p, pq = p * N + q;
+      const double hp = ev.hsc[p], hq = ev.hsc[q];
+      c[e] = (R)(Si[pq] * hq);
+      // the rows of the dense block are multiplied through before
+      c[HL + e] = (R)(-0.25 * (p < ns ? 1.0 : Q[p * N + p] / hp) * (q < ns ? 1.0 : Q[q * N + q] / hq));
+      c[L::CS + e] = (R)(ev.Sb[pq] / hp);
+      c[L::CS + HL + e] = (R)(ev.Cb[pq] / hp);
+    }
+    for (int q = 0; q < N; ++q) c[2 * HL + q * N + p] = (R)Ci[p * N + q];
+    c[2 * HL + N * N + p] = (R)(1.0 / ev.hsc[p]);
+  }
+  for (int p = 0; p < ns; ++p)
+    for (int q = 0; q < ns; ++q) c[2 * HL + N * N + N + p * ns + q] = (R)Q[p * N + q];
+  DBuf<R> ds(c.size());
+  ds.upload(c.data(), c.size());
+  DBuf<unsigned> list(nmat), count(1);
+  count.zero();
+  PGB_SMEM_LIMIT_ONCE((k_vertex_sym<R, N, W>), 220 * 1024);
+  SymTabs tb{ev.d_sin.p, ev.d_sout.p, ev.cls_el.p, ev.mem.p, ev.memcj.p, ev.nmem.p, nc, ns, full ? 1 : 0, list.p, count.p};
+  const long long tiles = (nmat + L::T - 1) / L::T;
+  const long long blocks = std::max(1LL, std::min<long long>(tiles, (long long)ctx().num_sms * 8));
+  k_vertex_sym<R, N, W><<<(unsigned)blocks, 32 * W, L::bytes(nc), ctx().stream>>>(chi, nmat, estride, ds.p, tb, mode,
+                                                                                        ctx().err);
+  count_launch("vertex_sym");
+  vertex_even_launch<R, N>(ev, chi, nmat, estride, dc, mode, full, list.p, count.p);
+  return true;
 }
 
 // ------------------------------------------------------------------- stoner
@@ -1002,22 +1437,22 @@ void chi0_even(const Geom& g, const double2* G, double temp, const TailRef* tail
   }
 }
 
-// transforms of the classes' vertex elements V, static slots a S + b C
+// transforms of the classes' vertex elements V without their static parts stat = a S + b C
 template <typename R>
 void vertex_transforms(const Geom& g, const cx<R>* V, const double* S, const double* C, double wS, double wC, cx<R>* W,
-                       cudaStream_t st) {
+                       DBuf<R>& stat, cudaStream_t st) {
   const Even& ev = *g.even;
   const int nc = (int)ev.cls.size(), ch = even_batch<R>(ev);
   const size_t P = (size_t)ev.H * ev.Nw;
-  DBuf<R> dstat(nc);
-  k_even_static<R><<<(nc + 127) / 128, 128, 0, st>>>(dstat.p, S, C, ev.cls_el.p, wS, wC, nc);
+  stat.alloc(nc);
+  k_even_static<R><<<(nc + 127) / 128, 128, 0, st>>>(stat.p, S, C, ev.cls_el.p, wS, wC, nc);
   count_launch("even_static");
   SpaceArgs<R> b{};
   b.Nk = g.Nk;
   b.src = V;
   for (int c0 = 0; c0 < nc; c0 += ch) {
     b.el = ev.cls_el.p + c0;
-    b.stat = dstat.p + c0;
+    b.stat = stat.p + c0;
     even_forward<R, kInBoson>(ev, b, W + c0 * P, std::min(ch, nc - c0), true, st);
   }
 }
@@ -1037,7 +1472,9 @@ void sigma_even(const Geom& g, const double2* G, const cx<R>* V, const double* S
   a.src = G;
   a.el = ev.d_sym_el.p;
   fermi_transform<R>(ev, a, F.p, ns, false, st);
-  vertex_transforms<R>(g, V, S, C, 1.5, -0.5, W.p, st);
+  DBuf<R> stat;
+  DBuf<double> c0(ns);
+  vertex_transforms<R>(g, V, S, C, 1.5, -0.5, W.p, stat, st);
   const FFT4D& ft = fft_plan_t(H, Nw, (int)sizeof(cx<R>));
   const unsigned tiles = (unsigned)(((H + 255) / 256) * Nw);
   k_even_contract<R><<<tiles * ns, 256, 0, st>>>(T.p, W.p, F.p, ev.sig_terms.p, ev.sig_tb.p, fft_roots<R>(2 * Nw), H, Nw, ft.d_pos(3),
@@ -1050,6 +1487,10 @@ void sigma_even(const Geom& g, const double2* G, const cx<R>* V, const double* S
   o.elt = ev.d_sym_elt.p;
   o.scale = temp / (double)g.Nkall / (double)g.P;
   o.thresh = 1;
+  o.c0 = c0.p;
+  k_even_const<R><<<(ns + 31) / 32, 32, 0, st>>>(c0.p, stat.p, F.p, ev.sig_terms.p, ev.sig_tb.p, (long long)P, ft.d_pos(3), H,
+                                                o.scale * (double)g.P, ns);
+  count_launch("even_const");
   even_backward<R, kInPostFermi, kOutSigma>(ev, o, T.p, T2.p, ns, st);
 }
 
@@ -1063,7 +1504,7 @@ void mkdelta_even(const Geom& g, const Pairs& p, const double2* F64, const cx<R>
   if (!cache.built) {
     cache.built = true;
     cache.W.alloc((size_t)nc * P);
-    vertex_transforms<R>(g, Vd, S, C, 0.5, 0.5, cache.W.p, st);
+    vertex_transforms<R>(g, Vd, S, C, 0.5, 0.5, cache.W.p, cache.stat, st);
     std::vector<EvenTerm> terms;
     std::vector<int> tb(1, 0), el;
     for (int e = 0; e < No * No; ++e) {
@@ -1107,6 +1548,11 @@ void mkdelta_even(const Geom& g, const Pairs& p, const double2* F64, const cx<R>
     o.dst = out;
     o.el = o.elt = cache.els.p;
     o.scale = scale;
+    DBuf<double> c0(no);
+    o.c0 = c0.p;
+    k_even_const<R><<<(no + 31) / 32, 32, 0, st>>>(c0.p, cache.stat.p, F.p, reinterpret_cast<const EvenTerm*>(cache.ef.p),
+                                                  cache.tb.p, (long long)P, ft.d_pos(3), H, scale * (double)g.P, no);
+    count_launch("even_const");
     even_backward<R, kInPostFermi, kOutSigma>(ev, o, T.p, T2.p, no, st);
   }
   hermitize(out, g.K, No);
@@ -1117,10 +1563,18 @@ bool vertex_even(const Even& ev, cx<R>* chi, long long nmat, long long estride, 
   const int n = (int)ev.perm.size();
   std::vector<double> Si(ev.Sb), Ci(ev.Cb);
   PGB_CHECK(host_inverse(Si, n) && host_inverse(Ci, n), "singular interaction matrix in the real-basis vertex");
+  std::vector<R> Sr(Si.size(), (R)0), Cr(Sr);
+  if (n > 1) {
+    Sr = inverse_as<R>(ev.Sb, n);
+    Cr = inverse_as<R>(ev.Cb, n);
+  } else {
+    Sr[0] = (R)Si[0];
+    Cr[0] = (R)Ci[0];
+  }
   std::vector<R> consts(5 * n * n);
   for (int e = 0; e < n * n; ++e) {
-    consts[e] = (R)Si[e];
-    consts[n * n + e] = (R)Ci[e];
+    consts[e] = Sr[e];
+    consts[n * n + e] = Cr[e];
     consts[2 * n * n + e] = (R)(ev.Sb[e] + ev.Cb[e]);
     consts[3 * n * n + e] = (R)ev.Sb[e];
     consts[4 * n * n + e] = (R)ev.Cb[e];
@@ -1128,6 +1582,17 @@ bool vertex_even(const Even& ev, cx<R>* chi, long long nmat, long long estride, 
   DBuf<R> dc(consts.size());
   dc.upload(consts.data(), consts.size());
   reset_err();
+  // FP64, where the pipe bounds an elimination, takes k_vertex_sym: three orbitals
+  // 32x32x512 (263,168 matrices) 2.74 -> 1.73 ms, four 32x32x256 (131,584) 4.43 -> 3.32,
+  // five 16.6 -> 11.0.  In double-float its bookkeeping takes as long as it saves
+  // (N = 9 even, 16 slower), FP32 and N <= 4 are bound by instructions of other kinds.
+  if constexpr (std::is_same<R, double>::value) {
+    bool done = false;
+    if (n == 9) done = vertex_sym_launch<R, 9, 8>(ev, chi, nmat, estride, dc.p, mode, full);
+    if (n == 16) done = vertex_sym_launch<R, 16, 8>(ev, chi, nmat, estride, dc.p, mode, full);
+    if (n == 25) done = vertex_sym_launch<R, 25, 8>(ev, chi, nmat, estride, dc.p, mode, full);
+    if (done) return fetch_err() == 0;
+  }
   switch (n) {
     case 1: vertex_even_launch<R, 1>(ev, chi, nmat, estride, dc.p, mode, full); break;
     case 4: vertex_even_launch<R, 4>(ev, chi, nmat, estride, dc.p, mode, full); break;

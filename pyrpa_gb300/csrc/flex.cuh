@@ -173,6 +173,7 @@ template <typename R> struct DeltaKernelCache {
   std::vector<int> out_elems;
   DBuf<int> ef, tb;
   DBuf<int> els;  // even form: output elements, then the a <= b elements of F
+  DBuf<R> stat;              // static parts of W (even models)
 };
 // Fbulk: F already in the bulk type (then F is not read; the parity factors
 // prt must be +-1).  even: the even form applies to F (mkdelta_even)

@@ -205,3 +205,40 @@ def test_broken_symmetry_keeps_the_general_form(F):
                                   scf_loop=2, eps=1e-12, arnoldi_m=0, itemax=1, sigma_seed=seed, seed_mu=m["mu"],
                                   seed_mu_old=m["mu"])["sigmak"]
     assert np.array_equal(fused(), general(fused))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dims", [(3, 8, 8, 1, 30), (4, 4, 4, 1, 8), (5, 4, 6, 1, 10)])
+@pytest.mark.parametrize("size", [0.05, 8.0])
+@pytest.mark.parametrize("gap_sym", [0, -1])
+def test_pairing_vertex_of_any_matrix(F, dims, size, gap_sym):
+    """V_Delta of random matrices with an even model's relations in double-float:
+    below the instability (size 0.05) k_vertex_sym keeps every one, far above it
+    the indefinite ones go to the pivoted kernel.  The general form carries 1e-14 too;
+    the worst of some thousand random matrices has a condition number of about 1e5,
+    which leaves 1e-8 of the largest element."""
+    m = model(*dims)
+    No, Nk, n = m["Norb"], len(m["hamk"]), m["Norb"] ** 2
+    rng = np.random.default_rng(No)
+    o = np.asarray(m["olist"])
+    at = {(a, b): i for i, (a, b) in enumerate(zip(o[:, 0], o[:, 1]))}
+    P = [at[(b, a)] for a, b in zip(o[:, 0], o[:, 1])]
+    chi = rng.normal(size=(n, n, m["Nw"], Nk)) + 1j * rng.normal(size=(n, n, m["Nw"], Nk))
+    chi[:, :, 0] = chi[:, :, 0].real
+    chi = chi + chi.transpose(1, 0, 2, 3)
+    chi = np.ascontiguousarray(size * (chi + chi[P][:, P].conj()))
+    init = F.get_initial_gap(m["klist"], No, 0) + 0.1
+    G = dressed(m)
+
+    def run():
+        v = chi.copy()
+        F.linearized_eliashberg(v, G, m["uni"], init, m["S"], m["C"], m["olist"], np.ones(No), m["kmap"], m["invk"],
+                                *m["mesh"], m["temp"], gap_sym, arnoldi_m=0, itemax=1)
+        return v
+
+    F.set_precision(48)
+    try:
+        v, g = run(), general(run)
+    finally:
+        F.set_precision(64)
+    close(v, g, 1e-8, 0.0)
