@@ -480,9 +480,11 @@ double chi0_entry(double2* chi_out, const double* Smat, const double* Cmat, cons
   //    1e-9 .. 2e-8 of the gap (twelve two-orbital models), so its bits stay;
   //  * small calls, which launches bound: 16x16x256, one orbital, 0.27 ms
   //    against 0.33 ms with the even form's tables and checks.
+  // A G without the symmetry shows it in a few host elements, which spares it the
+  // check on the device and its wait (50 us of 1.2 ms: three orbitals 16x16x64).
   const bool even_call = !irr_chi && !chi_map && !(tail && std::is_same<R, double>::value) &&
                          g.P * Nchi * Nchi >= kEvenMinWork;
-  if (even_call && (!tail || symmetric_bands(eig, uni, Nk, (int)Norb)) &&
+  if (even_call && symmetric_sample(Gk, g.K, (int)Norb) && (!tail || symmetric_bands(eig, uni, Nk, (int)Norb)) &&
       symmetric_blocks(G.p, g.K, (int)Norb, 1.0e-12)) {
     if (with_stoner) g.even = make_even(g, p, Smat, Cmat, (int)sizeof(cx<R>));
     if (!g.even) g.even = make_even(g, p, nullptr, nullptr, (int)sizeof(cx<R>));

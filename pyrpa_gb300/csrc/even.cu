@@ -436,6 +436,21 @@ std::shared_ptr<Even> make_even(const Geom& g, const Pairs& p, const double* S, 
   return ev;
 }
 
+bool symmetric_sample(const double2* X, long long n, int No) {
+  double d = 0, m = 0;
+  const long long pts = std::min<long long>(n, 8);  // every element read is a cache miss
+  for (long long s = 0; s < pts; ++s) {
+    const double2* x = X + s * (n / pts);
+    for (int b = 0; b < No; ++b)
+      for (int a = 0; a <= b; ++a) {
+        const double2 u = x[n * (a + No * b)], v = x[n * (b + No * a)];
+        d = std::max(d, std::fabs(u.x - v.x) + std::fabs(u.y - v.y));
+        m = std::max(m, std::fabs(u.x) + std::fabs(u.y));
+      }
+  }
+  return !(d > 1e-9 * m);
+}
+
 bool symmetric_blocks(const double2* X, long long n, int No, double tol) {
   DBuf<unsigned long long> out(2);
   out.zero();

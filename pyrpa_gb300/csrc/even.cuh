@@ -93,6 +93,9 @@ std::shared_ptr<Even> make_even(const Geom& g, const Pairs& p, const double* S, 
 // max |X_ab - X_ba| <= tol max |X| over n matrices of No x No elements at
 // X[i + n (a + No b)]
 bool symmetric_blocks(const double2* X, long long n, int No, double tol);
+// the same of eight of the n matrices in host memory, to 1e-9: false where the whole
+// cannot pass, without the wait for the device that symmetric_blocks ends with
+bool symmetric_sample(const double2* X, long long n, int No);
 // the same with H(k) in the (No, No, Nk) layout of the boundary, on the host
 bool symmetric_h(const double2* H, long long Nk, int No);
 // bands and eigenvectors of a symmetric H: U e U^+ symmetric on every k (host)
