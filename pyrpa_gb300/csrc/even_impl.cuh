@@ -797,8 +797,9 @@ __global__ void __launch_bounds__(32 * W, sizeof(R) == 4 ? 4 : 2)
       }
       const cx<R> z = cmk<R>(part[0], part[1]);
       const int n = tb.full ? tb.nmem[e] : 1;
+      const long long mat = tb.list ? tb.list[m0 + tt] : m0 + tt;
       for (int m = 0; m < n; ++m)
-        chi[m0 + tt + estride * tb.mem[4 * e + m]] = tb.memcj[4 * e + m] ? conj(z) : z;
+        chi[mat + estride * tb.mem[4 * e + m]] = tb.memcj[4 * e + m] ? conj(z) : z;
     }
   }
 }

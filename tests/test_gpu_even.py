@@ -212,11 +212,11 @@ def test_broken_symmetry_keeps_the_general_form(F):
 @pytest.mark.parametrize("size", [0.05, 8.0])
 @pytest.mark.parametrize("gap_sym", [0, -1])
 def test_pairing_vertex_of_any_matrix(F, dims, size, gap_sym):
-    """V_Delta of random matrices with an even model's relations in double-float:
-    below the instability (size 0.05) k_vertex_sym keeps every one, far above it
-    the indefinite ones go to the pivoted kernel.  The general form carries 1e-14 too;
-    the worst of some thousand random matrices has a condition number of about 1e5,
-    which leaves 1e-8 of the largest element."""
+    """V_Delta of random matrices with an even model's relations in double-float (the
+    pivoted real-basis kernel), far below the instability and far above it.  The
+    general form carries 1e-14 too; the worst of some thousand random matrices has a
+    condition number of about 1e5, which leaves 1e-8 of the largest element.
+    """
     m = model(*dims)
     No, Nk, n = m["Norb"], len(m["hamk"]), m["Norb"] ** 2
     rng = np.random.default_rng(No)
@@ -242,3 +242,17 @@ def test_pairing_vertex_of_any_matrix(F, dims, size, gap_sym):
     finally:
         F.set_precision(64)
     close(v, g, 1e-8, 0.0)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dims", [(3, 8, 8, 1, 30), (4, 4, 4, 1, 8), (5, 4, 6, 1, 10)])
+@pytest.mark.parametrize("factor", [0.5, 3.0, 6.0, 20.0])
+def test_fp64_vertex_beyond_the_instability(F, dims, factor):
+    """One FP64 iteration without the rescaling, at interactions below and above the
+    instability, where S^-1 - chi0 is indefinite and k_vertex_sym may leave matrices to
+    the pivoted kernel.  Condition numbers of 1e4 leave 1e-12; the bound is that of the
+    other FP64 tests."""
+    m = model(*dims)
+    m["S"], m["C"] = factor * m["S"], factor * m["C"]
+    run = lambda: F.mkself(*step_args(m), scf_loop=1, eps=0.0, pp=0.5, sw_rescale=False, sw_tail=True)[0]  # noqa: E731
+    close(run(), general(run))
