@@ -335,7 +335,7 @@ class HostPrefault {
   HostPrefault(const HostPrefault&) = delete;
   HostPrefault& operator=(const HostPrefault&) = delete;
   void join();
-  // whether a result of this size may be started on before its last stage
+  // whether a result of this size gains by it (prefault.cu)
   static bool early(size_t bytes) { return bytes <= (1u << 30); }
 
  private:

@@ -865,8 +865,7 @@ void run_mkself(const MkselfArgs& a, int prec) {
   std::unique_ptr<HostPrefault> pages;
   if (a.scf_loop <= 4 && HostPrefault::early(bytes)) pages.reset(new HostPrefault(a.sigmak, bytes));
   mkself_core(in, prm, sig.p, a.mu_out, nullptr, 0.0, 0.0, prec);
-  if (!pages) pages.reset(new HostPrefault(a.sigmak, bytes));
-  pages->join();
+  pages.reset();
   sig.download(a.sigmak, KE);
   sync();
 }
@@ -1293,7 +1292,6 @@ void run_lin_eliash(const LinEliashArgs& a) {
   }
   EliashParams prm{a.temp, a.eps, a.itemax, a.gap_sym, a.arnoldi_m};
   *a.lambda_out = eliash_core<R>(in, chi.p, G.p, init.p, prt.p, prm, D.p, a.clobber_chi ? a.chi : nullptr);
-  HostPrefault(a.delta, sizeof(double2) * KE).join();
   D.download(a.delta, KE);
   sync();
 }
@@ -1444,11 +1442,10 @@ void run_pipeline_impl(const PipelineArgs& a, int prec) {
   double stoner_v = 0;
   const size_t bytes = sizeof(double2) * KE;
   std::unique_ptr<HostPrefault> pages_s, pages_d;
-  auto prefault = [&]() {
+  if (HostPrefault::early(bytes)) {
     pages_s.reset(new HostPrefault(a.sigmak, bytes));
     pages_d.reset(new HostPrefault(a.delta, bytes));
-  };
-  if (HostPrefault::early(bytes)) prefault();
+  }
   {
     DBuf<cx<R>> chi(KC);
     TailRef tr{in.eig.p, in.uni.p, mu};
@@ -1462,9 +1459,8 @@ void run_pipeline_impl(const PipelineArgs& a, int prec) {
   }
   g_stats.iterations = iters;
   const double t_compute = t.stop();
-  if (!pages_s) prefault();
-  pages_s->join();
-  pages_d->join();
+  pages_s.reset();
+  pages_d.reset();
   t.start();
   sig.download(a.sigmak, KE);
   D.download(a.delta, KE);

@@ -6,10 +6,10 @@
 // with large results start a few threads here that make the pages
 // (MADV_POPULATE_WRITE, which leaves the contents as they are) while the solve
 // runs, and join them before the copy: one FLEX iteration of five orbitals,
-// 64x64x1024 (840 MB of Sigma) 83 -> 58 ms.  Large sets of pages that wait for their copy
-// take longer to copy into than none, the longer they wait (2 x 1.7 GB made a second
-// before the copy 200 to 660 ms, without 122): results above 1 GB, and those of a loop
-// of many iterations, are started at the solve's end.
+// 64x64x1024 (840 MB of Sigma) 83 -> 58 ms.  Large sets of pages that wait for their
+// copy take longer to copy into than none, the longer they wait (2 x 1.7 GB made a
+// second before the copy 200 to 660 ms, just before it 340 in all, without 122):
+// results above 1 GB, and those of loops of many iterations, are left to the copy.
 #include <sys/mman.h>
 #include <unistd.h>
 
