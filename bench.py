@@ -370,7 +370,15 @@ def cpu_reference_estimate(cfg, tail: bool, iters: int, applies: int):
 
 
 # ------------------------------------------------------------------ main
-def solve_traffic(Norb: int, Nk: int, Nkall: int, Nw: int, stats: dict, precision: str) -> float:
+def pair_classes(Norb: int) -> int:
+    """Classes of pair elements (l, m) ~ (m, l) ~ (Pl, Pm), P(a, b) = (b, a): the
+    transforms of an even model (175 at five orbitals)."""
+    pairs = [(a, b) for a in range(Norb) for b in range(Norb)]
+    return len({frozenset([(x, y), (y, x), (x[::-1], y[::-1]), (y[::-1], x[::-1])]) for x in pairs for y in pairs})
+
+
+def solve_traffic(Norb: int, Nk: int, Nkall: int, Nw: int, stats: dict, precision: str,
+                  half_mesh: int | None = None) -> float:
     """Algorithmic HBM bytes of one fine solve (the coarse warm start left
     out), with P = Nkall 2Nw, K = Nk Nw, Nchi = Norb^2 and an ideal 4-D FFT of
     two read-write sweeps:
@@ -378,13 +386,18 @@ def solve_traffic(Norb: int, Nk: int, Nkall: int, Nw: int, stats: dict, precisio
                                 + Bv 2 K Nchi^2
       per Eliashberg application  Be [8P Norb^2 + 2P Nchi^2 + 4K Norb^2]
     B, Bv and Be are the bytes of a complex chi0/Sigma, vertex and Eliashberg
-    element in each phase: 8 for FP32, 16 for FP64 and double-float."""
+    element in each phase: 8 for FP32, 16 for FP64 and double-float.  half_mesh:
+    the points of half the mesh, for an even model, whose arrays have half_mesh Nw
+    elements, Norb (Norb + 1) / 2 orbital elements and pair_classes pair elements."""
     nchi = Norb * Norb
     P, K = Nkall * 2 * Nw, Nk * Nw
+    n_el, n_fwd, n_pair = Norb ** 2, nchi * (nchi + 1) // 2, nchi ** 2
+    if half_mesh:
+        P, n_el, n_fwd, n_pair = half_mesh * Nw, Norb * (Norb + 1) // 2, pair_classes(Norb), pair_classes(Norb)
 
     def it_bytes(B, Bv):
-        return (B * (4 * P * (2 * Norb ** 2 + nchi * (nchi + 1) // 2 + nchi ** 2) + P * nchi ** 2
-                     + 16 * K * Norb ** 2) + Bv * 2 * K * nchi ** 2)
+        return (B * (4 * P * (2 * n_el + n_fwd + n_pair) + P * n_pair + 16 * K * Norb ** 2)
+                + Bv * 2 * K * n_pair)
 
     n = int(stats["iterations"])
     if precision == "mixed":
@@ -395,7 +408,7 @@ def solve_traffic(Norb: int, Nk: int, Nkall: int, Nw: int, stats: dict, precisio
         flex, be = n * it_bytes(8, 8), 8
     else:
         flex, be = n * it_bytes(16, 16), 16
-    return float(flex + int(stats["applies"]) * be * (8 * P * Norb ** 2 + 2 * P * nchi ** 2 + 4 * K * Norb ** 2))
+    return float(flex + int(stats["applies"]) * be * (8 * P * n_el + 2 * P * n_pair + 4 * K * Norb ** 2))
 
 
 def max_over_ranks(values, dist):
@@ -518,7 +531,12 @@ def main():
                                         m["uni"], m["init"], m["plist"]))
     out_bytes = res["sigmak"].nbytes + res["gap"].nbytes
     iters, applies = int(stats["iterations"]), int(stats["applies"])
-    solve_bytes = solve_traffic(c["Norb"], len(m["klist"]), len(m["kmap"]), c["Nw"], stats, a.precision)
+    # the library takes the even form for a symmetric H(k)
+    even = (abs(m["hamk"] - m["hamk"].transpose(0, 2, 1)).max() <= 1e-13 * abs(m["hamk"]).max()
+            and os.environ.get("PYRPA_GB_EVEN") != "0")
+    axis = c["Nz"] if c["Nz"] > 1 else c["Ny"]
+    half = len(m["kmap"]) // axis * (axis // 2 + 1) if even else None
+    solve_bytes = solve_traffic(c["Norb"], len(m["klist"]), len(m["kmap"]), c["Nw"], stats, a.precision, half)
     solve_s = value - stats["t_warm_ms"] / 1e3
     ritz = [float(x) for x in F.last_ritz(4)]
     fp64 = None if a.no_fp64 else plain_fp64_comparison(F, solve_args=(m, call), res=res)
