@@ -67,6 +67,7 @@ struct RealBasis {
 
 // index tables of the real basis: its matrix from the class representatives (vin) and back (vout)
 void build_index(Even& ev, int n, const std::vector<RealBasis>& basis, const std::vector<int>* idx) {
+  PGB_CHECK(2 * ev.cls.size() <= (size_t)kSrcMask + 1, "more pair classes than the real-basis tables can address");
   auto src = [&](int row, int col, int part, int* sign) {  // part of element (row, col) of the vertex matrix
     const int x = row + n * col;
     *sign = (part && ev.cj_of[x]) ? -1 : 1;
@@ -92,7 +93,7 @@ void build_index(Even& ev, int n, const std::vector<RealBasis>& basis, const std
         b = src(l, pm, im, &s);
         cb *= s;
       }
-      ev.vin[(size_t)q * n + p] = a | b << 9 | (ca + 2) << 18 | (cb + 2) << 21;
+      ev.vin[(size_t)q * n + p] = a | b << kSrcBits | (ca + 2) << 2 * kSrcBits | (cb + 2) << (2 * kSrcBits + 3);
     }
   ev.vout.clear();
   for (const EvenClass& c : ev.cls) {
@@ -140,9 +141,9 @@ void build_sym(Even& ev, int n, const std::vector<RealBasis>& basis) {
   for (int d = 0; d <= n / 2; ++d)
     for (int p = 0; p < n; ++p) {
       const int q = (p + d) % n, w = ev.vin[(size_t)q * n + p];
-      const int ca = (((w >> 18) & 7) - 2) * (int)ev.hsc[q], cb = (((w >> 21) & 7) - 2) * (int)ev.hsc[q];
-      ev.sin.push_back((w & 511) | ((w >> 9) & 511) << 9 | (ca < 0) << 18 | (cb < 0) << 19 | (cb != 0) << 20 |
-                       (std::abs(ca) == 2) << 21);
+      const int ca = src_ca(w) * (int)ev.hsc[q], cb = src_cb(w) * (int)ev.hsc[q];
+      ev.sin.push_back(src_a(w) | src_b(w) << kSrcBits |
+                       ((ca < 0) | (cb < 0) << 1 | (cb != 0) << 2 | (std::abs(ca) == 2) << 3) << 2 * kSrcBits);
     }
   ev.sout.clear();
   for (int w : ev.vout) {

@@ -46,6 +46,17 @@ struct EvenClass {
   int mem[4], cj[4];
 };
 
+// A word of vin names its two sources 2 class + part in kSrcBits each, then their
+// coefficients ca + 2 and cb + 2 in three bits each; a word of sin has four flags after
+// the sources (k_vertex_sym).  Two four-orbital sites, the most pairs (32) of the
+// engine, have 288 classes: sources up to 575.
+constexpr int kSrcBits = 10, kSrcMask = (1 << kSrcBits) - 1;
+__host__ __device__ constexpr int src_a(int w) { return w & kSrcMask; }
+__host__ __device__ constexpr int src_b(int w) { return w >> kSrcBits & kSrcMask; }
+__host__ __device__ constexpr int src_ca(int w) { return (w >> 2 * kSrcBits & 7) - 2; }
+__host__ __device__ constexpr int src_cb(int w) { return (w >> (2 * kSrcBits + 3) & 7) - 2; }
+__host__ __device__ constexpr bool src_flag(int w, int i) { return w >> (2 * kSrcBits + i) & 1; }
+
 struct EvenPair {
   int f13, f42;  // a <= b copies of G13 and G42
   int a13, b13, a42, b42;  // their orbitals

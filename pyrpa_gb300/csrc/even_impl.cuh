@@ -490,7 +490,7 @@ __global__ void k_even_const(double* c0, const R* stat, const cx<R>* F, const Ev
 // ------------------------------------------------------------------- vertex
 // Real-basis index tables.  vin, entry (row p, column q) at q N + p:
 // value = ca t[a] + cb t[b] with t[2 c + part] the parts of class c's matrix
-// element; word = a | b << 9 | (ca + 2) << 18 | (cb + 2) << 21.  vout, per class two
+// element; word: see even.cuh.  vout, per class two
 // words (real, imaginary part): value = cf (sa v[a] + sb v[b]) over the result
 // v[q N + p]; word = a | b << 10 | (sa + 1) << 20 | (sb + 1) << 22 | (cf = 1/2) << 24.
 __device__ __forceinline__ float real_mag(float a) { return fabsf(a); }
@@ -654,8 +654,7 @@ __global__ void __launch_bounds__(32 * W, sizeof(R) == 4 ? 4 : 2)
     // the two sources as offsets into the tile, with the signs in bit 31 and
     // "twice" in bit 30 of the first, "absent" in bit 30 of the second
     const int word = tb.vin[e];
-    const int ia = word & 511, ib = (word >> 9) & 511;
-    const int ca = ((word >> 18) & 7) - 2, cb = ((word >> 21) & 7) - 2;
+    const int ia = src_a(word), ib = src_b(word), ca = src_ca(word), cb = src_cb(word);
     const unsigned oa = (unsigned)((ia >> 1) * TP * 2 + (ia & 1)), ob = (unsigned)((ib >> 1) * TP * 2 + (ib & 1));
     vin[e] = make_int2((int)(oa | (ca < 0 ? 1u << 31 : 0u) | (ca == 2 || ca == -2 ? 1u << 30 : 0u)),
                        (int)(ob | (cb < 0 ? 1u << 31 : 0u) | (cb == 0 ? 1u << 30 : 0u)));
@@ -909,14 +908,14 @@ __global__ void __launch_bounds__(32 * W, N == 9 ? 2 : 1)
   // entry e of the symmetric form of X, of matrix tt of the staged half
   auto entry = [&](int e, int tt) {
     const R* tr = reinterpret_cast<const R*>(tile) + 2 * tt;
-    const int word = sin[e], ia = word & 511, ib = (word >> 9) & 511;
+    const int word = sin[e], ia = src_a(word), ib = src_b(word);
     R v = tr[2 * (ia >> 1) * TP + (ia & 1)];
-    if (word >> 18 & 1) v = -v;
-    if (word >> 20 & 1) {
+    if (src_flag(word, 0)) v = -v;
+    if (src_flag(word, 2)) {
       const R u = tr[2 * (ib >> 1) * TP + (ib & 1)];
-      v = v + ((word >> 19 & 1) ? -u : u);
+      v = v + (src_flag(word, 1) ? -u : u);
     }
-    if (word >> 21 & 1) v = v + v;
+    if (src_flag(word, 3)) v = v + v;
     return v;
   };
   for (long long m0 = (long long)blockIdx.x * T; m0 < nmat; m0 += (long long)gridDim.x * T) {
@@ -1251,9 +1250,9 @@ __global__ void __launch_bounds__(32 * kEvenStonerWarps) k_stoner_even(double* o
   if (lane < m) {
     for (int q = 0; q < m; ++q) {
       const int word = vin[(i0 + q) * n + i0 + lane];
-      const int ca = ((word >> 18) & 7) - 2, cb = ((word >> 21) & 7) - 2;
-      double x = ca * part(word & 511);
-      if (cb) x += cb * part((word >> 9) & 511);
+      const int ca = src_ca(word), cb = src_cb(word);
+      double x = ca * part(src_a(word));
+      if (cb) x += cb * part(src_b(word));
       const bool a = i0 + lane < nself, b = i0 + q < nself;
       if (a != b) x *= a ? 1.4142135623730951 : 0.70710678118654752;
       A[lane * ld + q] = x;
