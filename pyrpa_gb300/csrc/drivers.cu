@@ -858,7 +858,9 @@ void run_mkself(const MkselfArgs& a, int prec) {
                 a.hamk, a.eig, a.uni);
   FlexParams prm{a.mu_init, a.fill, a.temp, a.scf_loop, a.pp, a.eps, a.sub_sigma, a.sw_out, a.sw_in, a.m_diis,
                  a.sw_rescale, a.sw_tail, a.sigma_scale};
-  detect_even(in, a.Smat, a.Cmat, a.hamk, a.eig, a.uni, prec == 32 ? 8 : 16);
+  // a stage that the FP32 loop leaves in FP64 needs planes of 16-byte elements
+  const bool narrow = prec == 32 && (fp32_stage_mask() & 5) == 5;
+  detect_even(in, a.Smat, a.Cmat, a.hamk, a.eig, a.uni, narrow ? 8 : 16);
   const long long KE = in.g.K * a.Norb * a.Norb;
   DBuf<double2> sig(KE);
   const size_t bytes = sizeof(double2) * KE;
