@@ -326,8 +326,8 @@ void ensure_context();
 constexpr int kErrSlots = 64;
 int* err_slot_address(int slot);
 
-// Makes the pages of a result array in the background (prefault.cu); joined
-// before the copy into it, and at the end of the scope.
+// Makes the pages of a result array in the background where its size gains by it
+// (prefault.cu); joined before the copy into it, and at the end of the scope.
 class HostPrefault {
  public:
   HostPrefault(void* p, size_t bytes);
@@ -335,8 +335,6 @@ class HostPrefault {
   HostPrefault(const HostPrefault&) = delete;
   HostPrefault& operator=(const HostPrefault&) = delete;
   void join();
-  // whether a result of this size gains by it (prefault.cu)
-  static bool early(size_t bytes) { return bytes <= (1u << 30); }
 
  private:
   std::vector<std::thread> threads_;

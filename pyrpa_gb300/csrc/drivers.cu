@@ -865,7 +865,7 @@ void run_mkself(const MkselfArgs& a, int prec) {
   DBuf<double2> sig(KE);
   const size_t bytes = sizeof(double2) * KE;
   std::unique_ptr<HostPrefault> pages;
-  if (a.scf_loop <= 4 && HostPrefault::early(bytes)) pages.reset(new HostPrefault(a.sigmak, bytes));
+  if (a.scf_loop <= 4) pages.reset(new HostPrefault(a.sigmak, bytes));
   mkself_core(in, prm, sig.p, a.mu_out, nullptr, 0.0, 0.0, prec);
   pages.reset();
   sig.download(a.sigmak, KE);
@@ -1443,11 +1443,7 @@ void run_pipeline_impl(const PipelineArgs& a, int prec) {
   PGB_CHECK(dyson(G.p, sig.p, in.H.p, mu, a.temp, in.Nk, in.Nw, in.Norb), "singular G^-1 in the Dyson step");
   double stoner_v = 0;
   const size_t bytes = sizeof(double2) * KE;
-  std::unique_ptr<HostPrefault> pages_s, pages_d;
-  if (HostPrefault::early(bytes)) {
-    pages_s.reset(new HostPrefault(a.sigmak, bytes));
-    pages_d.reset(new HostPrefault(a.delta, bytes));
-  }
+  HostPrefault pages_s(a.sigmak, bytes), pages_d(a.delta, bytes);
   {
     DBuf<cx<R>> chi(KC);
     TailRef tr{in.eig.p, in.uni.p, mu};
@@ -1461,8 +1457,8 @@ void run_pipeline_impl(const PipelineArgs& a, int prec) {
   }
   g_stats.iterations = iters;
   const double t_compute = t.stop();
-  pages_s.reset();
-  pages_d.reset();
+  pages_s.join();
+  pages_d.join();
   t.start();
   sig.download(a.sigmak, KE);
   D.download(a.delta, KE);

@@ -6,10 +6,14 @@
 // with large results start a few threads here that make the pages
 // (MADV_POPULATE_WRITE, which leaves the contents as they are) while the solve
 // runs, and join them before the copy: one FLEX iteration of five orbitals,
-// 64x64x1024 (840 MB of Sigma) 83 -> 58 ms.  Large sets of pages that wait for their
-// copy take longer to copy into than none, the longer they wait (2 x 1.7 GB made a
-// second before the copy 200 to 660 ms, just before it 340 in all, without 122):
-// results above 1 GB, and those of loops of many iterations, are left to the copy.
+// 64x64x1024 (840 MB of Sigma) 83 -> 58 ms; a tail-corrected FP64 chi0 of 649 MB
+// 53 -> 32 ms, of 1013 MB 83 -> 50.  Above 1 GB the time varies from call to call
+// and can be far longer than the copy's own faults: the same chi0 of 1297 MB 62 to
+// 278 ms against 104 without, of 1622 MB 78 to 383 against 131, of 5.2 GB 464 to 2135
+// against 460.  Large sets of pages that wait for their copy also take longer to copy
+// into, the longer they wait (2 x 1.7 GB made a second before the copy 200 to 660 ms,
+// without 122).  So every result above 1 GB is left to the copy, and so are those of
+// loops of many iterations (drivers.cu).
 #include <sys/mman.h>
 #include <unistd.h>
 
@@ -27,13 +31,14 @@ namespace pgb {
 
 namespace {
 constexpr size_t kPrefaultMin = 32u << 20;  // 36 MB 8.9 -> 8.4 ms a call, 28 MB 2.00 -> 2.05
+constexpr size_t kPrefaultMax = 1u << 30;   // the whole of the result
 constexpr size_t kPerThread = 64u << 20;
 constexpr size_t kMaxThreads = 4;
 constexpr size_t kPiece = 1u << 20;
 }  // namespace
 
 HostPrefault::HostPrefault(void* p, size_t bytes) {
-  if (!p || bytes < kPrefaultMin) return;
+  if (!p || bytes < kPrefaultMin || bytes > kPrefaultMax) return;
   const size_t page = (size_t)sysconf(_SC_PAGESIZE);
   const uintptr_t a = ((uintptr_t)p + page - 1) / page * page, b = ((uintptr_t)p + bytes) / page * page;
   if (b <= a) return;
