@@ -19,7 +19,7 @@
 
 #include <algorithm>
 #include <cstdint>
-#include <system_error>
+#include <exception>
 
 #include "common.cuh"
 
@@ -55,8 +55,9 @@ HostPrefault::HostPrefault(void* p, size_t bytes) {
         for (uintptr_t x = s; x < e; x += piece)
           if (madvise(reinterpret_cast<void*>(x), std::min<size_t>(piece, e - x), MADV_POPULATE_WRITE) != 0) return;
       });
-  } catch (const std::system_error&) {
-    // no thread to be had: the copy takes the faults
+  } catch (const std::exception&) {
+    // no thread or no memory for one: the copy takes the faults (an exception that left
+    // the constructor would end the process at the threads already running)
   }
 }
 

@@ -53,3 +53,41 @@ def test_sizes_that_get_their_pages(tmp_path):
         pytest.skip("no MADV_POPULATE_WRITE in this kernel")
     assert have[64] == 64
     assert have[1024 + 64] == 0
+
+
+NO_MEMORY = r'''
+#include <sys/mman.h>
+#include <cstdio>
+#include <cstdlib>
+#include <new>
+#include "common.cuh"
+static thread_local int left = -1;  // allocations of the calling thread until one fails; -1: none fails
+void* operator new(size_t n) {
+  if (left >= 0 && left-- == 0) throw std::bad_alloc();
+  void* p = std::malloc(n);
+  if (!p) throw std::bad_alloc();
+  return p;
+}
+void operator delete(void* p) noexcept { std::free(p); }
+void operator delete(void* p, size_t) noexcept { std::free(p); }
+int main() {
+  const size_t n = 256u << 20;
+  void* p = mmap(nullptr, n, PROT_READ | PROT_WRITE, MAP_PRIVATE | MAP_ANONYMOUS | MAP_NORESERVE, -1, 0);
+  if (p == MAP_FAILED) return 1;
+  for (int k = 0; k < 16; ++k) {
+    left = k;
+    pgb::HostPrefault pages(p, n);
+    left = -1;
+    pages.join();
+  }
+  std::puts("done");
+  return 0;
+}
+'''
+
+
+def test_failed_allocations_leave_the_pages_to_the_copy(tmp_path):
+    """Every allocation of the constructor fails once, also after threads have started."""
+    exe = compile_host(tmp_path, NO_MEMORY, "no_memory")
+    r = subprocess.run([str(exe)], capture_output=True, text=True)
+    assert r.returncode == 0 and r.stdout == "done\n", r.stderr
