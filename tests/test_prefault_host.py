@@ -32,15 +32,20 @@ int main(int, char** argv) {
 '''
 
 
-def compile_host(tmp_path, source, name):
+def compile_host(tmp_path, source, name, plain=None):
+    """source: a .cu file; plain: a C++ file beside it"""
     nvcc = shutil.which("nvcc") or "/usr/local/cuda/bin/nvcc"
     if not Path(nvcc).exists():
         pytest.skip("nvcc not found")
     csrc = ROOT / "pyrpa_gb300" / "csrc"
     (tmp_path / f"{name}.cu").write_text(source)
     exe = tmp_path / name
-    subprocess.run([nvcc, "-std=c++17", "-O2", "-I", str(csrc), str(tmp_path / f"{name}.cu"), str(csrc / "prefault.cu"),
-                    "-o", str(exe)], check=True, capture_output=True, text=True)
+    files = [tmp_path / f"{name}.cu", csrc / "prefault.cu"]
+    if plain:
+        files.append(tmp_path / f"{name}_plain.cpp")
+        files[-1].write_text(plain)
+    subprocess.run([nvcc, "-std=c++17", "-O2", "-I", str(csrc), *map(str, files), "-o", str(exe)], check=True,
+                   capture_output=True, text=True)
     return exe
 
 
@@ -55,13 +60,10 @@ def test_sizes_that_get_their_pages(tmp_path):
     assert have[1024 + 64] == 0
 
 
-NO_MEMORY = r'''
-#include <sys/mman.h>
-#include <cstdio>
+ALLOC = r'''
 #include <cstdlib>
 #include <new>
-#include "common.cuh"
-static thread_local int left = -1;  // allocations of the calling thread until one fails; -1: none fails
+thread_local int left = -1;  // allocations of the calling thread until one fails; -1: none fails
 void* operator new(size_t n) {
   if (left >= 0 && left-- == 0) throw std::bad_alloc();
   void* p = std::malloc(n);
@@ -70,6 +72,12 @@ void* operator new(size_t n) {
 }
 void operator delete(void* p) noexcept { std::free(p); }
 void operator delete(void* p, size_t) noexcept { std::free(p); }
+'''
+NO_MEMORY = r'''
+#include <sys/mman.h>
+#include <cstdio>
+#include "common.cuh"
+extern thread_local int left;
 int main() {
   const size_t n = 256u << 20;
   void* p = mmap(nullptr, n, PROT_READ | PROT_WRITE, MAP_PRIVATE | MAP_ANONYMOUS | MAP_NORESERVE, -1, 0);
@@ -88,6 +96,6 @@ int main() {
 
 def test_failed_allocations_leave_the_pages_to_the_copy(tmp_path):
     """Every allocation of the constructor fails once, also after threads have started."""
-    exe = compile_host(tmp_path, NO_MEMORY, "no_memory")
+    exe = compile_host(tmp_path, NO_MEMORY, "no_memory", ALLOC)
     r = subprocess.run([str(exe)], capture_output=True, text=True)
     assert r.returncode == 0 and r.stdout == "done\n", r.stderr
