@@ -1005,7 +1005,8 @@ template <> constexpr float kEpsOf<float> = 1.1920929e-7f;
 // type, float for an FP32 chi0 in the fast schedule (stoner() decides)
 template <typename R, typename T>
 __global__ void __launch_bounds__(32 * kStonerWarps) k_stoner(double* out, const cx<R>* chi, const double* S,
-                                                              const double* C, int Nk, int Nw, int n, int* err) {
+                                                              const double* C, int Nk, int Nw, int n, int t0,
+                                                              int* err) {
   using cT = cx<T>;
   extern __shared__ __align__(16) unsigned char sm_st[];
   const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -1013,7 +1014,7 @@ __global__ void __launch_bounds__(32 * kStonerWarps) k_stoner(double* out, const
   cT* A = reinterpret_cast<cT*>(sm_st) + (size_t)w * (n * ld + 64);
   cT* v = A + n * ld;   // Householder vector / rotation sines
   T* cs = reinterpret_cast<T*>(v + 32);
-  const int t = blockIdx.x * kStonerWarps + w;
+  const int t = t0 + blockIdx.x * kStonerWarps + w;
   if (t >= 2 * Nk) return;  // warp-uniform
   const int k0 = t % Nk, which = t / Nk;
   const double* V = which ? C : S;
@@ -1135,15 +1136,17 @@ __global__ void __launch_bounds__(32 * kStonerWarps) k_stoner(double* out, const
   }
 }
 
-// false if the QR of some matrix did not converge
+// false if the QR of some matrix did not converge; charge: the second half of h alone
 template <typename R, typename T>
-bool stoner_launch(const Geom& g, const cx<R>* chi, const double* S, const double* C, std::vector<double>& h) {
+bool stoner_launch(const Geom& g, const cx<R>* chi, const double* S, const double* C, std::vector<double>& h,
+                   bool charge = false) {
   reset_err();
   DBuf<double> out(2 * (size_t)g.Nk);
   const size_t smem = (size_t)kStonerWarps * ((size_t)g.Nchi * (g.Nchi + 1) + 64) * sizeof(cx<T>);
   PGB_SMEM_LIMIT_ONCE((k_stoner<R, T>), 96 * 1024);
-  const unsigned blocks = (unsigned)((2LL * g.Nk + kStonerWarps - 1) / kStonerWarps);
-  k_stoner<R, T><<<blocks, 32 * kStonerWarps, smem, ctx().stream>>>(out.p, chi, S, C, g.Nk, g.Nw, g.Nchi,
+  const int t0 = charge ? g.Nk : 0;
+  const unsigned blocks = (unsigned)((2LL * g.Nk - t0 + kStonerWarps - 1) / kStonerWarps);
+  k_stoner<R, T><<<blocks, 32 * kStonerWarps, smem, ctx().stream>>>(out.p, chi, S, C, g.Nk, g.Nw, g.Nchi, t0,
                                                                      ctx().err);
   count_launch("stoner");
   h.resize(2 * (size_t)g.Nk);
@@ -1159,32 +1162,33 @@ template <typename R>
 void stoner(const Geom& g, const cx<R>* chi, const double* S, const double* C, double* sdw, double* cdw,
             int* q_sdw, int* q_cdw) {
   std::vector<double> h;
-  // even models: a symmetric problem for chi0 S; the charge factor is only
-  // printed, so it is computed (below, with the other) when something prints
-  if (g.even && g.even->stoner_ok && !ctx().verbose) {
-    PGB_CHECK(stoner_even<R>(g, chi, h), "eigenvalue iteration of chi0(q,0)S did not converge");
-    const auto m = std::max_element(h.begin(), h.end());
-    *sdw = std::max(-1.0e5, *m);
-    *cdw = -1.0e5;
-    if (q_sdw) *q_sdw = (int)(m - h.begin());
-    if (q_cdw) *q_cdw = 0;
-    return;
-  }
-  bool done = false;
-  if constexpr (std::is_same<R, float>::value) {
-    if (stoner_launch<R, float>(g, chi, S, C, h)) {
-      double s32 = -1.0e5;
-      for (int k = 0; k < g.Nk; ++k) s32 = std::max(s32, h[k]);
-      done = std::fabs(s32 - 1.0) >= 1.0e-3;
-    }
-  }
-  if (!done)
-    PGB_CHECK((stoner_launch<R, double>(g, chi, S, C, h)), "eigenvalue iteration of chi0(q,0)S did not converge");
+  // even models: a symmetric problem for chi0 S, with printing on or off (the factor
+  // decides on the rescaling, and must not depend on it); the charge factor is only
+  // printed, and computed where something prints
+  const bool even = g.even && g.even->stoner_ok;
   double s2 = -1.0e5, c2 = -1.0e5;
   int qs = 0, qc = 0;
-  for (int k = 0; k < g.Nk; ++k) {
-    if (h[k] > s2) { s2 = h[k]; qs = k; }
-    if (h[g.Nk + k] > c2) { c2 = h[g.Nk + k]; qc = k; }
+  if (even) {
+    PGB_CHECK(stoner_even<R>(g, chi, h), "eigenvalue iteration of chi0(q,0)S did not converge");
+    for (int k = 0; k < g.Nk; ++k)
+      if (h[k] > s2) { s2 = h[k]; qs = k; }
+  }
+  if (!even || ctx().verbose) {
+    bool done = false;
+    if constexpr (std::is_same<R, float>::value) {
+      if (stoner_launch<R, float>(g, chi, S, C, h, even)) {
+        double s32 = s2;
+        for (int k = 0; !even && k < g.Nk; ++k) s32 = std::max(s32, h[k]);
+        done = std::fabs(s32 - 1.0) >= 1.0e-3;
+      }
+    }
+    if (!done)
+      PGB_CHECK((stoner_launch<R, double>(g, chi, S, C, h, even)),
+                "eigenvalue iteration of chi0(q,0)S did not converge");
+    for (int k = 0; k < g.Nk; ++k) {
+      if (!even && h[k] > s2) { s2 = h[k]; qs = k; }
+      if (h[g.Nk + k] > c2) { c2 = h[g.Nk + k]; qc = k; }
+    }
   }
   *sdw = s2;
   *cdw = c2;

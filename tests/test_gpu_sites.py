@@ -98,3 +98,25 @@ def test_stoner_factor_in_other_arithmetics(F, prof, Nx, Ny, Nw, bits, tol):
     finally:
         F.set_precision(64)
     assert abs(F.last_stats()["stoner"] - 0.7) <= tol
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("prof,Nx,Ny,Nw", SITES + [((5,), 8, 8, 8)])
+@pytest.mark.parametrize("bits", [64, 32])
+def test_results_do_not_depend_on_printing(F, prof, Nx, Ny, Nw, bits):
+    """The factor of a chi0 beyond the instability scales chi0, so that another rounding of
+    it would reach Sigma: the same bits with printing on and off."""
+    m = model(F, prof, Nx, Ny, Nw, 1.2)
+    out = []
+    for verbose in (0, 1):
+        F.set_precision(bits)
+        F.set_verbose(verbose)
+        try:
+            st = F.get_chi0(m["S"], m["C"], m["G"], m["olist"], m["kmap"], m["invk"], m["temp"], *m["mesh"])[1]
+            sg, mu = F.mkself(*m["step"], scf_loop=1, eps=0.0, pp=0.5, sw_rescale=True)
+        finally:
+            F.set_verbose(0)
+            F.set_precision(64)
+        out.append((st, F.last_stats()["stoner"], mu, sg))
+    for a, b in zip(*out):
+        assert np.array_equal(a, b)
