@@ -26,6 +26,7 @@
 // one orbital 32x32x1024 2.6 -> 0.8 ms; five orbitals 64x64x1024 26 -> 5.5 ms (9.8
 // with a Householder reduction).
 #include <algorithm>
+#include <cstdlib>
 
 #include "flex.cuh"
 #include "flex_dev.cuh"
@@ -149,11 +150,21 @@ __device__ double im_digamma(double a, double y) {
 
 constexpr int kMuThreads = 256;
 constexpr long long kMuWaitCycles = 4000000000LL;  // about 2 s
+constexpr int kMuAttempts = 40;
+
+// Cycles of a wait between the blocks in the first attempt (PYRPA_GB_MU_WAIT; a
+// search whose blocks gave up starts again with eight times as many)
+long long mu_wait_cycles() {
+  const char* s = std::getenv("PYRPA_GB_MU_WAIT");
+  return s ? std::min(kMuWaitCycles, std::max(1LL, std::atoll(s))) : kMuWaitCycles;
+}
 
 // Sum over the grid of v, the same in every thread.  Blocks meet at a counter
 // that only grows; every wait is bounded, and a block that gives up tells the
-// caller through `dead`.  The launch is cooperative, so all blocks are resident.
-__device__ double grid_sum(double v, double* part, unsigned* bar, unsigned round, bool& dead) {
+// caller through `dead`.  The launch is cooperative, so all blocks are resident
+// at once, but another thread's kernel may hold some SMs for longer than a wait
+// (the vertex of a large FP64 model runs for seconds): mu_search then starts again.
+__device__ double grid_sum(double v, double* part, unsigned* bar, unsigned round, long long wait, bool& dead) {
   __shared__ double red[kMuThreads / 32];
   __shared__ double total;
   __shared__ int gave_up;
@@ -177,7 +188,7 @@ __device__ double grid_sum(double v, double* part, unsigned* bar, unsigned round
     const unsigned want = (round + 1) * gridDim.x;
     const long long t0 = clock64();
     while (*(volatile unsigned*)bar < want)
-      if (clock64() - t0 > kMuWaitCycles) {
+      if (clock64() - t0 > wait) {
         gave_up = 1;
         break;
       }
@@ -200,7 +211,7 @@ __device__ double grid_sum(double v, double* part, unsigned* bar, unsigned round
 template <int N>
 __global__ void __launch_bounds__(kMuThreads) k_mu_search(MuState* io, const double2* cp, double center,
                                                           const double* eig, double fill, double esterr, double temp,
-                                                          int Nk, int Nw, double* part, unsigned* bar) {
+                                                          int Nk, int Nw, double* part, unsigned* bar, long long wait) {
   const long long K = (long long)Nk * Nw, S = (long long)gridDim.x * blockDim.x;
   const long long first = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   MuState st = *io;
@@ -245,7 +256,7 @@ __global__ void __launch_bounds__(kMuThreads) k_mu_search(MuState* io, const dou
         }
       acc += num[0] / den[0];
     }
-    const double s = grid_sum(fma(2.0 * temp, acc, tail / kPi), part, bar, round, dead);
+    const double s = grid_sum(fma(2.0 * temp, acc, tail / kPi), part, bar, round, wait, dead);
     ++round;
     return 0.5 * N + s / Nk;
   };
@@ -337,19 +348,23 @@ __global__ void __launch_bounds__(kMuThreads) k_mu_search(MuState* io, const dou
     mu = (rnL == rnS) ? (muS + muL) * 0.5 : (muS * rnL - muL * rnS) / (rnL - rnS);
     rnM = get_rn(mu);
   }
-  if (dead) err = 3;
-  if (threadIdx.x == 0 && (blockIdx.x == 0 || dead)) {
-    st.mu = st.mu_old = mu;
-    st.filling = rnM;
-    st.err = err;
-    *io = st;
+  // any block that gave up: the host starts again from the same state
+  if (threadIdx.x == 0 && dead) atomicMax(&io->err, 3);
+  if (threadIdx.x == 0 && blockIdx.x == 0 && !dead) {
+    io->mu = io->mu_old = mu;
+    io->muS = st.muS;
+    io->muL = st.muL;
+    io->bracket_valid = st.bracket_valid;
+    io->cached = st.cached;
+    io->filling = rnM;
+    atomicMax(&io->err, err);
   }
 }
 
 template <int N>
 void mu_launch(MuState* io, const double2* cp, double center, const double* eig, double fill, double esterr, double temp,
-               int Nk, int Nw, double* part, unsigned* bar, unsigned blocks, unsigned threads) {
-  void* args[] = {&io, &cp, &center, &eig, &fill, &esterr, &temp, &Nk, &Nw, &part, &bar};
+               int Nk, int Nw, double* part, unsigned* bar, long long wait, unsigned blocks, unsigned threads) {
+  void* args[] = {&io, &cp, &center, &eig, &fill, &esterr, &temp, &Nk, &Nw, &part, &bar, &wait};
   PGB_CUDA(cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(&k_mu_search<N>), dim3(blocks), dim3(threads),
                                        args, 0, ctx().stream));
 }
@@ -385,17 +400,24 @@ void mu_search(MuState& s, const double2* cp, double center, const double* eig, 
   DBuf<MuState> io(1);
   DBuf<double> part(2 * blocks);
   DBuf<unsigned> bar(1);
-  bar.zero();
-  io.upload(&s, 1);
-  switch (Norb) {
-#define PGB_MU(n_) case n_: mu_launch<n_>(io.p, cp, center, eig, fill, esterr, temp, Nk, Nw, part.p, bar.p, blocks, threads); break;
-    PGB_MU(1) PGB_MU(2) PGB_MU(3) PGB_MU(4) PGB_MU(5) PGB_MU(6) PGB_MU(7) PGB_MU(8)
+  const MuState start = s;
+  long long wait = mu_wait_cycles();
+  for (int attempt = 1;; ++attempt) {
+    s = start;
+    bar.zero();
+    io.upload(&s, 1);
+    switch (Norb) {
+#define PGB_MU(n_) case n_: mu_launch<n_>(io.p, cp, center, eig, fill, esterr, temp, Nk, Nw, part.p, bar.p, wait, blocks, threads); break;
+      PGB_MU(1) PGB_MU(2) PGB_MU(3) PGB_MU(4) PGB_MU(5) PGB_MU(6) PGB_MU(7) PGB_MU(8)
 #undef PGB_MU
-    default: throw Error("Norb above the engine limit of 8 orbitals");
+      default: throw Error("Norb above the engine limit of 8 orbitals");
+    }
+    count_launch("mu_search");
+    io.download(&s, 1);
+    sync();
+    if (s.err != 3 || attempt == kMuAttempts) break;
+    wait = std::min(kMuWaitCycles, 8 * wait);
   }
-  count_launch("mu_search");
-  io.download(&s, 1);
-  sync();
   PGB_CHECK(s.err != 1, "Too many");
   PGB_CHECK(s.err != 2, "Too many loop!");
   PGB_CHECK(s.err == 0, "the chemical-potential search gave up a wait between its blocks");
