@@ -1118,8 +1118,9 @@ __global__ void __launch_bounds__(32 * W, N == 9 ? 2 : 1)
 // their elimination of S^-1 -+ X then undoes these roundings.  The rounding of an exact
 // C^-1 does not cancel like that; C^-1's same-orbital block has entries of 30 times its
 // smallest eigenvalue, and the error is the same in every matrix, so that it adds up in
-// Sigma.
-template <typename R> std::vector<R> inverse_as(const std::vector<double>& X, int n) {
+// Sigma.  A matrix that is singular in this arithmetic though not in FP64 (C of J within
+// 1e-8 of U / 5, in FP32) takes `fp64`, its FP64 inverse, rounded.
+template <typename R> std::vector<R> inverse_as(const std::vector<double>& X, const std::vector<double>& fp64, int n) {
   std::vector<R> A((size_t)n * n);
   for (size_t e = 0; e < A.size(); ++e) A[e] = (R)X[e];
   std::vector<int> piv(n);
@@ -1143,6 +1144,10 @@ template <typename R> std::vector<R> inverse_as(const std::vector<double>& X, in
   for (int k = n - 1; k >= 0; --k)
     if (piv[k] != k)
       for (int r = 0; r < n; ++r) std::swap(A[r * n + k], A[r * n + piv[k]]);
+  bool finite = true;
+  for (const R& v : A) finite = finite && std::isfinite((double)v);
+  if (!finite)
+    for (size_t e = 0; e < A.size(); ++e) A[e] = (R)fp64[e];
   return A;
 }
 
@@ -1565,8 +1570,8 @@ bool vertex_even(const Even& ev, cx<R>* chi, long long nmat, long long estride, 
   PGB_CHECK(host_inverse(Si, n) && host_inverse(Ci, n), "singular interaction matrix in the real-basis vertex");
   std::vector<R> Sr(Si.size(), (R)0), Cr(Sr);
   if (n > 1) {
-    Sr = inverse_as<R>(ev.Sb, n);
-    Cr = inverse_as<R>(ev.Cb, n);
+    Sr = inverse_as<R>(ev.Sb, Si, n);
+    Cr = inverse_as<R>(ev.Cb, Ci, n);
   } else {
     Sr[0] = (R)Si[0];
     Cr[0] = (R)Ci[0];
