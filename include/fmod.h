@@ -183,6 +183,9 @@ void pyrpa_gb_clear_error(void);
  * context unless pyrpa_gb_set_thread_stream gave it one; all engine kernels,
  * FFT passes included) */
 void pyrpa_gb_kernel_launches(int64_t* n);
+/* vertex matrices of FP64 even models that the swept inverse of the symmetric form
+ * left to the one with row pivots, so far, through the calling thread's context */
+void pyrpa_gb_pivoted_vertices(int64_t* n);
 /* statistics of the last mkself / lin_eliash called from this thread: iterations, esterr, Stoner, mu, lambda,
  * Eliashberg applications, then device milliseconds of chi0, vertex, Sigma, DIIS,
  * mu, Dyson, Eliashberg applications, then the FLEX iterations run on FP32 bulk,

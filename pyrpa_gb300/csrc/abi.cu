@@ -98,6 +98,7 @@ void set_thread_context(bool on) {
     c->verbose = pc.verbose;
     c->arnoldi_tol = pc.arnoldi_tol;
     c->kernel_launches = 0;
+    c->pivoted_vertices = 0;
     c->ready = true;
     t_context = c;
   } else {
@@ -605,6 +606,7 @@ void pyrpa_gb_set_thread_stream(const int64_t* on) {
   ABI_TRY set_thread_context(*on != 0); ABI_CATCH("pyrpa_gb_set_thread_stream", (void)0)
 }
 void pyrpa_gb_kernel_launches(int64_t* n) { *n = ctx().kernel_launches; }
+void pyrpa_gb_pivoted_vertices(int64_t* n) { *n = ctx().pivoted_vertices; }
 void pyrpa_gb_last_stats(double* out) {
   const LastStats& s = last_stats();
   const double v[20] = {(double)s.iterations, s.esterr, s.stoner, s.mu, s.lambda, (double)s.applies, s.t_chi0,

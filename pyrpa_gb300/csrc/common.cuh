@@ -311,8 +311,11 @@ struct Context {
   double arnoldi_tol = 0.0;
   // bumped by the entry points, some of which run on callers' own threads
   std::atomic<long long> kernel_launches{0};
+  // vertex matrices that the swept inverse left to the pivoted one
+  std::atomic<long long> pivoted_vertices{0};
   // this context's slot of the device error flags that kernels raise
-  // (singular matrices, unconverged eigenvalue iterations)
+  // (singular matrices, unconverged eigenvalue iterations), and the count for
+  // pivoted_vertices beside it
   int* err = nullptr;
   // this context's timeout flag of the TMA passes, in mapped pinned host
   // memory (made on first use)

@@ -1204,16 +1204,16 @@ bool vertex_sym_launch(const Even& ev, cx<R>* chi, long long nmat, long long est
     for (int q = 0; q < ns; ++q) c[2 * HL + N * N + N + p * ns + q] = (R)Q[p * N + q];
   DBuf<R> ds(c.size());
   ds.upload(c.data(), c.size());
-  DBuf<unsigned> list(nmat), count(1);
-  count.zero();
+  DBuf<unsigned> list(nmat);
+  unsigned* count = reinterpret_cast<unsigned*>(ctx().err + 1);  // zeroed with the error flag
   PGB_SMEM_LIMIT_ONCE((k_vertex_sym<R, N, W>), 220 * 1024);
-  SymTabs tb{ev.d_sin.p, ev.d_sout.p, ev.cls_el.p, ev.mem.p, ev.memcj.p, ev.nmem.p, nc, ns, full ? 1 : 0, list.p, count.p};
+  SymTabs tb{ev.d_sin.p, ev.d_sout.p, ev.cls_el.p, ev.mem.p, ev.memcj.p, ev.nmem.p, nc, ns, full ? 1 : 0, list.p, count};
   const long long tiles = (nmat + L::T - 1) / L::T;
   const long long blocks = std::max(1LL, std::min<long long>(tiles, (long long)ctx().num_sms * 8));
   k_vertex_sym<R, N, W><<<(unsigned)blocks, 32 * W, L::bytes(nc), ctx().stream>>>(chi, nmat, estride, ds.p, tb, mode,
                                                                                         ctx().err);
   count_launch("vertex_sym");
-  vertex_even_launch<R, N>(ev, chi, nmat, estride, dc, mode, full, list.p, count.p);
+  vertex_even_launch<R, N>(ev, chi, nmat, estride, dc, mode, full, list.p, count);
   return true;
 }
 

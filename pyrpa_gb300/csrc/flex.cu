@@ -18,15 +18,16 @@ namespace pgb {
 namespace {
 // Device error flags, one slot per context: a kernel that finds a singular
 // matrix or an unconverged eigenvalue iteration writes its code to the slot
-// its launch was given (ctx().err), and the host reads it after the stage
-__device__ int g_err_slots[kErrSlots];
+// its launch was given (ctx().err), and the host reads it after the stage.  The
+// slot's second word counts the matrices that k_vertex_sym leaves to k_vertex_even
+__device__ int g_err_slots[kErrSlots][2];
 
 }  // namespace
 
 int* err_slot_address(int slot) {
   void* p = nullptr;
   PGB_CUDA(cudaGetSymbolAddress(&p, g_err_slots));
-  return static_cast<int*>(p) + slot;
+  return static_cast<int*>(p) + 2 * slot;
 }
 
 void log(const char* fmt, ...) {

@@ -28,13 +28,14 @@ template <typename T> __device__ __forceinline__ T thresh(T v) {
 // every launch of a flag-raising kernel follows a reset_err on its context
 inline void reset_err() {
   PGB_CHECK(ctx().err != nullptr, "the engine context is not set up (no device error flag)");
-  PGB_CUDA(cudaMemsetAsync(ctx().err, 0, sizeof(int), ctx().stream));
+  PGB_CUDA(cudaMemsetAsync(ctx().err, 0, 2 * sizeof(int), ctx().stream));
 }
 inline int fetch_err() {
-  int e = 0;
-  PGB_CUDA(cudaMemcpyAsync(&e, ctx().err, sizeof(int), cudaMemcpyDeviceToHost, ctx().stream));
+  int e[2] = {0, 0};
+  PGB_CUDA(cudaMemcpyAsync(e, ctx().err, sizeof(e), cudaMemcpyDeviceToHost, ctx().stream));
   sync();
-  return e;
+  ctx().pivoted_vertices += e[1];
+  return e[0];
 }
 
 inline void count_launch(const char* what) {

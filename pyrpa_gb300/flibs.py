@@ -119,6 +119,7 @@ _SIGNATURES = {
     "pyrpa_gb_last_error": [POINTER(c_char), _pi, _pi],
     "pyrpa_gb_clear_error": [],
     "pyrpa_gb_kernel_launches": [_pi],
+    "pyrpa_gb_pivoted_vertices": [_pi],
     "pyrpa_gb_last_stats": [_f64],
     "pyrpa_gb_device_info": [_pi, _pi],
     "pyrpa_gb_fft_profile": [_pi],
@@ -214,6 +215,14 @@ def set_verbose(level: int) -> None:
 def kernel_launches() -> int:
     v = c_int64(0)
     load_library().pyrpa_gb_kernel_launches(byref(v))
+    return v.value
+
+
+def pivoted_vertices() -> int:
+    """Vertex matrices of FP64 even models, so far, that the swept inverse of the
+    symmetric form left to the one with row pivots (chi0 beyond its instability)."""
+    v = c_int64(0)
+    load_library().pyrpa_gb_pivoted_vertices(byref(v))
     return v.value
 
 
