@@ -446,7 +446,31 @@ int64_t make_irr_mesh(int64_t nx, int64_t ny, int64_t nz, std::vector<int64_t>& 
 
 // chi0 entry shared by get_chi0 / get_chi0_tail / get_chi0_conv_
 namespace {
-constexpr long long kEvenMinWork = 1 << 19;  // padded mesh points times pair elements
+// Whether the even form is the faster one for a get_chi0 of `work` padded mesh points times
+// pair elements.  Its tables and checks take 60 us and 0.035 us for each of the `points`
+// mesh points.  Against them stand, per 2^20 of work, the us below, least for the cheapest
+// arithmetic; FP32 transforms of many pairs are bound by memory in both forms.  From four
+// pairs on (FP32: 16) the complex QR of the Stoner factor that it spares decides alone.
+// General and even form in us, one call on each side of the line:
+//   FP64                 one orbital 32x32x200 354 and 372, 32x32x512 610 and 505; 64x64x64 402 and 533,
+//                        64x64x256 1091 and 833; two 16x16x64 388 and 332
+//   double-float         one 32x32x512 405 and 455, 32x32x1024 635 and 596; 64x64x320 773 and 810,
+//                        64x64x512 1084 and 1030; two 16x16x64 361 and 326
+//   double-float, tail   one 32x32x200 500 and 502, 32x32x512 826 and 700; 64x64x64 573 and 676
+//   FP32                 one 64x64x512 847 and 919, 32x32x4096 2412 and 2331; two 64x64x32 704 and 898;
+//                        three 16x16x100 726 and 742, 32x32x40 983 and 986; four 64x64x4 1470 and 1691,
+//                        8x8x16 456 and 422; five 32x32x4 1392 and 1125
+//   FP32, tail           one 64x64x320 903 and 947, 64x64x512 1242 and 1171; two 64x64x32 889 and 1072;
+//                        three 32x32x32 975 and 999, 32x32x40 1161 and 1134
+template <typename R> bool even_chi0_pays(double work, double points, int64_t n, bool tail) {
+  constexpr bool fp32 = std::is_same<R, float>::value;
+  if (work < (1 << 19)) return false;
+  if (fp32 ? (n >= 25 || (n >= 16 && points <= 1024)) : n >= 4) return true;
+  double saved = 200.0;
+  if (fp32) saved = n >= 4 ? 15.0 : (tail ? 60.0 : 30.0);
+  else if (std::is_same<R, dfl>::value && !tail) saved = 62.0;
+  return saved * work / (1 << 20) >= 60.0 + 0.035 * points;
+}
 template <typename R>
 double chi0_entry(double2* chi_out, const double* Smat, const double* Cmat, const double2* Gk, const int64_t* kmap,
                   const int64_t* invk, const int64_t* olist, double temp, int64_t Nx, int64_t Ny, int64_t Nz, int64_t Nw,
@@ -479,12 +503,11 @@ double chi0_entry(double2* chi_out, const double* Smat, const double* Cmat, cons
   //  * the tail-corrected FP64 bubble: it is what lin_eliash is given, whose
   //    fixed-size two-pass Krylov space amplifies a change of 1e-16 in chi0 to
   //    1e-9 .. 2e-8 of the gap (twelve two-orbital models), so its bits stay;
-  //  * small calls, which launches bound: 16x16x256, one orbital, 0.27 ms
-  //    against 0.33 ms with the even form's tables and checks.
+  //  * small calls (even_chi0_pays).
   // A G without the symmetry shows it in a few host elements, which spares it the
   // check on the device and its wait (50 us of 1.2 ms: three orbitals 16x16x64).
   const bool even_call = !irr_chi && !chi_map && !(tail && std::is_same<R, double>::value) &&
-                         g.P * Nchi * Nchi >= kEvenMinWork;
+                         even_chi0_pays<R>((double)g.P * Nchi * Nchi, (double)Nkall, Nchi, tail);
   if (even_call && symmetric_sample(Gk, g.K, (int)Norb) && (!tail || symmetric_bands(eig, uni, Nk, (int)Norb)) &&
       symmetric_blocks(G.p, g.K, (int)Norb, 1.0e-12)) {
     if (with_stoner) g.even = make_even(g, p, Smat, Cmat, (int)sizeof(cx<R>));

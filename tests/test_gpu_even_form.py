@@ -51,7 +51,7 @@ def calls(F, m, G):  # noqa: F811
 
     return {
         "chi0": (lambda: F.get_chi0(*chi0), (64,), ()),
-        "chi0_tail": (lambda: F.get_chi0_tail(*tail), (48, 32), (64,)),
+        "chi0_tail": (lambda: F.get_chi0_tail(*tail), (48,), (64, 32)),
         "mkself": (lambda: F.mkself(*step_args(m), scf_loop=1, eps=0.0, pp=0.5, sw_rescale=True), (64, 48, 32, 3264), ()),
         "flex_eliash": (lambda: F.flex_eliash(m["S"], m["C"], m["kmap"], m["invk"], m["olist"], m["hamk"], m["eig"],
                                               m["uni"], init, np.ones(m["Norb"]), m["mu"], m["fill"], m["temp"],
@@ -168,3 +168,36 @@ def test_fp32_pairing_vertex_of_any_matrix(F, dims, size, gap_sym):  # noqa: F81
     err = np.abs(v - ref).transpose(2, 3, 1, 0).reshape(-1, n * n).max(axis=1)
     allowed = 4 * n * 2.0 ** -24 * (allowed + np.abs(m["S"]).max() + np.abs(m["C"]).max())
     assert (err <= allowed).all(), (err / allowed).max()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dims,bits,tail,even", [
+    ((1, 32, 32, 1, 250), 64, False, False), ((1, 32, 32, 1, 256), 64, False, True),
+    ((1, 64, 64, 1, 64), 64, False, False), ((1, 64, 64, 1, 250), 64, False, True),
+    ((2, 16, 16, 1, 64), 64, False, True),
+    ((1, 32, 32, 1, 512), 48, False, False), ((1, 32, 32, 1, 800), 48, False, True),
+    ((1, 64, 64, 1, 64), 48, True, False), ((1, 32, 32, 1, 256), 48, True, True),
+    ((2, 16, 16, 1, 64), 48, False, True),
+    ((1, 32, 32, 1, 1024), 32, False, False), ((1, 32, 32, 1, 2048), 32, False, True),
+    ((3, 16, 16, 1, 100), 32, False, False), ((3, 16, 16, 1, 128), 32, False, True),
+    ((2, 32, 32, 1, 64), 32, True, False), ((1, 32, 32, 1, 1024), 32, True, True),
+    ((4, 8, 8, 1, 15), 32, False, False), ((4, 8, 8, 1, 16), 32, False, True),
+    ((4, 64, 64, 1, 2), 32, False, False), ((5, 32, 32, 1, 2), 32, False, True)])
+def test_size_from_which_chi0_takes_the_even_form(F, dims, bits, tail, even):  # noqa: F811
+    """The even form where it is the faster one (csrc/abi.cu, even_chi0_pays)."""
+    m = model(*dims)
+    G = dressed(m)
+    if tail:
+        run = lambda: F.get_chi0_tail(m["S"], m["C"], G, m["eig"], m["uni"], m["olist"], m["kmap"],  # noqa: E731
+                                      m["invk"], m["mu"], m["temp"], *m["mesh"])
+    else:
+        run = lambda: F.get_chi0(m["S"], m["C"], G, m["olist"], m["kmap"], m["invk"], m["temp"], *m["mesh"])  # noqa: E731
+    F.set_precision(bits)
+    try:
+        assert takes_even_form(F, run) == even
+        (chi, st), (gchi, gst) = run(), general(run)
+    finally:
+        F.set_precision(64)
+    tol = 2e-5 if bits == 32 else 1e-9
+    close(chi, gchi, tol, 2e-9)
+    assert abs(st - gst) <= tol
