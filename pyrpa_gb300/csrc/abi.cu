@@ -447,29 +447,29 @@ int64_t make_irr_mesh(int64_t nx, int64_t ny, int64_t nz, std::vector<int64_t>& 
 // chi0 entry shared by get_chi0 / get_chi0_tail / get_chi0_conv_
 namespace {
 // Whether the even form is the faster one for a get_chi0 of `work` padded mesh points times
-// pair elements.  Its tables and checks take 60 us and 0.035 us for each of the `points`
+// pair elements.  Its tables and checks take 60 us and 0.008 us for each of the `points`
 // mesh points.  Against them stand, per 2^20 of work, the us below, least for the cheapest
-// arithmetic; FP32 transforms of many pairs are bound by memory in both forms.  From four
-// pairs on (FP32: 16) the complex QR of the Stoner factor that it spares decides alone.
-// General and even form in us, one call on each side of the line:
-//   FP64                 one orbital 32x32x200 354 and 372, 32x32x512 610 and 505; 64x64x64 402 and 533,
-//                        64x64x256 1091 and 833; two 16x16x64 388 and 332
-//   double-float         one 32x32x512 405 and 455, 32x32x1024 635 and 596; 64x64x320 773 and 810,
-//                        64x64x512 1084 and 1030; two 16x16x64 361 and 326
-//   double-float, tail   one 32x32x200 500 and 502, 32x32x512 826 and 700; 64x64x64 573 and 676
-//   FP32                 one 64x64x512 847 and 919, 32x32x4096 2412 and 2331; two 64x64x32 704 and 898;
-//                        three 16x16x100 726 and 742, 32x32x40 983 and 986; four 64x64x4 1470 and 1691,
-//                        8x8x16 456 and 422; five 32x32x4 1392 and 1125
-//   FP32, tail           one 64x64x320 903 and 947, 64x64x512 1242 and 1171; two 64x64x32 889 and 1072;
-//                        three 32x32x32 975 and 999, 32x32x40 1161 and 1134
+// arithmetic; FP32 transforms of several pairs are bound by memory in both forms.  From
+// four pairs on (FP32: 16) the complex QR of the Stoner factor that it spares decides alone.
+// General and even form in us, calls on both sides of the line:
+//   FP64                 one orbital 32x32x200 351 and 352, 32x32x400 522 and 446; 64x64x64 408 and 446,
+//                        64x64x100 582 and 501; two 16x16x64 390 and 340
+//   double-float         one 32x32x512 400 and 423, 32x32x1024 635 and 571; 64x64x128 430 and 478,
+//                        64x64x256 661 and 624; two 16x16x64 367 and 330
+//   double-float, tail   one 32x32x200 497 and 487, 32x32x400 694 and 601; 64x64x64 581 and 593
+//   FP32                 one 32x32x1024 493 and 531, 32x32x2048 822 and 809; two 64x64x32 710 and 813,
+//                        32x32x200 967 and 963; three 32x32x32 818 and 848, 32x32x40 989 and 973;
+//                        four 8x8x16 457 and 440
+//   FP32, tail           one 32x32x512 515 and 539, 32x32x1024 749 and 715; two 64x64x32 896 and 987,
+//                        32x32x200 1177 and 1104
 template <typename R> bool even_chi0_pays(double work, double points, int64_t n, bool tail) {
   constexpr bool fp32 = std::is_same<R, float>::value;
   if (work < (1 << 19)) return false;
-  if (fp32 ? (n >= 25 || (n >= 16 && points <= 1024)) : n >= 4) return true;
-  double saved = 200.0;
-  if (fp32) saved = n >= 4 ? 15.0 : (tail ? 60.0 : 30.0);
-  else if (std::is_same<R, dfl>::value && !tail) saved = 62.0;
-  return saved * work / (1 << 20) >= 60.0 + 0.035 * points;
+  if (n >= (fp32 ? 16 : 4)) return true;
+  double saved = 165.0;
+  if (fp32) saved = n >= 4 ? 11.0 : (tail ? 48.0 : 25.0);
+  else if (std::is_same<R, dfl>::value && !tail) saved = 60.0;
+  return saved * work / (1 << 20) >= 60.0 + 0.008 * points;
 }
 template <typename R>
 double chi0_entry(double2* chi_out, const double* Smat, const double* Cmat, const double2* Gk, const int64_t* kmap,
