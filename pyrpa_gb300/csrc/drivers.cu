@@ -1284,7 +1284,12 @@ void run_lin_eliash(const LinEliashArgs& a) {
     // The even form for a G and a chi that have an even model's relations, but
     // not in FP64: the two-pass Krylov space amplifies the rounding of an
     // application to 1e-9 .. 2e-8 of the gap, and its bits stay
-    if (!std::is_same<R, double>::value && symmetric_blocks(G.p, in.g.K, (int)a.Norb, 1.0e-12)) {
+    // Nor for a triplet or orbitals of both parities, whose F is not even: the vertex alone
+    // saves less than the checks take (triplet, one application, FP32: five orbitals
+    // 32x32x128 14.7 ms, with the even vertex 16.2; one orbital 4x4x64 0.63 and 0.72)
+    bool even_gap = a.gap_sym >= 0;
+    for (int64_t i = 0; i < a.Norb; ++i) even_gap = even_gap && a.prt[i] == a.prt[0] && std::fabs(a.prt[i]) == 1.0;
+    if (!std::is_same<R, double>::value && even_gap && symmetric_blocks(G.p, in.g.K, (int)a.Norb, 1.0e-12)) {
       in.g.even = make_even(in.g, in.p, a.Smat, a.Cmat, (int)sizeof(cx<R>));
       if (in.g.even && (!in.g.even->vertex_ok || !even_chi(in.g, *in.g.even, tmp.p, 1.0e-12))) in.g.even.reset();
     }

@@ -130,8 +130,8 @@ def test_swept_vertex_leaves_indefinite_matrices(F, dims):  # noqa: F811
 @pytest.mark.parametrize("gap_sym", [0, -1])
 def test_fp32_pairing_vertex_of_any_matrix(F, dims, size, gap_sym):  # noqa: F811
     """V_Delta of random matrices with an even model's relations through lin_eliash in 32
-    bits (the pivoted real-basis kernel), far below the instability and far above it,
-    against the FP64 general form.  An elimination of n rows in arithmetic of rounding eps
+    bits (the pivoted real-basis kernel for a singlet, the general one for a triplet), far
+    below the instability and far above it, against the FP64 general form.  An elimination of n rows in arithmetic of rounding eps
     leaves some n eps kappa of an inverse's largest element; 4 n eps kappa is allowed."""
     m = model(*dims)
     No, Nk, n = m["Norb"], len(m["hamk"]), m["Norb"] ** 2
@@ -156,7 +156,7 @@ def test_fp32_pairing_vertex_of_any_matrix(F, dims, size, gap_sym):  # noqa: F81
     F.set_precision(32)
     try:
         v = run()
-        assert takes_even_form(F, run)
+        assert takes_even_form(F, run) == (gap_sym >= 0)
     finally:
         F.set_precision(64)
     X = chi.transpose(2, 3, 1, 0).reshape(-1, n, n)
@@ -201,3 +201,22 @@ def test_size_from_which_chi0_takes_the_even_form(F, dims, bits, tail, even):  #
     tol = 2e-5 if bits == 32 else 1e-9
     close(chi, gchi, tol, 2e-9)
     assert abs(st - gst) <= tol
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dims", [(1, 16, 16, 1, 32), (2, 32, 32, 1, 24), (3, 8, 8, 1, 30), (5, 4, 6, 1, 10)])
+@pytest.mark.parametrize("bits,rtol", [(64, 1e-9), (3264, 1e-4)])
+def test_fused_triplet_matches_general_form(F, dims, bits, rtol):  # noqa: F811
+    """One application of the triplet operator in the fused call: the real-basis vertex with
+    every element written, and the general form of the rest."""
+    m = model(*dims)
+    init = F.get_initial_gap(m["klist"], m["Norb"], 0) + 0.1
+    F.set_precision(bits)
+    try:
+        run = lambda: F.flex_eliash(m["S"], m["C"], m["kmap"], m["invk"], m["olist"], m["hamk"], m["eig"],  # noqa: E731
+                                    m["uni"], init, np.ones(m["Norb"]), m["mu"], m["fill"], m["temp"], m["Nw"],
+                                    *m["mesh"], -1, scf_loop=1, eps=1e-12, sw_tail=True, arnoldi_m=0, itemax=1)
+        r, g = run(), general(run)
+    finally:
+        F.set_precision(64)
+    close(r["gap"], g["gap"], rtol, max(2e-9, 1e-2 * rtol * np.abs(g["gap"]).max()))
