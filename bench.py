@@ -522,11 +522,12 @@ def main():
     peak = peaks.get("hbm_gbs", 6800.0)
     achieved = (fft["bytes"] / (fft["ms"] / 1e3) / 1e9) if fft["ms"] > 0 else None
     per_launch_bytes = fft["bytes"] / max(1, fft["launches"])
-    # DRAM bytes per algorithmic byte of an FFT pass, from an ncu capture of
-    # fft2_kernel<float,8,8> on one 64x64x4096 array (dram__bytes_read.sum +
-    # dram__bytes_write.sum = 208.7 MB over 268.4 MB algorithmic, mean of 3
-    # launches; the write total misses what is still in L2 at kernel end)
-    traffic_per_byte = 208.7 / 268.4
+    # DRAM bytes per algorithmic byte of a time-axis pass over the half mesh, from
+    # ncu captures of fft2_kernel<dfl,8,8> and <dfl,4,8> on one 2112x2048 array
+    # (dram__bytes_read.sum + dram__bytes_write.sum = 75.8 MB over 138.4 MB
+    # algorithmic, mean of 6 launches from a flushed cache; most of the result is
+    # still in L2 at kernel end.  The FP32 passes: 34.6 over 69.2 MB)
+    traffic_per_byte = 75.8 / 138.4
     in_bytes = sum(x.nbytes for x in (m["S"], m["C"], m["kmap"], m["invk"], m["olist"], m["hamk"], m["eig"],
                                         m["uni"], m["init"], m["plist"]))
     out_bytes = res["sigmak"].nbytes + res["gap"].nbytes
@@ -562,13 +563,14 @@ def main():
         "config": config,
         "e2e": {"value": e2e, "unit": "s", "h2d_bytes_per_step": int(in_bytes), "d2h_bytes_per_step": int(out_bytes)},
         "gpu_launches": int(launches),
-        "roofline": {"bound": "hbm", "kernel": "fft2_kernel (FFT passes)", "achieved": achieved, "peak": peak,
+        "roofline": {"bound": "hbm", "kernel": "fft2_kernel, fft2_tma_kernel (FFT passes)", "achieved": achieved, "peak": peak,
                      "unit": "GB/s", "frac": (achieved / peak) if achieved else None,
                      "peak_source": "measured (MEASURED_PEAKS.json hbm_gbs)" if peaks else "fallback",
                      "bytes_per_launch": per_launch_bytes, "launches": fft["launches"],
                      "avg_launch_ms": fft["ms"] / max(1, fft["launches"]),
                      "traffic": per_launch_bytes * traffic_per_byte,
-                     "traffic_source": "ncu capture of one 64x64x4096 FP32 pass, scaled by bytes per launch"},
+                     "traffic_source": "ncu captures of double-float time-axis passes over 2112x2048 points, scaled by "
+                                       "bytes per launch"},
         "solve_roofline": {"bound": "hbm", "bytes": solve_bytes, "seconds": solve_s,
                            "achieved": solve_bytes / solve_s / 1e9 if solve_s > 0 else None, "peak": peak,
                            "unit": "GB/s", "frac": solve_bytes / solve_s / 1e9 / peak if solve_s > 0 else None,

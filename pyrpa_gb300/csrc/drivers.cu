@@ -1109,7 +1109,9 @@ double eliash_core(Inputs& in, cx<R>* chi, const double2* G, const double* init,
   std::vector<double> hprt(Norb);
   PGB_CUDA(cudaMemcpyAsync(hprt.data(), prt, sizeof(double) * Norb, cudaMemcpyDeviceToHost, st));
   sync();
-  // F is even in k for a singlet of orbitals of one parity
+  // F is even in k for a singlet of orbitals of one parity.  mkfk makes it Hermitian in its
+  // orbitals whatever the vector is, so this also holds for the vectors that are not, after a
+  // complex pair of Ritz values
   bool even_delta = in.g.even && singlet;
   for (double x : hprt) even_delta = even_delta && (x == 1.0 || x == -1.0) && x == hprt[0];
   {

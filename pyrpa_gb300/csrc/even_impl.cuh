@@ -753,7 +753,7 @@ __global__ void __launch_bounds__(32 * W, sizeof(R) == 4 ? 4 : 2)
       constexpr int NH = N < 8 ? N : 8;
       const bool head = i < ns;
       // D from the left mixes the ns same-orbital rows only.  Outside of their block
-      // they are the columns of the others, row i entry q / row q entry i = h_q / h_i
+      // they are the columns of the others, row i entry q / row q entry i = h_i / h_q
       // with h = 1, 2, -2 for the three kinds of rows
       const R hi = (R)(i < tb.nplus ? 0.5f : -0.5f);
 #pragma unroll
